@@ -33,6 +33,7 @@
 
 #include <cuda/atomic>
 #include "device_util.cuh"
+#include "order.cuh"
 
 #include <algorithm>
 #include <mutex>
@@ -1552,32 +1553,6 @@ __global__ void k_setup_list(Workers W, const int* __restrict__ list, int n, con
     W.state[w] = WS_DONE;
 }
 
-/// Per set, the exponent span of its vertex coordinates (Span: lowest set bit,
-/// just above the highest), reduced over runs of vertices of one set.
-__global__ void k_set_span(const double* __restrict__ vx, int nv, const int32_t* __restrict__ vset,
-                           int* __restrict__ smin, int* __restrict__ stop) {
-    constexpr int kRun = 64;
-    const int64_t first = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) * kRun;
-    if (first >= nv) return;
-    const int last = int(min(int64_t(nv), first + kRun));
-    int set = vset[first];
-    Span sp;
-    for (int v = int(first); v <= last; ++v) {
-        if (v == last || vset[v] != set) {
-            if (!sp.empty()) {
-                atomicMin(smin + set, sp.emin);
-                atomicMax(stop + set, sp.top);
-            }
-            if (v == last) break;
-            set = vset[v];
-            sp = Span();
-        }
-        sp.add(vx[3 * int64_t(v)]);
-        sp.add(vx[3 * int64_t(v) + 1]);
-        sp.add(vx[3 * int64_t(v) + 2]);
-    }
-}
-
 /// A set whose span makes the orient3d and in_sphere filters exact.
 __global__ void k_set_exact(const int* __restrict__ smin, const int* __restrict__ stop, int nsets,
                             uint8_t* __restrict__ ex) {
@@ -1727,12 +1702,6 @@ __global__ void k_split(Workers W, SplitState S, int n_before) {
 
 // ---- set-up: validation, duplicates, initial tet ----------------------------------
 
-__global__ void k_check_finite(const double* __restrict__ xyz, int64_t n3, uint32_t* bad) {
-    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n3;
-         i += int64_t(gridDim.x) * blockDim.x)
-        if (!isfinite(xyz[i])) atomicOr(bad, 1u);
-}
-
 /// The set holding position g: off[s] <= g < off[s+1].
 __device__ __forceinline__ int set_of(const int64_t* __restrict__ off, int nsets, int64_t g) {
     int lo = 0, hi = nsets - 1;
@@ -1742,32 +1711,6 @@ __device__ __forceinline__ int set_of(const int64_t* __restrict__ off, int nsets
         else hi = mid - 1;
     }
     return lo;
-}
-
-/// Per set, the exponent span of its input coordinates, before any ordering
-/// (as k_set_span; duplicates do not change it).
-__global__ void k_raw_span(const double* __restrict__ xyz, const int64_t* __restrict__ off, int nsets, int64_t n,
-                           int* __restrict__ smin, int* __restrict__ stop) {
-    constexpr int kRun = 64;
-    const int64_t first = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) * kRun;
-    if (first >= n) return;
-    const int64_t last = min(n, first + kRun);
-    int set = set_of(off, nsets, first);
-    Span sp;
-    for (int64_t p = first; p <= last; ++p) {
-        if (p == last || p >= off[set + 1]) {
-            if (!sp.empty()) {
-                atomicMin(smin + set, sp.emin);
-                atomicMax(stop + set, sp.top);
-            }
-            if (p == last) break;
-            while (p >= off[set + 1]) ++set;
-            sp = Span();
-        }
-        sp.add(xyz[3 * p]);
-        sp.add(xyz[3 * p + 1]);
-        sp.add(xyz[3 * p + 2]);
-    }
 }
 
 /// Global index of the input point at rank r (position r of its set's order).
@@ -1848,6 +1791,29 @@ __global__ void k_vertices(const double* __restrict__ xyz, const int32_t* __rest
         vert_point[v] = dups ? rep_at_first[r] : order[r];
         vset[v] = set;
     }
+}
+
+/// Vertex records in the build's own order (own_order_sets): as k_vertices.
+__global__ void k_own_vertices(const double* __restrict__ xyz, const int32_t* __restrict__ vert,
+                               const int32_t* __restrict__ rep, const int64_t* __restrict__ off, int nsets,
+                               int64_t nv, double* __restrict__ vx, int32_t* __restrict__ vert_point,
+                               int32_t* __restrict__ vset) {
+    for (int64_t v = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; v < nv; v += int64_t(gridDim.x) * blockDim.x) {
+        const int64_t g = vert[v];
+        const int set = nsets > 1 ? set_of(off, nsets, g) : 0;
+        vx[3 * v] = xyz[3 * g];
+        vx[3 * v + 1] = xyz[3 * g + 1];
+        vx[3 * v + 2] = xyz[3 * g + 2];
+        vert_point[v] = rep ? rep[v] : int32_t(g - off[set]);
+        vset[v] = set;
+    }
+}
+
+/// voff[s] = the first vertex of set s, from the starts of its levels.
+__global__ void k_own_voff(const int32_t* __restrict__ level_start, int nsets, int levels,
+                           int32_t* __restrict__ voff) {
+    for (int s = int(blockIdx.x) * blockDim.x + threadIdx.x; s <= nsets; s += gridDim.x * blockDim.x)
+        voff[s] = level_start[int64_t(s) * levels];
 }
 
 /// Per set: the first vertex (in insertion order) not collinear with its first
@@ -2270,7 +2236,6 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
     D3G_TRY(d_off.alloc(size_t(nsets) + 1, s));
     D3G_CUDA(cudaMemsetAsync(status.p, 0, 4 * sizeof(uint32_t), s));
     D3G_CUDA(cudaMemcpyAsync(d_off.p, h_off, sizeof(int64_t) * (size_t(nsets) + 1), cudaMemcpyHostToDevice, s));
-    k_check_finite<<<grid_for(3 * n, 256), 256, 0, s>>>(d_xyz, 3 * n, status.p + 1);
 
     cudaEvent_t ph[4];
     for (auto& e : ph) cudaEventCreate(&e);
@@ -2290,38 +2255,44 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
     // take more and shorter levels than the reference's 8, as it does by default
     // when a set's coordinates make the filters exact (lattices and coarse grids,
     // whose long levels collide most) and for a build too small to fill the GPU
-    // (whose levels are inserted chunk by chunk, so shorter ones finish sooner).  The one thing the reference's order
-    // decides is which copy of a repeated point keeps its index (the last one in
-    // that order), so input with repeated points is ordered again by it.
+    // (whose levels are inserted chunk by chunk, so shorter ones finish sooner).
     int growth = opt.level_growth;
+    SetScan scan;
+    D3G_TRY(scan_sets(d_xyz, d_off.p, nsets, n, scan, status.p + 1, s));
     if (growth == 0) {
-        DevBuf<int> span;
         DevBuf<uint8_t> ex;
-        D3G_TRY(span.alloc(size_t(2) * size_t(nsets), s));
         D3G_TRY(ex.alloc(size_t(nsets), s));
-        std::vector<int> init(size_t(2) * size_t(nsets));
-        for (int i = 0; i < nsets; ++i) {
-            init[size_t(i)] = 1 << 20;
-            init[size_t(nsets) + size_t(i)] = -(1 << 20);
-        }
-        D3G_CUDA(cudaMemcpyAsync(span.p, init.data(), sizeof(int) * init.size(), cudaMemcpyHostToDevice, s));
-        k_raw_span<<<grid_for((n + 63) / 64, 128, 1 << 30), 128, 0, s>>>(d_xyz, d_off.p, nsets, n, span.p,
-                                                                         span.p + nsets);
-        k_set_exact<<<grid_for(nsets, 128), 128, 0, s>>>(span.p, span.p + nsets, nsets, ex.p);
+        k_set_exact<<<grid_for(nsets, 128), 128, 0, s>>>(scan.span.p, scan.span.p + nsets, nsets, ex.p);
         std::vector<uint8_t> hex(static_cast<size_t>(nsets));
         D3G_CUDA(cudaMemcpyAsync(hex.data(), ex.p, size_t(nsets), cudaMemcpyDeviceToHost, s));
-        D3G_CUDA(cudaStreamSynchronize(s));   // `init` must outlive the copy
+        D3G_CUDA(cudaStreamSynchronize(s));
         growth = n < kSmallBuildPoints ? kExactSetGrowth : 8;
         for (const uint8_t e : hex) growth = e ? kExactSetGrowth : growth;
     }
-    DevBuf<int32_t> order;
-    D3G_TRY(order.alloc(size_t(N), s));
-
     DevBuf<double> vx;
     DevBuf<int32_t> vert_point, vset, voff;
     int nv = N;
     D3G_TRY(voff.alloc(size_t(nsets) + 1, s));
-    for (;;) {
+    // The own order, or - where its keys cannot tell the points apart - the
+    // spatial sort with the sorts that find repeated points.
+    OwnOrder own;
+    D3G_TRY(own_order_sets(d_xyz, h_off, d_off.p, nsets, growth, scan, own, s));
+    std::vector<int32_t> hlevel;   // own order: first vertex of each (set, level)
+    if (own.ok) {
+        nv = int(own.nv);
+        D3G_TRY(vx.alloc(size_t(3) * nv, s));
+        D3G_TRY(vert_point.alloc(size_t(nv), s));
+        D3G_TRY(vset.alloc(size_t(nv), s));
+        k_own_vertices<<<grid_for(nv, 256), 256, 0, s>>>(d_xyz, own.vert.p, own.rep.p, d_off.p, nsets, nv, vx.p,
+                                                         vert_point.p, vset.p);
+        k_own_voff<<<grid_for(nsets + 1, 128), 128, 0, s>>>(own.level_start.p, nsets, own.levels, voff.p);
+        hlevel.resize(size_t(nsets) * size_t(own.levels) + 1);
+        D3G_CUDA(cudaMemcpyAsync(hlevel.data(), own.level_start.p, sizeof(int32_t) * hlevel.size(),
+                                 cudaMemcpyDeviceToHost, s));
+    }
+    while (!own.ok) {
+        DevBuf<int32_t> order;
+        D3G_TRY(order.alloc(size_t(N), s));
         D3G_TRY(spatial_order_sets_device(d_xyz, h_off, d_off.p, nsets, order.p, s, 1.0 / double(growth)));
         DevBuf<int32_t> ranks, sranks, first, rep, vid;
         DevBuf<unsigned long long> keys, keys2;
@@ -2369,7 +2340,6 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
         break;
     }
     const double level_ratio = 1.0 / double(growth);
-    order.release();
     R.n_vertices = nv;
     std::vector<int32_t> hvoff(size_t(nsets) + 1);
     D3G_CUDA(cudaMemcpyAsync(hvoff.data(), voff.p, sizeof(int32_t) * hvoff.size(), cudaMemcpyDeviceToHost, s));
@@ -2454,23 +2424,9 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
     k_init_tets<<<grid_for(nsets, 64), 64, 0, s>>>(T, vx.p, skips.p, nsets, status.p);
     // Sets whose coordinates span few bits (integer lattices, coarse grids):
     // their filters are exact, so their degenerate queries skip the exact stage.
-    DevBuf<int> set_span;
     DevBuf<uint8_t> set_exact;
-    D3G_TRY(set_span.alloc(size_t(2) * size_t(nsets), s));
     D3G_TRY(set_exact.alloc(size_t(nsets), s));
-    {
-        std::vector<int> init(size_t(2) * size_t(nsets));
-        for (int i = 0; i < nsets; ++i) {
-            init[size_t(i)] = 1 << 20;                   // emin of an empty span
-            init[size_t(nsets) + size_t(i)] = -(1 << 20); // top of an empty span
-        }
-        D3G_CUDA(cudaMemcpyAsync(set_span.p, init.data(), sizeof(int) * init.size(), cudaMemcpyHostToDevice, s));
-        if (nv > 0)
-            k_set_span<<<grid_for((int64_t(nv) + 63) / 64, 128, 1 << 30), 128, 0, s>>>(vx.p, nv, vset.p, set_span.p,
-                                                                                 set_span.p + nsets);
-        k_set_exact<<<grid_for(nsets, 128), 128, 0, s>>>(set_span.p, set_span.p + nsets, nsets, set_exact.p);
-        D3G_CUDA(cudaStreamSynchronize(s));   // `init` must outlive the copy
-    }
+    k_set_exact<<<grid_for(nsets, 128), 128, 0, s>>>(scan.span.p, scan.span.p + nsets, nsets, set_exact.p);
 
     // ---- workers ----
     // A level of s points goes into a triangulation of p earlier points.  Two
@@ -2499,11 +2455,17 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
     int nlev = 0;
     for (int st = 0; st < nsets; ++st) {
         if (hskips[size_t(st)].x < 0) continue;
-        int64_t hb[64];
-        const int nb = multiscale_bounds(R.set_nv[size_t(st)], hb, 63, level_ratio);
         std::vector<int>& L = levels[size_t(st)];
         L.push_back(0);
-        for (int k = nb - 1; k >= 0; --k) L.push_back(int(hb[k]));
+        if (own.ok) {
+            const int32_t* b = hlevel.data() + size_t(st) * size_t(own.levels);
+            const int n_st = int(R.set_nv[size_t(st)]);
+            for (int k = 1; k <= own.levels && L.back() < n_st; ++k) L.push_back(b[k] - b[0]);
+        } else {
+            int64_t hb[64];
+            const int nb = multiscale_bounds(R.set_nv[size_t(st)], hb, 63, level_ratio);
+            for (int k = nb - 1; k >= 0; --k) L.push_back(int(hb[k]));
+        }
         nlev = std::max(nlev, int(L.size()) - 1);
     }
     // The effective alpha of a level: alpha, lowered (to kAlphaSmall at most)

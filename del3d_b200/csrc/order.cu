@@ -1,0 +1,361 @@
+// The build's own insertion order.
+//
+// The cells do not depend on the order points go in (see build.cu), so a build
+// need not pay for the reference's order, whose quickselects are serial in
+// depth and take passes over every run of equal coordinates: 63 ms of "big
+// splits" for 10^7 uniform points, 62 ms for the 100^3 lattice, where the runs
+// are 10^4 long.  Here a point's place is one 64-bit key,
+//
+//     set | level | Hilbert index of its cell in the set's bounding cube
+//
+// sorted by one radix sort.  The level comes from a hash of the coordinates, so
+// equal points share their whole key and end up next to each other: the
+// repeated points are found in the sorted keys, without the sorts of every
+// coordinate that the spatial sort needs after it.  The reference's order
+// decides one thing, which copy of a repeated point keeps its index (the last
+// one in that order, src/triangulation.cpp:77-81); it is worked out only when
+// there are repeated points.
+//
+// Bound by the radix sort's passes over 12-byte pairs (8 of them).  Whole builds
+// on one B200, spatial sort and coordinate sorts -> this: 10^7 uniform points
+// 272 -> 191 ms, the 100^3 lattice 131-224 -> 69 ms, 10^6 uniform 71.8 -> 57.3
+// ms, 4096 mixed sets (35 M points) 664 -> 593 ms.
+#include "device_util.cuh"
+#include "order.cuh"
+
+#include <algorithm>
+
+namespace d3g {
+
+int spatial_order_sets_device(const double* d_xyz, const int64_t* h_off, const int64_t* d_off, int nsets,
+                              int32_t* d_order, cudaStream_t s, double level_ratio = 0.125);
+
+namespace {
+
+constexpr unsigned kFullMask = 0xffffffffu;
+/// Points with equal keys looked through for equal points; a longer run (many
+/// copies of one point, or a set far denser than its bounding cube's grid in
+/// one place) sends the call to the spatial sort.
+constexpr int kKeyRun = 32;
+
+__device__ __forceinline__ int set_of(const int64_t* __restrict__ off, int nsets, int64_t g) {
+    int lo = 0, hi = nsets - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (off[mid] <= g) lo = mid;
+        else hi = mid - 1;
+    }
+    return lo;
+}
+
+__global__ void k_scan_init(unsigned long long* box, int* span, int nsets) {
+    for (int i = int(blockIdx.x) * blockDim.x + threadIdx.x; i < 6 * nsets; i += gridDim.x * blockDim.x) {
+        box[i] = i % 6 < 3 ? ~0ull : 0ull;
+        if (i < 2 * nsets) span[i] = i < nsets ? (1 << 20) : -(1 << 20);
+    }
+}
+
+/// One pass over the coordinates: each warp takes kScanRun consecutive points,
+/// keeps box and span of the set it is in in registers and adds them to the
+/// set's with one atomic each when the set ends.  Bound by reading the points.
+constexpr int kScanRun = 1024;
+__global__ void __launch_bounds__(256) k_scan_sets(const double* __restrict__ xyz, const int64_t* __restrict__ off,
+                                                   int nsets, int64_t n, unsigned long long* __restrict__ box,
+                                                   int* __restrict__ span, uint32_t* __restrict__ nonfinite) {
+    const int lane = threadIdx.x & 31;
+    const int64_t first = ((int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5) * kScanRun;
+    if (first >= n) return;
+    const int64_t last = min(n, first + kScanRun);
+    unsigned long long lo[3], hi[3];
+    Span sp;
+    bool bad = false;
+    auto clear = [&]() {
+        for (int a = 0; a < 3; ++a) {
+            lo[a] = ~0ull;
+            hi[a] = 0ull;
+        }
+        sp = Span();
+    };
+    auto flush = [&](int set) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            for (int a = 0; a < 3; ++a) {
+                lo[a] = min(lo[a], __shfl_xor_sync(kFullMask, lo[a], o));
+                hi[a] = max(hi[a], __shfl_xor_sync(kFullMask, hi[a], o));
+            }
+            sp.emin = min(sp.emin, __shfl_xor_sync(kFullMask, sp.emin, o));
+            sp.top = max(sp.top, __shfl_xor_sync(kFullMask, sp.top, o));
+        }
+        if (lane < 3) {
+            const unsigned long long l = lane == 0 ? lo[0] : (lane == 1 ? lo[1] : lo[2]);
+            const unsigned long long h = lane == 0 ? hi[0] : (lane == 1 ? hi[1] : hi[2]);
+            atomicMin(box + 6 * int64_t(set) + lane, l);
+            atomicMax(box + 6 * int64_t(set) + 3 + lane, h);
+        } else if (lane == 3 && !sp.empty()) {
+            atomicMin(span + set, sp.emin);
+            atomicMax(span + nsets + set, sp.top);
+        }
+        clear();
+    };
+    clear();
+    int cur = set_of(off, nsets, first);
+    int64_t end = off[cur + 1];
+    for (int64_t p0 = first; p0 < last;) {
+        while (p0 >= end) end = off[++cur + 1];   // empty sets hold no point
+        const int64_t stop = min(last, end);
+        for (int64_t p = p0 + lane; p < stop; p += 32) {
+            for (int a = 0; a < 3; ++a) {
+                const double x = xyz[3 * p + a];
+                if (!isfinite(x)) {
+                    bad = true;
+                    continue;
+                }
+                const unsigned long long k = dbl_order_key(x);
+                lo[a] = min(lo[a], k);
+                hi[a] = max(hi[a], k);
+                sp.add(x);
+            }
+        }
+        p0 = stop;
+        __syncwarp();
+        flush(cur);
+    }
+    if (__any_sync(kFullMask, bad) && lane == 0) atomicOr(nonfinite, 1u);
+}
+
+/// A 64-bit finaliser (shift, multiply, shift): every input bit reaches every
+/// output bit.
+__device__ __forceinline__ unsigned long long mix64(unsigned long long x) {
+    x ^= x >> 32;
+    x *= 0xD6E8FEB86659FD93ull;
+    x ^= x >> 32;
+    x *= 0xD6E8FEB86659FD93ull;
+    x ^= x >> 32;
+    return x;
+}
+
+__device__ __forceinline__ unsigned long long coord_bits(double x) {   // -0.0 equals +0.0
+    return x == 0.0 ? 0ull : (unsigned long long)__double_as_longlong(x);
+}
+
+/// Spreads the low 21 bits of x to every third bit.
+__device__ __forceinline__ unsigned long long spread3(unsigned x) {
+    unsigned long long v = x & 0x1FFFFFu;
+    v = (v | v << 32) & 0x001F00000000FFFFull;
+    v = (v | v << 16) & 0x001F0000FF0000FFull;
+    v = (v | v << 8) & 0x100F00F00F00F00Full;
+    v = (v | v << 4) & 0x10C30C30C30C30C3ull;
+    v = (v | v << 2) & 0x1249249249249249ull;
+    return v;
+}
+
+/// Hilbert index of cell (x, y, z) of a 2^bits grid, by Skilling's transform
+/// ("Programming the Hilbert curve", AIP Conf. Proc. 707, 2004): from the high
+/// bit down, undo the rotations and reflections of each subcube, then Gray
+/// encode.
+__device__ __forceinline__ unsigned long long hilbert3(unsigned x, unsigned y, unsigned z, int bits) {
+    for (unsigned q = 1u << (bits - 1); q > 1; q >>= 1) {
+        const unsigned p = q - 1;
+        if (x & q) x ^= p;
+        if (y & q) x ^= p;
+        else {
+            const unsigned t = (x ^ y) & p;
+            x ^= t;
+            y ^= t;
+        }
+        if (z & q) x ^= p;
+        else {
+            const unsigned t = (x ^ z) & p;
+            x ^= t;
+            z ^= t;
+        }
+    }
+    y ^= x;
+    z ^= y;
+    unsigned t = 0;
+    for (unsigned q = 1u << (bits - 1); q > 1; q >>= 1)
+        if (z & q) t ^= q - 1;
+    x ^= t;
+    y ^= t;
+    z ^= t;
+    return spread3(x) << 2 | spread3(y) << 1 | spread3(z);
+}
+
+/// The key of every point.  A point's level is how often its hash, as a
+/// fraction of 2^32, can be multiplied by `growth` before it reaches 1, counted
+/// from the finest level: a level is then growth times the points before it.
+__global__ void __launch_bounds__(256) k_order_keys(const double* __restrict__ xyz, const int64_t* __restrict__ off,
+                                                    int nsets, int64_t n, const unsigned long long* __restrict__ box,
+                                                    int growth, int bits, int level_bits,
+                                                    unsigned long long* __restrict__ keys,
+                                                    int32_t* __restrict__ idx) {
+    for (int64_t p = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; p < n; p += int64_t(gridDim.x) * blockDim.x) {
+        const int set = nsets > 1 ? set_of(off, nsets, p) : 0;
+        const unsigned long long* b = box + 6 * int64_t(set);
+        double ext = 0.0, lo[3];
+        for (int a = 0; a < 3; ++a) {
+            lo[a] = dbl_from_order_key(b[a]);
+            ext = fmax(ext, dbl_from_order_key(b[3 + a]) - lo[a]);
+        }
+        // 2^bits cells along the longest side; 0 for one point or an overflow.
+        const double scale = ext > 0.0 ? double((1u << bits) - 1) / ext : 0.0;
+        unsigned q[3];
+        unsigned long long h = 0;
+        for (int a = 0; a < 3; ++a) {
+            const double x = xyz[3 * p + a];
+            const double f = (x - lo[a]) * scale;
+            q[a] = f > 0.0 ? min(unsigned(f), (1u << bits) - 1) : 0u;
+            h = mix64(h + 0x9E3779B97F4A7C15ull + coord_bits(x));
+        }
+        const int nlev = order_levels(off[set + 1] - off[set], growth);
+        uint32_t r = uint32_t(h >> 32);
+        int down = 0;   // levels below the finest
+        while (down + 1 < nlev && uint64_t(r) * unsigned(growth) < (uint64_t(1) << 32)) {
+            r *= unsigned(growth);
+            ++down;
+        }
+        const unsigned long long code = (unsigned long long)set << level_bits | unsigned(nlev - 1 - down);
+        keys[p] = code << (3 * bits) | hilbert3(q[0], q[1], q[2], bits);
+        idx[p] = int32_t(p);
+    }
+}
+
+__device__ __forceinline__ bool equal_points(const double* __restrict__ xyz, int64_t i, int64_t j) {
+    return xyz[3 * i] == xyz[3 * j] && xyz[3 * i + 1] == xyz[3 * j + 1] && xyz[3 * i + 2] == xyz[3 * j + 2];
+}
+
+/// Over the sorted keys: flags the first copy of every point and counts the
+/// others (flags[0]); flags[1] is raised by a run of equal keys too long to be
+/// looked through.
+__global__ void __launch_bounds__(256) k_first_copies(const double* __restrict__ xyz,
+                                                      const unsigned long long* __restrict__ keys,
+                                                      const int32_t* __restrict__ idx, int64_t n,
+                                                      int32_t* __restrict__ first, int* __restrict__ flags) {
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
+        const unsigned long long k = keys[i];
+        bool copy = false;
+        int64_t j = i - 1;
+        for (; j >= 0 && i - j <= kKeyRun && keys[j] == k; --j) copy = copy || equal_points(xyz, idx[i], idx[j]);
+        if (i - j > kKeyRun && j >= 0 && keys[j] == k) atomicOr(flags + 1, 1);
+        first[i] = copy ? 0 : 1;
+        if (copy) atomicAdd(flags, 1);
+    }
+}
+
+__global__ void k_ranks(const int32_t* __restrict__ order, const int64_t* __restrict__ off, int nsets, int64_t n,
+                        int32_t* __restrict__ rank) {
+    for (int64_t r = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; r < n; r += int64_t(gridDim.x) * blockDim.x)
+        rank[off[set_of(off, nsets, r)] + order[r]] = int32_t(r);
+}
+
+/// With repeated points: the vertices are the first copies, each reported under
+/// the copy whose rank in the reference's order is the last.
+__global__ void __launch_bounds__(256) k_compact_copies(const double* __restrict__ xyz,
+                                                        const unsigned long long* __restrict__ keys,
+                                                        const int32_t* __restrict__ idx,
+                                                        const int32_t* __restrict__ first,
+                                                        const int32_t* __restrict__ pos,
+                                                        const int32_t* __restrict__ rank,
+                                                        const int64_t* __restrict__ off, int nsets, int64_t n,
+                                                        int32_t* __restrict__ vert, int32_t* __restrict__ rep,
+                                                        unsigned long long* __restrict__ vkeys) {
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
+        if (!first[i]) continue;
+        const unsigned long long k = keys[i];
+        const int32_t g = idx[i];
+        int32_t best = g;
+        for (int64_t j = i + 1; j < n && keys[j] == k; ++j)
+            if (rank[idx[j]] > rank[best] && equal_points(xyz, g, idx[j])) best = idx[j];
+        const int32_t v = pos[i];
+        vert[v] = g;
+        rep[v] = int32_t(best - off[set_of(off, nsets, g)]);
+        vkeys[v] = k;
+    }
+}
+
+/// start[c] = the first vertex of (set, level) c, over the vertices' sorted
+/// keys (c = key >> shift, or its rank set * levels + level).
+__global__ void k_level_starts(const unsigned long long* __restrict__ keys, int64_t nv, int shift, int level_bits,
+                               int levels, int64_t total, int32_t* __restrict__ start) {
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i <= nv; i += int64_t(gridDim.x) * blockDim.x) {
+        auto code = [&](int64_t v) {
+            const unsigned long long c = keys[v] >> shift;
+            return int64_t(c >> level_bits) * levels + int64_t(c & ((1ull << level_bits) - 1));
+        };
+        const int64_t from = i > 0 ? code(i - 1) + 1 : 0;
+        const int64_t to = i < nv ? code(i) : total;
+        for (int64_t c = from; c <= to; ++c) start[c] = int32_t(i);
+    }
+}
+
+}  // namespace
+
+int scan_sets(const double* d_xyz, const int64_t* d_off, int nsets, int64_t n, SetScan& S, uint32_t* d_nonfinite,
+              cudaStream_t s) {
+    D3G_TRY(S.box.alloc(size_t(6) * size_t(nsets), s));
+    D3G_TRY(S.span.alloc(size_t(2) * size_t(nsets), s));
+    k_scan_init<<<grid_for(6 * int64_t(nsets), 256), 256, 0, s>>>(S.box.p, S.span.p, nsets);
+    const int64_t warps = (n + kScanRun - 1) / kScanRun;
+    k_scan_sets<<<grid_for(warps * 32, 256, 1 << 30), 256, 0, s>>>(d_xyz, d_off, nsets, n, S.box.p, S.span.p,
+                                                                   d_nonfinite);
+    D3G_CUDA(cudaGetLastError());
+    return D3G_OK;
+}
+
+int own_order_sets(const double* d_xyz, const int64_t* h_off, const int64_t* d_off, int nsets, int growth,
+                   const SetScan& S, OwnOrder& O, cudaStream_t s) {
+    const int64_t n = h_off[nsets];
+    O.ok = false;
+    O.nv = 0;
+    int64_t max_n = 0;
+    for (int i = 0; i < nsets; ++i) max_n = std::max<int64_t>(max_n, h_off[i + 1] - h_off[i]);
+    O.levels = order_levels(max_n, growth);
+    const int level_bits = bits_for(uint64_t(O.levels - 1));
+    const int set_bits = nsets > 1 ? bits_for(uint64_t(nsets - 1)) : 0;
+    const int bits = std::min(21, (64 - level_bits - set_bits) / 3);
+    const int shift = 3 * bits;
+    DevBuf<unsigned long long> keys, keys2;
+    DevBuf<int32_t> idx, idx2, first;
+    DevBuf<int> flags;
+    D3G_TRY(keys.alloc(size_t(n), s));
+    D3G_TRY(keys2.alloc(size_t(n), s));
+    D3G_TRY(idx.alloc(size_t(n), s));
+    D3G_TRY(idx2.alloc(size_t(n), s));
+    D3G_TRY(first.alloc(size_t(n), s));
+    D3G_TRY(flags.alloc(2, s));
+    D3G_CUDA(cudaMemsetAsync(flags.p, 0, 2 * sizeof(int), s));
+    k_order_keys<<<grid_for(n, 256), 256, 0, s>>>(d_xyz, d_off, nsets, n, S.box.p, growth, bits, level_bits, keys2.p,
+                                                  idx2.p);
+    D3G_TRY(sort_pairs(keys2.p, keys.p, idx2.p, idx.p, n, 0, shift + level_bits + set_bits, s));
+    k_first_copies<<<grid_for(n, 256), 256, 0, s>>>(d_xyz, keys.p, idx.p, n, first.p, flags.p);
+    const int64_t total = int64_t(nsets) * O.levels;
+    D3G_TRY(O.level_start.alloc(size_t(total) + 1, s));
+    k_level_starts<<<grid_for(n + 1, 256), 256, 0, s>>>(keys.p, n, shift, level_bits, O.levels, total,
+                                                        O.level_start.p);
+    int hflags[2] = {0, 0};
+    D3G_CUDA(cudaMemcpyAsync(hflags, flags.p, sizeof hflags, cudaMemcpyDeviceToHost, s));
+    D3G_CUDA(cudaStreamSynchronize(s));
+    if (hflags[1]) return D3G_OK;
+    O.nv = n - hflags[0];
+    if (hflags[0] > 0) {
+        DevBuf<int32_t> order, rank;
+        D3G_TRY(order.alloc(size_t(n), s));
+        D3G_TRY(rank.alloc(size_t(n), s));
+        D3G_TRY(spatial_order_sets_device(d_xyz, h_off, d_off, nsets, order.p, s));
+        k_ranks<<<grid_for(n, 256), 256, 0, s>>>(order.p, d_off, nsets, n, rank.p);
+        D3G_TRY(exclusive_scan(first.p, idx2.p, n, s));
+        D3G_TRY(O.vert.alloc(size_t(O.nv), s));
+        D3G_TRY(O.rep.alloc(size_t(O.nv), s));
+        k_compact_copies<<<grid_for(n, 256), 256, 0, s>>>(d_xyz, keys.p, idx.p, first.p, idx2.p, rank.p, d_off,
+                                                          nsets, n, O.vert.p, O.rep.p, keys2.p);
+        k_level_starts<<<grid_for(O.nv + 1, 256), 256, 0, s>>>(keys2.p, O.nv, shift, level_bits, O.levels, total,
+                                                               O.level_start.p);
+    } else {
+        O.vert.swap(idx);
+    }
+    D3G_CUDA(cudaGetLastError());
+    O.ok = true;
+    return D3G_OK;
+}
+
+}  // namespace d3g
