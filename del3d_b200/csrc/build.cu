@@ -64,9 +64,15 @@ constexpr int kBigSlots = 64, kBigCav = 16384;   // boundary facets: twice the t
 
 enum : int { WS_DONE = 0, WS_CAND = 1, WS_LOST = 2, WS_WIN = 3, WS_PARKED = 4, WS_FAIL = 5 };
 
+/// Vertex v's coordinates.  A vertex takes 32 bytes (x, y, z and a pad): one
+/// sector and one 256-bit load, where three packed doubles straddle two sectors
+/// half of the time and take three loads.
 __device__ __forceinline__ Pt vpt(const double* __restrict__ vx, int v) {
-    const double* p = vx + 3 * int64_t(v);
-    return Pt{p[0], p[1], p[2]};
+    double x, y, z, pad;
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+        : "=d"(x), "=d"(y), "=d"(z), "=d"(pad)
+        : "l"(vx + 4 * int64_t(v)));
+    return Pt{x, y, z};
 }
 
 __device__ __forceinline__ int at(const int4& t, int i) {
@@ -86,16 +92,27 @@ __device__ __forceinline__ int pos_of(const int4& t, int v) {
 }
 
 struct Tables {
-    int4* tv;                  // vertices (kInf = the infinite vertex)
-    int4* tn;                  // neighbours: tet * 4 + the facet of that tet facing back
+    int4* rec;                 // per tet 32 bytes, one sector: its vertices (kInf = the infinite
+                               // vertex) and its neighbours (tet * 4 + the facet facing back);
+                               // a slot without a live tet has its first two vertices equal
     unsigned long long* claim; // per-round ownership claims
-    uint8_t* alive;
     int* fnew;                 // per tet facet: the new tet built on it (restar scratch)
     int* vert_tet;             // one live tet incident to each inserted vertex
     int* tet_count;
     int cap;
     int walk_limit;            // steps of a lockstep walk before ST_WALK_LIMIT
     const int32_t* vset;       // the point set of each vertex (batched builds share the tables)
+    __device__ int4& tv(int t) const { return rec[2 * int64_t(t)]; }
+    __device__ int4& tn(int t) const { return rec[2 * int64_t(t) + 1]; }
+    /// Neighbour entry `enc` (tet * 4 + facet).
+    __device__ int& link(int enc) const { return reinterpret_cast<int*>(&tn(enc >> 2))[enc & 3]; }
+    __device__ bool alive(int t) const { return tv(t).x != tv(t).y; }
+    /// Ends tet t: all four vertices one of its own, so that a walk which still
+    /// reads the slot stays in range.
+    __device__ void kill(int t) const {
+        const int x = max(tv(t).x, tv(t).y);   // at most one vertex is kInf
+        tv(t) = make_int4(x, x, x, x);
+    }
 };
 
 struct Workers {
@@ -355,11 +372,11 @@ __device__ int walk_g(bool live, int t, const Pt& p, int pid, const Tables& T, c
                       bool ex, uint32_t* st, const Lanes<G>& L, int* nsteps) {
     int4 tv = make_int4(0, 0, 0, 0);
     if (live) {
-        tv = T.tv[t];
+        tv = T.tv(t);
         const int ip = inf_pos(tv);
         if (ip >= 0) {
-            t = at(T.tn[t], ip) >> 2;
-            tv = T.tv[t];
+            t = at(T.tn(t), ip) >> 2;
+            tv = T.tv(t);
         }
     }
     int prev = -1, found = -1;
@@ -369,7 +386,7 @@ __device__ int walk_g(bool live, int t, const Pt& p, int pid, const Tables& T, c
         int4 tn = make_int4(0, 0, 0, 0);
         bool neg = false;
         if (walking) {
-            tn = T.tn[t];
+            tn = T.tn(t);
             h = h * 1664525u + 1013904223u;
             if (L.sub < 4 && (at(tn, L.sub) >> 2) != prev) {
                 const Pt q[4] = {vpt(vx, tv.x), vpt(vx, tv.y), vpt(vx, tv.z), vpt(vx, tv.w)};
@@ -387,7 +404,7 @@ __device__ int walk_g(bool live, int t, const Pt& p, int pid, const Tables& T, c
                 const unsigned rot = ((m >> s0) | (m << (4 - s0))) & 0xFu;
                 const int i = (s0 + __ffs(int(rot)) - 1) & 3;
                 const int next = at(tn, i) >> 2;
-                const int4 nv = T.tv[next];
+                const int4 nv = T.tv(next);
                 if (inf_pos(nv) >= 0) {
                     found = next;
                     walking = false;
@@ -467,7 +484,7 @@ __global__ void __launch_bounds__(128, 8) k_cavity(Tables T, Workers W, Round R,
         bool abort = false;
         if (valid) {
             c = cav[head + (L.sub >> 2)];
-            nb = at(T.tn[c], i) >> 2;
+            nb = at(T.tn(c), i) >> 2;
             const unsigned long long old = atomicMin(T.claim + nb, key | 1ull);
             if (old == key) {
                 kind = 0;                               // already in the region
@@ -476,7 +493,7 @@ __global__ void __launch_bounds__(128, 8) k_cavity(Tables T, Workers W, Round R,
             } else if ((old >> 1) < mine) {
                 abort = true;                           // an earlier point holds it
             } else {
-                const int r = conflict_test(T.tv[nb], p, v, vx, ex, R.status);
+                const int r = conflict_test(T.tv(nb), p, v, vx, ex, R.status);
                 ctr.count(r);
                 if (r & CT_IN) {
                     const unsigned long long o2 = atomicMin(T.claim + nb, key);
@@ -560,7 +577,7 @@ __global__ void __launch_bounds__(128, 8) k_check(Tables T, Workers W, Round R, 
         for (int k = L.sub; k < ncav; k += G) ok = ok && T.claim[cav[k]] == key;
         for (int k = L.sub; k < nfac; k += G) {
             const int f = fac[k];
-            ok = ok && T.claim[at(T.tn[f >> 2], f & 3) >> 2] == (key | 1ull);
+            ok = ok && T.claim[at(T.tn(f >> 2), f & 3) >> 2] == (key | 1ull);
         }
     }
     const bool win = L.own(__ballot_sync(kFull, !ok)) == 0;
@@ -586,15 +603,15 @@ __device__ int restar_neighbour(const Tables& T, int c, const int4& cv, int i, i
     const int va = at(cv, a), vb = at(cv, b);
     int cur = c, f = j, steps = 0;
     for (;;) {
-        const int enc = at(T.tn[cur], f);
+        const int enc = at(T.tn(cur), f);
         const int nb = enc >> 2;
         if (T.claim[nb] != key) {   // (cur, f) is a boundary facet
-            const int4 tc = T.tv[cur];
+            const int4 tc = T.tv(cur);
             const int wpos = 6 - f - pos_of(tc, va) - pos_of(tc, vb);
             if (wpos < 0 || wpos > 3 || wpos == f) return -1;
             return T.fnew[cur * 4 + f] * 4 + wpos;
         }
-        const int4 tb = T.tv[nb];
+        const int4 tb = T.tv(nb);
         const int g = enc & 3;
         f = 6 - g - pos_of(tb, va) - pos_of(tb, vb);
         cur = nb;
@@ -645,8 +662,8 @@ __global__ void __launch_bounds__(128, 8) k_restar(Tables T, Workers W, Round R,
             const int k = k0 + L.sub;
             if (ok && k < F) {
                 const int c = fac[k] >> 2, i = fac[k] & 3;
-                const int4 cv = T.tv[c];
-                const int4 cn = T.tn[c];
+                const int4 cv = T.tv(c);
+                const int4 cn = T.tn(c);
                 int4 nv = cv, nn = cn;
                 set_at(nv, i, v);
                 for (int j = 0; j < 4 && !bad; ++j) {
@@ -670,17 +687,16 @@ __global__ void __launch_bounds__(128, 8) k_restar(Tables T, Workers W, Round R,
                 const int id = k < C ? cav[k] : base + (k - C);
                 const int4 nv = sv[k], nn = sn[k];
                 const int i = fac[k] & 3;
-                T.tv[id] = nv;
-                T.tn[id] = nn;
-                T.alive[id] = 1;
-                const int enc = at(nn, i);
-                reinterpret_cast<int*>(T.tn)[(enc >> 2) * 4 + (enc & 3)] = id * 4 + i;
+                T.tv(id) = nv;
+                T.tn(id) = nn;
+                    const int enc = at(nn, i);
+                T.link(enc) = id * 4 + i;
                 if (nv.x != kInf) T.vert_tet[nv.x] = id;
                 if (nv.y != kInf) T.vert_tet[nv.y] = id;
                 if (nv.z != kInf) T.vert_tet[nv.z] = id;
                 if (nv.w != kInf) T.vert_tet[nv.w] = id;
             }
-            for (int k = F + L.sub; k < C; k += G) T.alive[cav[k]] = 0;
+            for (int k = F + L.sub; k < C; k += G) T.kill(cav[k]);
             advanced = true;
             if (L.sub == 0) {
                 atomicAdd(R.sums, (unsigned long long)C);
@@ -794,15 +810,15 @@ __device__ __forceinline__ int orient_replaced_filter(const Pt& a, const Pt& b, 
 template <bool kFast>
 __device__ int walk_async(int t, const Pt& p, int pid, const Tables& T, const double* __restrict__ vx,
                           bool ex, uint32_t* st, int lane) {
-    int4 tv = ld4(T.tv + t);
+    int4 tv = ld4(&T.tv(t));
     {
         const int ip = inf_pos(tv);
         if (ip >= 0) {
-            t = at(ld4(T.tn + t), ip) >> 2;
-            tv = ld4(T.tv + t);
+            t = at(ld4(&T.tn(t)), ip) >> 2;
+            tv = ld4(&T.tv(t));
         }
     }
-    int4 tn = ld4(T.tn + t);
+    int4 tn = ld4(&T.tn(t));
     int prev = -1;
     uint32_t h = uint32_t(pid) * 2654435761u + 12345u;
     const int limit = min(kAsyncWalkLimit, T.walk_limit);
@@ -813,7 +829,7 @@ __device__ int walk_async(int t, const Pt& p, int pid, const Tables& T, const do
         int4 pre = make_int4(0, 0, 0, 0);
         if (lane >= 4 && lane < 12) {
             const int nbr = at(tn, lane & 3) >> 2;
-            pre = lane < 8 ? ld4(T.tv + nbr) : ld4(T.tn + nbr);
+            pre = lane < 8 ? ld4(&T.tv(nbr)) : ld4(&T.tn(nbr));
         }
         h = h * 1664525u + 1013904223u;
         const int s0 = int(h >> 30);
@@ -853,17 +869,15 @@ __device__ int walk_async(int t, const Pt& p, int pid, const Tables& T, const do
     return -1;
 }
 
-/// A vertex coordinate read again from memory (the read-only path), as a
-/// volatile load so that the compiler does not keep an earlier read of it
+/// A vertex's coordinates read again from memory (the read-only path), as a
+/// volatile load so that the compiler does not keep an earlier read of them
 /// alive in registers across the code in between.
-__device__ __forceinline__ double ld_coord(const double* p) {
-    double v;
-    asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(v) : "l"(p));
-    return v;
-}
 __device__ __forceinline__ Pt ld_vertex(const double* __restrict__ vx, int v) {
-    const double* q = vx + 3 * int64_t(v);
-    return Pt{ld_coord(q), ld_coord(q + 1), ld_coord(q + 2)};
+    double x, y, z, pad;
+    asm volatile("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+                 : "=d"(x), "=d"(y), "=d"(z), "=d"(pad)
+                 : "l"(vx + 4 * int64_t(v)));
+    return Pt{x, y, z};
 }
 
 /// The symbolic perturbation of an exactly cospherical in_sphere(a, b, c, d, p)
@@ -1024,8 +1038,8 @@ __device__ __forceinline__ int in_circle_tiebreak_ex(int va, int vb, int vd, int
 /// (the caller then leaves the test undecided).
 __device__ __forceinline__ int hull_in_circle_ex(const Tables& T, int tet, int ip, int va, int vb, int vd, int pid,
                                                  const double* __restrict__ vx) {
-    const int f = at(ld4(T.tn + tet), ip) >> 2;
-    const int4 fv = ld4(T.tv + f);
+    const int f = at(ld4(&T.tn(tet)), ip) >> 2;
+    const int4 fv = ld4(&T.tv(f));
     int x = -1;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -1137,9 +1151,9 @@ __device__ int insert_async(int v, int t0, const Tables& T, const Workers& W, co
             // slot not yet filled in - into another set's tets in a batched
             // build.  Only a live tet of v's own set can seed the region.
             int r = 0;
-            const int4 stv = ld4(T.tv + seed);
-            htn[0] = ld4(T.tn + seed);
-            if (__ldcg(T.alive + seed) && T.vset[stv.x != kInf ? stv.x : stv.y] == T.vset[v]) {
+            const int4 stv = ld4(&T.tv(seed));
+            htn[0] = ld4(&T.tn(seed));
+            if (stv.x != stv.y && T.vset[stv.x != kInf ? stv.x : stv.y] == T.vset[v]) {
                 if (kFast) r = in_conflict_fast(T, seed, stv, p, v, vx, ex);
                 else r = conflict_test_seed(stv, p.x, p.y, p.z, v, vx, ex, st);
                 ctr.count(r);
@@ -1171,13 +1185,13 @@ __device__ int insert_async(int v, int t0, const Tables& T, const Workers& W, co
         if (valid) {
             const int pidx = head + (lane >> 2);
             c = cav[pidx];
-            nb = at(pidx < kHandedTn ? htn[pidx] : ld4(T.tn + c), i) >> 2;
+            nb = at(pidx < kHandedTn ? htn[pidx] : ld4(&T.tn(c)), i) >> 2;
             int seen = 0;
             if (try_lock(A.lock, nb, ring, &seen)) {
                 got = nb;
                 int r;
-                const int4 ntv = ld4(T.tv + nb);
-                found_tn = ld4(T.tn + nb);
+                const int4 ntv = ld4(&T.tv(nb));
+                found_tn = ld4(&T.tn(nb));
                 if (kFast) r = in_conflict_fast(T, nb, ntv, p, v, vx, ex);
                 else r = conflict_test(ntv, p, v, vx, ex, st);
                 ctr.count(r);
@@ -1209,7 +1223,7 @@ __device__ int insert_async(int v, int t0, const Tables& T, const Workers& W, co
             __syncwarp();
             for (int k = lane; k < nfac; k += 32) {
                 const int f = fac[k];
-                unlock_if(A.lock, at(ld4(T.tn + (f >> 2)), f & 3) >> 2, ring);
+                unlock_if(A.lock, at(ld4(&T.tn(f >> 2)), f & 3) >> 2, ring);
             }
             __syncwarp();
             for (int k = lane; k < ncav; k += 32) unlock_if(A.lock, cav[k], region);
@@ -1276,11 +1290,11 @@ __device__ int insert_async(int v, int t0, const Tables& T, const Workers& W, co
         unsigned long long* keys = A.ekey + int64_t(slot) * 3 * W.fac_cap;
         for (int k = lane; k < F; k += 32) {
             const int c = fac[k] >> 2, i = fac[k] & 3;
-            const int4 cv = ld4(T.tv + c);
+            const int4 cv = ld4(&T.tv(c));
             int4 nv = cv;
             set_at(nv, i, v);
             sv[k] = nv;
-            sn[k] = ld4(T.tn + c);
+            sn[k] = ld4(&T.tn(c));
             facet_edge_keys(cv, i, keys[3 * k], keys[3 * k + 1], keys[3 * k + 2]);
         }
         __syncwarp();
@@ -1331,17 +1345,16 @@ __device__ int insert_async(int v, int t0, const Tables& T, const Workers& W, co
             const int id = k < C ? cav[k] : base + (k - C);
             const int4 nv = sv[k], nn = sn[k];
             const int i = fac[k] & 3;
-            T.tv[id] = nv;
-            T.tn[id] = nn;
-            T.alive[id] = 1;
+            T.tv(id) = nv;
+            T.tn(id) = nn;
             const int enc = at(nn, i);
-            reinterpret_cast<int*>(T.tn)[(enc >> 2) * 4 + (enc & 3)] = id * 4 + i;
+            T.link(enc) = id * 4 + i;
             if (nv.x != kInf) T.vert_tet[nv.x] = id;
             if (nv.y != kInf) T.vert_tet[nv.y] = id;
             if (nv.z != kInf) T.vert_tet[nv.z] = id;
             if (nv.w != kInf) T.vert_tet[nv.w] = id;
         }
-        for (int k = F + lane; k < C; k += 32) T.alive[cav[k]] = 0;
+        for (int k = F + lane; k < C; k += 32) T.kill(cav[k]);
     }
     // Publish, then give the locks back (ring tets first: their neighbour
     // entries now point at the new tets).
@@ -1352,7 +1365,7 @@ __device__ int insert_async(int v, int t0, const Tables& T, const Workers& W, co
         const int c = f >> 2, i = f & 3;
         // The outside tet across facet (c, i): read from the staged neighbours,
         // since slot c may now hold a new tet.
-        const int outside = ok ? (at(sn[k], i) >> 2) : (at(ld4(T.tn + c), i) >> 2);
+        const int outside = ok ? (at(sn[k], i) >> 2) : (at(ld4(&T.tn(c)), i) >> 2);
         unlock_if(A.lock, outside, ring);
     }
     __syncwarp();
@@ -1461,8 +1474,8 @@ __global__ void k_validate(Tables T, const int* __restrict__ lock, int ntet, int
     int code = 0, where = 0, detail = 0;
     if (i < ntet) {
         const int c = int(i);
-        if (T.alive[c]) {
-            const int4 tv = T.tv[c], tn = T.tn[c];
+        if (T.alive(c)) {
+            const int4 tv = T.tv(c), tn = T.tn(c);
             int ninf = 0;
             for (int k = 0; k < 4 && !code; ++k) {
                 const int v = at(tv, k);
@@ -1482,17 +1495,17 @@ __global__ void k_validate(Tables T, const int* __restrict__ lock, int ntet, int
                 detail = k;
                 const int e = at(tn, k);
                 const int n = e >> 2, f = e & 3;
-                if (e < 0 || n >= ntet || !T.alive[n]) {
+                if (e < 0 || n >= ntet || !T.alive(n)) {
                     code = VF_NEIGHBOUR;
                     break;
                 }
-                if (at(T.tn[n], f) != c * 4 + k) {
+                if (at(T.tn(n), f) != c * 4 + k) {
                     code = VF_BACK;
                     break;
                 }
                 // The facet of c opposite k and the facet of n opposite f: the same
                 // three vertices (in any order).
-                const int4 nvx = T.tv[n];
+                const int4 nvx = T.tv(n);
                 for (int m = 0; m < 4 && !code; ++m) {
                     if (m == k) continue;
                     const int v = at(tv, m);
@@ -1511,8 +1524,8 @@ __global__ void k_validate(Tables T, const int* __restrict__ lock, int ntet, int
         const int v = int(i - ntet);
         const int c = T.vert_tet[v];
         if (c >= 0) {   // -1: not inserted yet
-            if (c >= ntet || !T.alive[c]) code = VF_VERT_TET;
-            else if (pos_of(T.tv[c], v) == 3 && T.tv[c].w != v) code = VF_VERT_TET;
+            if (c >= ntet || !T.alive(c)) code = VF_VERT_TET;
+            else if (pos_of(T.tv(c), v) == 3 && T.tv(c).w != v) code = VF_VERT_TET;
             detail = c;
         }
         where = v;
@@ -1785,9 +1798,8 @@ __global__ void k_vertices(const double* __restrict__ xyz, const int32_t* __rest
         const int32_t v = dups ? vid_of_rank[r] : int32_t(r);
         const int set = set_of(off, nsets, r);
         const int64_t i = off[set] + order[r];
-        vx[3 * int64_t(v)] = xyz[3 * i];
-        vx[3 * int64_t(v) + 1] = xyz[3 * i + 1];
-        vx[3 * int64_t(v) + 2] = xyz[3 * i + 2];
+        reinterpret_cast<double2*>(vx)[2 * int64_t(v)] = make_double2(xyz[3 * i], xyz[3 * i + 1]);
+        reinterpret_cast<double2*>(vx)[2 * int64_t(v) + 1] = make_double2(xyz[3 * i + 2], 0.0);
         vert_point[v] = dups ? rep_at_first[r] : order[r];
         vset[v] = set;
     }
@@ -1801,9 +1813,8 @@ __global__ void k_own_vertices(const double* __restrict__ xyz, const int32_t* __
     for (int64_t v = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; v < nv; v += int64_t(gridDim.x) * blockDim.x) {
         const int64_t g = vert[v];
         const int set = nsets > 1 ? set_of(off, nsets, g) : 0;
-        vx[3 * v] = xyz[3 * g];
-        vx[3 * v + 1] = xyz[3 * g + 1];
-        vx[3 * v + 2] = xyz[3 * g + 2];
+        reinterpret_cast<double2*>(vx)[2 * v] = make_double2(xyz[3 * g], xyz[3 * g + 1]);
+        reinterpret_cast<double2*>(vx)[2 * v + 1] = make_double2(xyz[3 * g + 2], 0.0);
         vert_point[v] = rep ? rep[v] : int32_t(g - off[set]);
         vset[v] = set;
     }
@@ -1899,9 +1910,8 @@ __global__ void k_init_tets(Tables T, const double* __restrict__ vx, const int4*
                 }
             }
         for (int t = 0; t < 5; ++t) {
-            T.tv[base + t] = tv[t];
-            T.tn[base + t] = tn[t];
-            T.alive[base + t] = 1;
+            T.tv(base + t) = tv[t];
+            T.tn(base + t) = tn[t];
         }
         T.vert_tet[v0] = base;
         T.vert_tet[v1] = base;
@@ -1928,18 +1938,18 @@ __device__ __forceinline__ int4 canonical(int4 t) {
     return t;
 }
 
-__global__ void k_cell_flags(const int4* __restrict__ tv, const uint8_t* __restrict__ alive, int ntet,
+__global__ void k_cell_flags(const int4* __restrict__ rec, int ntet,
                              bool with_infinite, int32_t* __restrict__ flag) {
     for (int t = int(blockIdx.x) * blockDim.x + threadIdx.x; t < ntet; t += gridDim.x * blockDim.x) {
-        const int4 c = tv[t];
-        flag[t] = alive[t] && (with_infinite || inf_pos(c) < 0) ? 1 : 0;
+        const int4 c = rec[2 * int64_t(t)];
+        flag[t] = c.x != c.y && (with_infinite || inf_pos(c) < 0) ? 1 : 0;
     }
 }
 
 /// Writes the flagged tets, mapped to input point indices and canonicalised,
 /// plus (khi given) their sort keys (shifted by one so the infinite vertex, -1,
 /// is 0).
-__global__ void k_cells_out(const int4* __restrict__ tv, const int32_t* __restrict__ flag,
+__global__ void k_cells_out(const int4* __restrict__ rec, const int32_t* __restrict__ flag,
                             const int32_t* __restrict__ pos, int ntet,
                             const int32_t* __restrict__ vert_point, const int32_t* __restrict__ vset,
                             int kbits, int4* __restrict__ cells,
@@ -1947,7 +1957,7 @@ __global__ void k_cells_out(const int4* __restrict__ tv, const int32_t* __restri
                             int32_t* __restrict__ idx, int32_t* __restrict__ cset) {
     for (int t = int(blockIdx.x) * blockDim.x + threadIdx.x; t < ntet; t += gridDim.x * blockDim.x) {
         if (!flag[t]) continue;
-        const int4 c = tv[t];
+        const int4 c = rec[2 * int64_t(t)];
         if (cset) cset[pos[t]] = vset[c.x != kInf ? c.x : c.y];
         int4 q;
         q.x = c.x == kInf ? -1 : vert_point[c.x];
@@ -2280,7 +2290,7 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
     std::vector<int32_t> hlevel;   // own order: first vertex of each (set, level)
     if (own.ok) {
         nv = int(own.nv);
-        D3G_TRY(vx.alloc(size_t(3) * nv, s));
+        D3G_TRY(vx.alloc(size_t(4) * nv, s));
         D3G_TRY(vert_point.alloc(size_t(nv), s));
         D3G_TRY(vset.alloc(size_t(nv), s));
         k_own_vertices<<<grid_for(nv, 256), 256, 0, s>>>(d_xyz, own.vert.p, own.rep.p, d_off.p, nsets, nv, vx.p,
@@ -2326,7 +2336,7 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
             continue;
         }
         nv = N - hdup;
-        D3G_TRY(vx.alloc(size_t(3) * nv, s));
+        D3G_TRY(vx.alloc(size_t(4) * nv, s));
         D3G_TRY(vert_point.alloc(size_t(nv), s));
         D3G_TRY(vset.alloc(size_t(nv), s));
         if (hdup > 0) {
@@ -2393,29 +2403,22 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
     if (cap64 > (int64_t(1) << 29)) cap64 = int64_t(1) << 29;
     T.cap = int(cap64);
     T.walk_limit = opt.walk_limit > 0 ? opt.walk_limit : kWalkLimit;
-    DevBuf<int4> tv, tn;
+    DevBuf<int4> rec;
     DevBuf<unsigned long long> claim;
-    DevBuf<uint8_t> alive;
     DevBuf<int> fnew, vert_tet, tet_count;
-    D3G_TRY(tv.alloc(size_t(T.cap), s));
-    D3G_TRY(tn.alloc(size_t(T.cap), s));
+    D3G_TRY(rec.alloc(2 * size_t(T.cap), s));
     D3G_TRY(claim.alloc(size_t(T.cap), s));
-    D3G_TRY(alive.alloc(size_t(T.cap), s));
     D3G_TRY(fnew.alloc(size_t(T.cap) * 4, s));
     D3G_TRY(vert_tet.alloc(size_t(nv), s));
     D3G_TRY(tet_count.alloc(1, s));
     D3G_CUDA(cudaMemsetAsync(claim.p, 0xFF, sizeof(unsigned long long) * size_t(T.cap), s));
-    D3G_CUDA(cudaMemsetAsync(alive.p, 0, size_t(T.cap), s));
     // Every slot holds in-range indices from the start (the asynchronous walk
     // may read a slot before its tet is written), and a vertex not inserted yet
     // has no tet.
-    D3G_CUDA(cudaMemsetAsync(tv.p, 0, sizeof(int4) * size_t(T.cap), s));
-    D3G_CUDA(cudaMemsetAsync(tn.p, 0, sizeof(int4) * size_t(T.cap), s));
+    D3G_CUDA(cudaMemsetAsync(rec.p, 0, 2 * sizeof(int4) * size_t(T.cap), s));
     D3G_CUDA(cudaMemsetAsync(vert_tet.p, 0xFF, sizeof(int) * size_t(nv), s));
-    T.tv = tv.p;
-    T.tn = tn.p;
+    T.rec = rec.p;
     T.claim = claim.p;
-    T.alive = alive.p;
     T.fnew = fnew.p;
     T.vert_tet = vert_tet.p;
     T.tet_count = tet_count.p;
@@ -2994,7 +2997,7 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
         DevBuf<int32_t> flag, pos, idx, cset;
         D3G_TRY(flag.alloc(size_t(ntet), s));
         D3G_TRY(pos.alloc(size_t(ntet), s));
-        k_cell_flags<<<grid_for(ntet, 256), 256, 0, s>>>(tv.p, alive.p, ntet, with_inf, flag.p);
+        k_cell_flags<<<grid_for(ntet, 256), 256, 0, s>>>(rec.p, ntet, with_inf, flag.p);
         D3G_TRY(exclusive_scan(flag.p, pos.p, ntet, s));
         int last_pos = 0, last_flag = 0;
         D3G_CUDA(cudaMemcpyAsync(&last_pos, pos.p + ntet - 1, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -3011,7 +3014,7 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
         if (!with_inf) {
             // Buckets by first vertex; the radix sort of every cell only if a
             // bucket is too large for one thread.
-            k_cells_out<<<grid_for(ntet, 256), 256, 0, s>>>(tv.p, flag.p, pos.p, ntet, vert_point.p, vset.p,
+            k_cells_out<<<grid_for(ntet, 256), 256, 0, s>>>(rec.p, flag.p, pos.p, ntet, vert_point.p, vset.p,
                                                             kbits, raw.p, nullptr, nullptr, nullptr,
                                                             single ? nullptr : cset.p);
             DevBuf<int> bstart, bfill, big, mid;
@@ -3048,13 +3051,13 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
             if (!hbig[0] && hbig[1] > 0)
                 k_bucket_sort_block<<<unsigned(hbig[1]), 512, 0, s>>>(R.cells.p, bstart.p, mid.p);
             if (hbig[0]) {
-                k_cells_out<<<grid_for(ntet, 256), 256, 0, s>>>(tv.p, flag.p, pos.p, ntet, vert_point.p, vset.p,
+                k_cells_out<<<grid_for(ntet, 256), 256, 0, s>>>(rec.p, flag.p, pos.p, ntet, vert_point.p, vset.p,
                                                                 kbits, raw.p, khi.p, klo.p, idx.p,
                                                                 single ? nullptr : cset.p);
                 D3G_TRY(sort_cells(raw, khi, klo, idx, single ? nullptr : cset.p, nsets, nc, kbits, R.cells, s));
             }
         } else {
-            k_cells_out<<<grid_for(ntet, 256), 256, 0, s>>>(tv.p, flag.p, pos.p, ntet, vert_point.p, vset.p,
+            k_cells_out<<<grid_for(ntet, 256), 256, 0, s>>>(rec.p, flag.p, pos.p, ntet, vert_point.p, vset.p,
                                                             kbits, raw.p, khi.p, klo.p, idx.p, nullptr);
             D3G_TRY(sort_cells(raw, khi, klo, idx, nullptr, 1, nc, kbits, R.all, s));
             R.n_all = nc;
