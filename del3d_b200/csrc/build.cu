@@ -96,6 +96,7 @@ struct Tables {
                                // vertex) and its neighbours (tet * 4 + the facet facing back);
                                // a slot without a live tet has its first two vertices equal
     unsigned long long* claim; // per-round ownership claims
+    int* lock;                 // lock words of the asynchronous passes (null: lockstep rounds only)
     int* fnew;                 // per tet facet: the new tet built on it (restar scratch)
     int* vert_tet;             // one live tet incident to each inserted vertex
     int* tet_count;
@@ -689,7 +690,8 @@ __global__ void __launch_bounds__(128, 8) k_restar(Tables T, Workers W, Round R,
                 const int i = fac[k] & 3;
                 T.tv(id) = nv;
                 T.tn(id) = nn;
-                    const int enc = at(nn, i);
+                if (T.lock && k >= C) T.lock[id] = 0;   // the slot's first tet
+                const int enc = at(nn, i);
                 T.link(enc) = id * 4 + i;
                 if (nv.x != kInf) T.vert_tet[nv.x] = id;
                 if (nv.y != kInf) T.vert_tet[nv.y] = id;
@@ -753,6 +755,15 @@ constexpr int kLeftPasses = 8;
 constexpr int kExactSetGrowth = 4;
 constexpr int64_t kSmallBuildPoints = 65536;
 constexpr int kAsyncWalkLimit = 1 << 14;
+// BRIO level growth of an asynchronous build's own order: a level's depth is
+// (growth - 1) * alpha insertions in a row while the GPU is not full, so short
+// levels have the least depth per point.
+constexpr int kGroupGrowth = 2;
+// Passes of k_insert_groups over what the last level left.
+constexpr int kLastPasses = 3;
+// Vertices of the level before, to either side along the curve, among which a
+// vertex's guide is the nearest.
+constexpr int kGuideReach = 4;
 // The neighbour records of a warp's first kHandedTn region tets, read under
 // their locks together with their vertices, are kept in shared memory for the
 // growth step that expands them (instead of being read from L2 again there).
@@ -804,10 +815,6 @@ __device__ __forceinline__ int orient_replaced_filter(const Pt& a, const Pt& b, 
 /// Visibility walk on a mesh other warps are changing: reads go to L2 and may
 /// be stale, so the tet it returns is only a candidate, checked under its lock.
 /// Returns -1 after kAsyncWalkLimit steps (or the build's walk limit, if lower).
-/// kFast: orientations come from the filter alone, and a step the filter cannot
-/// decide ends the walk with -2 (the point is left to the other variant, which
-/// runs the exact stage).
-template <bool kFast>
 __device__ int walk_async(int t, const Pt& p, int pid, const Tables& T, const double* __restrict__ vx,
                           bool ex, uint32_t* st, int lane) {
     int4 tv = ld4(&T.tv(t));
@@ -833,24 +840,17 @@ __device__ int walk_async(int t, const Pt& p, int pid, const Tables& T, const do
         }
         h = h * 1664525u + 1013904223u;
         const int s0 = int(h >> 30);
-        bool neg = false, undecided = false;
+        bool neg = false;
         if (lane < 4 && (at(tn, lane) >> 2) != prev && tv.x != kInf && tv.y != kInf && tv.z != kInf &&
             tv.w != kInf) {
             const Pt a = vpt(vx, tv.x), b = vpt(vx, tv.y), c = vpt(vx, tv.z), d = vpt(vx, tv.w);
             int o = orient_replaced_filter(a, b, c, d, lane, p, ex);
             if (o == 2) {
-                if (kFast) {
-                    undecided = true;
-                    o = 0;
-                } else {
-                    const Pt A = lane == 0 ? p : a, B = lane == 1 ? p : b, C = lane == 2 ? p : c,
-                             D = lane == 3 ? p : d;
-                    o = orient3d(A, B, C, D, st);
-                }
+                const Pt A = lane == 0 ? p : a, B = lane == 1 ? p : b, C = lane == 2 ? p : c, D = lane == 3 ? p : d;
+                o = orient3d(A, B, C, D, st);
             }
             neg = o < 0;
         }
-        if (kFast && __any_sync(kFull, undecided)) return -2;
         const unsigned m = __ballot_sync(kFull, neg) & 0xFu;
         if (m == 0) return t;
         const unsigned rot = ((m >> s0) | (m << (4 - s0))) & 0xFu;
@@ -915,6 +915,21 @@ __device__ __forceinline__ int in_sphere_tiebreak_ex(const int4 t, int pid, cons
     return -1;
 }
 
+/// Error bound of in_sphere_filter from the squared distances alone.  Each pair
+/// sum |x1 y2| + |x2 y1| of the permanent is at most l = max lift (Cauchy-
+/// Schwarz), each coordinate at most sqrt(l), so the permanent is at most
+/// 12 l^(5/2), and det^2 > (12 bound)^2 l^5 certifies what the filter would
+/// certify.  `l` is taken from the lifts' high words, rounded up; the range
+/// check keeps l^5 and det^2 normal (outside it the filter's own bound decides).
+__device__ __forceinline__ bool in_sphere_far(double det, double alift, double blift, double clift, double dlift) {
+    const int h = max(max(__double2hiint(alift), __double2hiint(blift)),
+                      max(__double2hiint(clift), __double2hiint(dlift)));   // lifts are not negative
+    constexpr int kLow = (1023 - 180) << 20, kHigh = (1023 + 180) << 20;
+    const double l = __hiloint2double(h + 1, 0), l2 = fmul(l, l);
+    constexpr double c = 12.0 * kInSphereBound * (1.0 + 1e-6);
+    return h > kLow && h < kHigh && fmul(det, det) > fmul(fmul(fmul(l2, l2), l), c * c);
+}
+
 /// in_sphere_filter's arithmetic, operation for operation (so its value and
 /// its decision are bit-identical), in an order that retires values early:
 /// lifts right after the differences, each product pair folded at once into
@@ -929,42 +944,43 @@ __device__ __forceinline__ InSphereFilter in_sphere_filter_lean(const Pt& a, con
     const double blift = fadd(fadd(fmul(bex, bex), fmul(bey, bey)), fmul(bez, bez));
     const double clift = fadd(fadd(fmul(cex, cex), fmul(cey, cey)), fmul(cez, cez));
     const double dlift = fadd(fadd(fmul(dex, dex), fmul(dey, dey)), fmul(dez, dez));
-    double ab, bc, cd, da, ac, bd, sab, sbc, scd, sda, sac, sbd;
+    double ab, bc, cd, da, ac, bd;
     {
         const double p = fmul(aex, bey), q = fmul(bex, aey);
         ab = fsub(p, q);
-        sab = fadd(fabs_(p), fabs_(q));
     }
     {
         const double p = fmul(bex, cey), q = fmul(cex, bey);
         bc = fsub(p, q);
-        sbc = fadd(fabs_(p), fabs_(q));
     }
     {
         const double p = fmul(cex, dey), q = fmul(dex, cey);
         cd = fsub(p, q);
-        scd = fadd(fabs_(p), fabs_(q));
     }
     {
         const double p = fmul(dex, aey), q = fmul(aex, dey);
         da = fsub(p, q);
-        sda = fadd(fabs_(p), fabs_(q));
     }
     {
         const double p = fmul(aex, cey), q = fmul(cex, aey);
         ac = fsub(p, q);
-        sac = fadd(fabs_(p), fabs_(q));
     }
     {
         const double p = fmul(bex, dey), q = fmul(dex, bey);
         bd = fsub(p, q);
-        sbd = fadd(fabs_(p), fabs_(q));
     }
     const double abc = fadd(fsub(fmul(aez, bc), fmul(bez, ac)), fmul(cez, ab));
     const double bcd = fadd(fsub(fmul(bez, cd), fmul(cez, bd)), fmul(dez, bc));
     const double cda = fadd(fadd(fmul(cez, da), fmul(dez, ac)), fmul(aez, cd));
     const double dab = fadd(fadd(fmul(dez, ab), fmul(aez, bd)), fmul(bez, da));
     const double det = fadd(fsub(fmul(dlift, abc), fmul(clift, dab)), fsub(fmul(blift, cda), fmul(alift, bcd)));
+    if (in_sphere_far(det, alift, blift, clift, dlift)) return InSphereFilter{det, true};
+    const double sab = fadd(fabs_(fmul(aex, bey)), fabs_(fmul(bex, aey)));
+    const double sbc = fadd(fabs_(fmul(bex, cey)), fabs_(fmul(cex, bey)));
+    const double scd = fadd(fabs_(fmul(cex, dey)), fabs_(fmul(dex, cey)));
+    const double sda = fadd(fabs_(fmul(dex, aey)), fabs_(fmul(aex, dey)));
+    const double sac = fadd(fabs_(fmul(aex, cey)), fabs_(fmul(cex, aey)));
+    const double sbd = fadd(fabs_(fmul(bex, dey)), fabs_(fmul(dex, bey)));
     const double aezp = fabs_(aez), bezp = fabs_(bez), cezp = fabs_(cez), dezp = fabs_(dez);
     const double pa = fadd(fadd(fmul(scd, bezp), fmul(sbd, cezp)), fmul(sbc, dezp));
     const double pb = fadd(fadd(fmul(sda, cezp), fmul(sac, dezp)), fmul(scd, aezp));
@@ -1089,6 +1105,8 @@ __device__ __forceinline__ int in_conflict_fast(const Tables& T, int tet, const 
 
 enum : int { AI_DONE = 0, AI_RETRY = 1, AI_LEAVE = 2, AI_DEFER = 3 };
 
+#include "insert_groups.cuh"
+
 /// Key of the edge (a, b), either order.
 __device__ __forceinline__ unsigned long long edge_key(int a, int b) {
     const unsigned ua = unsigned(a + 1), ub = unsigned(b + 1);
@@ -1108,30 +1126,17 @@ __device__ __forceinline__ void facet_edge_keys(const int4 c, int i, unsigned lo
 
 /// One insertion of point v by the whole warp, starting the walk at tet t0.
 /// AI_DONE: inserted; AI_RETRY: a lock was taken by another warp (nothing
-/// changed, every lock given back); AI_LEAVE: leave it for the rounds;
-/// AI_DEFER (kFast only): a test the filter could not decide, nothing changed,
-/// leave it for the other variant.
-///
-/// kFast = true is the variant for the bulk of the points: its walk and
-/// conflict tests use the filters alone and make no calls.  A call anywhere in
-/// the insertion loop - even one the uniform case never takes - makes the
-/// compiler keep the loop's state in local memory around it; without calls the
-/// state stays in registers.  kFast = false runs the exact stage, the hull
-/// in-circle test and the tie-breaks, out of line, for the points the fast
-/// variant deferred.
-template <bool kFast>
-__device__ int insert_async(int v, int t0, const Tables& T, const Workers& W, const AsyncCtx& A,
+/// changed, every lock given back); AI_LEAVE: leave it for the rounds.  Every
+/// test runs to its end here: the exact stage, the hull in-circle test and the
+/// tie-breaks, out of line.
+__device__ int insert_full(int v, int t0, const Tables& T, const Workers& W, const AsyncCtx& A,
                             const double* __restrict__ vx, bool ex, uint32_t* st, int slot, int lane,
                             unsigned long long* nC, unsigned long long* nF, const SharedCounters& ctr,
                             int4* htn) {
     const int owner = slot + 1;
     const int region = owner << 1, ring = region | 1;
     const Pt p = vpt(vx, v);
-    const int seed = walk_async<kFast>(t0, p, v, T, vx, ex, st, lane);
-    if (kFast && seed == -2) {
-        if (lane == 0) atomicAdd(A.stats + 6, 1ull);
-        return AI_DEFER;
-    }
+    const int seed = walk_async(t0, p, v, T, vx, ex, st, lane);
     if (seed < 0) {
         if (lane == 0) atomicAdd(A.stats + 1, 1ull);
         return AI_RETRY;
@@ -1139,7 +1144,7 @@ __device__ int insert_async(int v, int t0, const Tables& T, const Workers& W, co
     int* cav = W.cav + int64_t(slot) * W.cav_cap;
     int* fac = W.fac + int64_t(slot) * W.fac_cap;
     // Seed: lock it, then check under the lock that it is alive and in conflict.
-    int res = 0;   // 0 ok, 1 lock held by another, 2 not a valid seed, 3 undecided (kFast)
+    int res = 0;   // 0 ok, 1 lock held by another, 2 not a valid seed
 
     if (lane == 0) {
         int seen = 0;
@@ -1154,22 +1159,21 @@ __device__ int insert_async(int v, int t0, const Tables& T, const Workers& W, co
             const int4 stv = ld4(&T.tv(seed));
             htn[0] = ld4(&T.tn(seed));
             if (stv.x != stv.y && T.vset[stv.x != kInf ? stv.x : stv.y] == T.vset[v]) {
-                if (kFast) r = in_conflict_fast(T, seed, stv, p, v, vx, ex);
-                else r = conflict_test_seed(stv, p.x, p.y, p.z, v, vx, ex, st);
+                r = conflict_test_seed(stv, p.x, p.y, p.z, v, vx, ex, st);
                 ctr.count(r);
             }
             if (r & CT_IN) {
                 cav[0] = seed;
             } else {
                 unlock_if(A.lock, seed, region);
-                res = (r & CT_UNDECIDED) ? 3 : 2;
+                res = 2;
             }
         }
     }
     res = __shfl_sync(kFull, res, 0);
     if (res != 0) {
-        if (lane == 0) atomicAdd(A.stats + (res == 1 ? 0 : (res == 2 ? 2 : 6)), 1ull);
-        return res == 3 ? AI_DEFER : AI_RETRY;
+        if (lane == 0) atomicAdd(A.stats + (res == 1 ? 0 : 2), 1ull);
+        return AI_RETRY;
     }
     __syncwarp();
     const unsigned lt = (1u << lane) - 1u;
@@ -1180,7 +1184,7 @@ __device__ int insert_async(int v, int t0, const Tables& T, const Workers& W, co
         const bool valid = (lane >> 2) < nproc;
         const int i = lane & 3;
         int c = 0, nb = 0, kind = 0, got = -1;   // got: a tet this lane locked in this step
-        bool abort = false, undecided = false;
+        bool abort = false;
         int4 found_tn = make_int4(0, 0, 0, 0);
         if (valid) {
             const int pidx = head + (lane >> 2);
@@ -1189,18 +1193,15 @@ __device__ int insert_async(int v, int t0, const Tables& T, const Workers& W, co
             int seen = 0;
             if (try_lock(A.lock, nb, ring, &seen)) {
                 got = nb;
-                int r;
                 const int4 ntv = ld4(&T.tv(nb));
                 found_tn = ld4(&T.tn(nb));
-                if (kFast) r = in_conflict_fast(T, nb, ntv, p, v, vx, ex);
-                else r = conflict_test(ntv, p, v, vx, ex, st);
+                const int r = conflict_test(ntv, p, v, vx, ex, st);
                 ctr.count(r);
                 if (r & CT_IN) {
                     LockRef(A.lock[nb]).store(region, cuda::memory_order_relaxed);
                     kind = 2;
                 } else {
-                    kind = 1;                             // undecided: held as ring
-                    undecided = (r & CT_UNDECIDED) != 0;
+                    kind = 1;
                 }
             } else if (seen == region) {
                 kind = 0;                                 // already in the region
@@ -1213,11 +1214,10 @@ __device__ int insert_async(int v, int t0, const Tables& T, const Workers& W, co
         __syncwarp();
         if (kind == 3) kind = __ldcg(A.lock + nb) == region ? 0 : 1;
         const bool ab = __any_sync(kFull, abort);
-        const bool und = kFast && __any_sync(kFull, undecided);
         const unsigned mc = __ballot_sync(kFull, kind == 2);
         const unsigned mf = __ballot_sync(kFull, kind == 1);
         const bool full = ncav + __popc(mc) > W.cav_cap || nfac + __popc(mf) > W.fac_cap;
-        if (ab || full || und) {
+        if (ab || full) {
             // Give everything back: this step's new locks, the region, the ring.
             if (got >= 0) unlock_if(A.lock, got, kind == 2 ? region : ring);
             __syncwarp();
@@ -1227,8 +1227,8 @@ __device__ int insert_async(int v, int t0, const Tables& T, const Workers& W, co
             }
             __syncwarp();
             for (int k = lane; k < ncav; k += 32) unlock_if(A.lock, cav[k], region);
-            if (lane == 0) atomicAdd(A.stats + (ab ? 0 : (und ? 6 : 3)), 1ull);
-            outcome = ab ? AI_RETRY : (und ? AI_DEFER : AI_LEAVE);
+            if (lane == 0) atomicAdd(A.stats + (ab ? 0 : 3), 1ull);
+            outcome = ab ? AI_RETRY : AI_LEAVE;
             break;
         }
         if (kind == 2) cav[ncav + __popc(mc & lt)] = nb;
@@ -1256,26 +1256,8 @@ __device__ int insert_async(int v, int t0, const Tables& T, const Workers& W, co
     ok = __shfl_sync(kFull, ok, 0);
     int4* sv = W.st_v + int64_t(slot) * W.fac_cap;
     int4* sn = W.st_n + int64_t(slot) * W.fac_cap;
-    // Fresh slots are locked too, so that whoever locks one later reads it only
-    // after this warp's release.  A stale walk of another warp may hold one for
-    // a moment (it finds it not alive and lets go): wait for that, bounded.
-    bool locked_fresh = true;
-    if (ok) {
-        for (int k = C + lane; k < F; k += 32) {
-            int seen = 0;
-            bool got = false;
-            for (int it = 0; it < (1 << 16) && !got; ++it) {
-                got = try_lock(A.lock, base + (k - C), region, &seen);
-                if (!got) __nanosleep(128);
-            }
-            locked_fresh = locked_fresh && got;
-        }
-        if (!__all_sync(kFull, locked_fresh)) {
-            for (int k = C + lane; k < F; k += 32) unlock_if(A.lock, base + (k - C), region);
-            if (lane == 0) report(st, ST_INTERNAL);
-            ok = 0;
-        }
-    }
+    // A fresh slot is locked from the start (no tet was ever in it), so whoever
+    // reads its tet reads it after this warp's release.
     if (ok) {
         // New tet k (on boundary facet (c, i), vertex i of c replaced by v) keeps
         // c's outside neighbour across facet i.  Its facet j != i is v plus the
@@ -1371,7 +1353,7 @@ __device__ int insert_async(int v, int t0, const Tables& T, const Workers& W, co
     __syncwarp();
     for (int k = lane; k < C; k += 32) unlock_if(A.lock, cav[k], region);
     if (ok)
-        for (int k = C + lane; k < F; k += 32) unlock_if(A.lock, base + (k - C), region);
+        for (int k = C + lane; k < F; k += 32) unlock_if(A.lock, base + (k - C), -1);
     if (lane == 0) {
         *nC += (unsigned long long)C;
         *nF += (unsigned long long)F;
@@ -1380,11 +1362,9 @@ __device__ int insert_async(int v, int t0, const Tables& T, const Workers& W, co
     return ok ? AI_DONE : AI_LEAVE;
 }
 
-/// Persistent warps over a level's chunks (set up by k_setup_level), or over
-/// the points a pass left, one worker each (k_setup_list).  kFast: the call-free
-/// variant; a point it cannot decide goes to A.leftover for the other variant.
-template <bool kFast>
-__global__ void __launch_bounds__(128, 8) k_insert_async(Tables T, Workers W, AsyncCtx A, Round R,
+/// The full variant: persistent warps over the points k_insert_groups left, one
+/// worker each (k_setup_list).
+__global__ void __launch_bounds__(128, 8) k_insert_full(Tables T, Workers W, AsyncCtx A, Round R,
                                                       const double* __restrict__ vx, int nslots) {
     const int lane = threadIdx.x & 31;
     const int slot = int((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
@@ -1410,7 +1390,7 @@ __global__ void __launch_bounds__(128, 8) k_insert_async(Tables T, Workers W, As
             for (int attempt = 0; attempt < kAsyncRetries && outcome == AI_RETRY; ++attempt) {
                 if (attempt > 0) __nanosleep(200u << min(attempt, 6));
                 const int t0 = __ldcg(T.vert_tet + (last >= 0 ? last : guide));
-                outcome = insert_async<kFast>(v, t0, T, W, A, vx, ex, R.status, slot, lane, &nC, &nF, ctr,
+                outcome = insert_full(v, t0, T, W, A, vx, ex, R.status, slot, lane, &nC, &nF, ctr,
                                               handed_tn[threadIdx.x >> 5]);
                 ++tries;
                 if (__ldcg(R.status) != 0) outcome = AI_LEAVE;
@@ -1575,6 +1555,60 @@ __global__ void k_set_exact(const int* __restrict__ smin, const int* __restrict_
     sp.emin = smin[s];
     sp.top = stop[s];
     ex[s] = (sp.exact_in_double(5, 7) && sp.exact_in_double(3, 3)) ? 1 : 0;
+}
+
+/// Puts every vertex but the first tets' in its level's list (items), and gives
+/// it the vertex its walk starts from: the nearest along the curve of the level
+/// before (`keys` sorted, the curve in their low bits; null: the one at the same
+/// fraction of that level), or in the first level its neighbour before it.
+__global__ void __launch_bounds__(256) k_level_items(const int32_t* __restrict__ vset, const int4* __restrict__ skips,
+                                                     const int* __restrict__ starts, int stride,
+                                                     const int* __restrict__ base, int nsets,
+                                                     const unsigned long long* __restrict__ keys, int curve_bits,
+                                                     const double* __restrict__ vx, int nv,
+                                                     int* __restrict__ items, int* __restrict__ guide) {
+    const unsigned long long mask = (1ull << curve_bits) - 1;
+    for (int v = int(blockIdx.x) * blockDim.x + threadIdx.x; v < nv; v += gridDim.x * blockDim.x) {
+        const int set = vset[v];
+        const int4 sk = skips[set];
+        if (sk.x < 0) continue;   // a flat set has no cells
+        const int* b = starts + int64_t(set) * stride;
+        int lev = stride - 1;
+        while (b[lev] > v) --lev;
+        const bool first_tet = v == sk.x || v == sk.y || v == sk.z || v == sk.w;
+        items[base[int64_t(lev) * nsets + set] + (v - b[lev])] = first_tet ? -1 : v;
+        int lo = lev, hi = b[lev];
+        while (lo > 0 && b[lo] == hi) --lo;   // the level before that has points: [b[lo], hi)
+        int g;
+        if (b[lo] == hi) {
+            g = v > hi ? v - 1 : -1;
+        } else if (keys) {
+            const unsigned long long k = keys[v] & mask;
+            int x = b[lo], y = hi;            // the first of [x, y) with key >= k
+            while (x < y) {
+                const int m = (x + y) >> 1;
+                if ((keys[m] & mask) < k) x = m + 1;
+                else y = m;
+            }
+            // The nearest of the kGuideReach vertices before and after it there.
+            const Pt p = vpt(vx, v);
+            double best = 1e300;
+            g = min(x, hi - 1);
+            for (int u = max(b[lo], x - kGuideReach); u < min(hi, x + kGuideReach); ++u) {
+                const Pt w = vpt(vx, u);
+                const double dx = w.x - p.x, dy = w.y - p.y, dz = w.z - p.z, d = dx * dx + dy * dy + dz * dz;
+                if (d < best) {
+                    best = d;
+                    g = u;
+                }
+            }
+        } else {
+            const int end = lev + 1 < stride ? b[lev + 1] : v + 1;
+            g = b[lo] + int(double(v - hi) / double(max(end - hi, 1)) * double(hi - b[lo]));
+            g = min(g, hi - 1);
+        }
+        guide[v] = g;
+    }
 }
 
 /// Launches one insertion kernel (0: k_cavity, 1: k_check, 2: k_restar) over
@@ -1912,6 +1946,7 @@ __global__ void k_init_tets(Tables T, const double* __restrict__ vx, const int4*
         for (int t = 0; t < 5; ++t) {
             T.tv(base + t) = tv[t];
             T.tn(base + t) = tn[t];
+            if (T.lock) T.lock[base + t] = 0;
         }
         T.vert_tet[v0] = base;
         T.vert_tet[v1] = base;
@@ -2240,6 +2275,8 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
     }
     const bool single = nsets == 1;
     const int N = int(n);
+    // Asynchronous insertion (k_insert_groups), or lockstep rounds only.
+    const bool use_async = opt.schedule != 1 && !(opt.chunk <= 0 && opt.split != 0);
     DevBuf<uint32_t> status;
     DevBuf<int64_t> d_off;
     D3G_TRY(status.alloc(4, s));
@@ -2269,6 +2306,7 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
     int growth = opt.level_growth;
     SetScan scan;
     D3G_TRY(scan_sets(d_xyz, d_off.p, nsets, n, scan, status.p + 1, s));
+    if (growth == 0 && use_async) growth = kGroupGrowth;
     if (growth == 0) {
         DevBuf<uint8_t> ex;
         D3G_TRY(ex.alloc(size_t(nsets), s));
@@ -2399,27 +2437,33 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
     // ---- tables ----
     Tables T;
     const int tets_per_vertex = opt.tet_capacity > 0 ? opt.tet_capacity : 8;
-    int64_t cap64 = int64_t(nv) * tets_per_vertex + 5 * int64_t(nsets) + 4096;
+    // (beyond it, room for the slots groups hold without using them: two blocks of
+    // kPoolSlots each, at most one group per kPoolSlots vertices)
+    int64_t cap64 = int64_t(nv) * tets_per_vertex + 5 * int64_t(nsets) + 4096 +
+                    (use_async ? 2 * std::min<int64_t>(nv, int64_t(kMaxGroups) * kPoolSlots) : 0);
     if (cap64 > (int64_t(1) << 29)) cap64 = int64_t(1) << 29;
     T.cap = int(cap64);
     T.walk_limit = opt.walk_limit > 0 ? opt.walk_limit : kWalkLimit;
     DevBuf<int4> rec;
     DevBuf<unsigned long long> claim;
-    DevBuf<int> fnew, vert_tet, tet_count;
+    DevBuf<int> fnew, vert_tet, tet_count, alock;
     D3G_TRY(rec.alloc(2 * size_t(T.cap), s));
-    D3G_TRY(claim.alloc(size_t(T.cap), s));
-    D3G_TRY(fnew.alloc(size_t(T.cap) * 4, s));
     D3G_TRY(vert_tet.alloc(size_t(nv), s));
     D3G_TRY(tet_count.alloc(1, s));
-    D3G_CUDA(cudaMemsetAsync(claim.p, 0xFF, sizeof(unsigned long long) * size_t(T.cap), s));
+    if (use_async) {
+        // A slot without a tet is locked until its first tet is written.
+        D3G_TRY(alock.alloc(size_t(T.cap), s));
+        D3G_CUDA(cudaMemsetAsync(alock.p, 0xFF, sizeof(int) * size_t(T.cap), s));
+    }
+    T.lock = alock.p;
     // Every slot holds in-range indices from the start (the asynchronous walk
     // may read a slot before its tet is written), and a vertex not inserted yet
     // has no tet.
     D3G_CUDA(cudaMemsetAsync(rec.p, 0, 2 * sizeof(int4) * size_t(T.cap), s));
     D3G_CUDA(cudaMemsetAsync(vert_tet.p, 0xFF, sizeof(int) * size_t(nv), s));
     T.rec = rec.p;
-    T.claim = claim.p;
-    T.fnew = fnew.p;
+    T.claim = nullptr;
+    T.fnew = nullptr;
     T.vert_tet = vert_tet.p;
     T.tet_count = tet_count.p;
     T.vset = vset.p;
@@ -2431,19 +2475,18 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
     D3G_TRY(set_exact.alloc(size_t(nsets), s));
     k_set_exact<<<grid_for(nsets, 128), 128, 0, s>>>(scan.span.p, scan.span.p + nsets, nsets, set_exact.p);
 
-    // ---- workers ----
+    // ---- levels ----
     // A level of s points goes into a triangulation of p earlier points.  Two
     // insertions collide when their regions (about 20 tets and their ring)
     // meet, so the useful number of simultaneous insertions grows with p, not
-    // with s: each level gets about p / alpha workers (a fixed chunk if the
-    // caller asks for one), each with a chunk of at least kMinChunk points.
-    // Several sets: their levels are aligned from the coarsest, and a round
-    // serves the workers of every set at once.
+    // with s: each level gets about p / alpha of them.  Several sets: their
+    // levels are aligned from the coarsest and served together.
+    const bool grow = opt.chunk <= 0 && opt.split != 0;   // the lockstep pool grows within levels
     const int alpha = opt.chunk < 0 ? -opt.chunk : 48;
     constexpr int kMinChunk = 16;
-    // Below one latency wave of the GPU (about 4K resident warps), a round costs
-    // the same whatever its size: then a denser pool (down to one worker per
-    // kAlphaSmall earlier points) trades more collisions for far fewer rounds.
+    // Below one latency wave of the GPU (about 4K resident warps), a level's time is
+    // its depth: then a denser pool (down to one worker per kAlphaSmall earlier
+    // points) trades more collisions for fewer insertions in a row.
     constexpr double kWaveWorkers = 4096.0;
     const double kAlphaSmall = opt.alpha_small > 0 ? double(opt.alpha_small) : double(alpha);
     auto level_chunk = [&](int64_t lb, int64_t le, double alpha_eff) -> int {
@@ -2499,120 +2542,34 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
         }
         return w;
     };
-    int maxw = 1;
-    {
-        std::vector<LevelDesc> tmp;
-        for (int lev = 0; lev < nlev; ++lev) maxw = std::max(maxw, level_descs(lev, level_alpha(lev), tmp));
-    }
-    // Room for the pool to grow within levels (at most one worker per 16 points).
-    const bool grow = opt.chunk <= 0 && opt.split != 0;
-    if (grow) maxw = std::max<int>(maxw, int(std::min<int64_t>(int64_t(nv) / 16, int64_t(1) << 18)));
-    // Asynchronous passes (see k_insert_async): a persistent grid of at most
-    // kAsyncWarps warps per level, the fast variant over the level's chunks,
-    // the full variant over what that leaves; the rounds finish the rest.
-    const bool use_async = opt.schedule != 1 && !grow;
-    constexpr int kAsyncWarps = kNumSMs * 32;   // resident at 64 registers a thread
-    // The passes over left points take all of them at once, one worker per
-    // point: the workers' own records are sized for that (wcap), the
-    // per-slot scratch (conflict region, boundary facets, staged tets) for the
-    // warps of a pass and the workers of a round, whichever is more (wslots).
-    const int wcap = use_async ? std::max<int>(maxw, int(std::min<int64_t>(nv, int64_t(1) << 20))) : maxw;
-    const int wslots = std::max(maxw, std::min(wcap, kAsyncWarps));
-    Workers W;
-    // Conflict-region scratch per worker (normal rounds and asynchronous
-    // passes) and per big-round slot; a caller's cavity_capacity lowers both.
-    const int cav_normal = opt.cavity_capacity > 0 ? std::min(kCavCap, int(opt.cavity_capacity)) : kCavCap;
-    const int cav_big = opt.cavity_capacity > 0 ? std::min(kBigCav, int(opt.cavity_capacity)) : kBigCav;
-    W.cav_cap = cav_normal;
-    W.fac_cap = 2 * cav_normal;
-    W.n = maxw;
-    DevBuf<int> wcur, wbeg, wend, wpos, wleft, wnwon, wlast, wguide, wstate, wncav, wnfac, wcav, wfac, counters;
-    DevBuf<int> set_p0, set_ins, set_w, set_split, nworkers;
-    DevBuf<int> wparked, wset, blist, bcount, bcav, bfac;
-    DevBuf<int4> bsv, bsn;
-    DevBuf<int4> wsv, wsn;
-    D3G_TRY(wcur.alloc(size_t(wcap), s));
-    D3G_TRY(wend.alloc(size_t(wcap), s));
-    D3G_TRY(wbeg.alloc(size_t(wcap), s));
-    D3G_TRY(wparked.alloc(size_t(wcap), s));
-    D3G_TRY(wset.alloc(size_t(wcap), s));
-    D3G_TRY(wpos.alloc(size_t(wcap), s));
-    D3G_TRY(wleft.alloc(size_t(wcap), s));
-    D3G_TRY(wnwon.alloc(size_t(wcap), s));
-    D3G_TRY(set_p0.alloc(size_t(nsets), s));
-    D3G_TRY(set_ins.alloc(size_t(nsets), s));
-    D3G_TRY(set_w.alloc(size_t(nsets), s));
-    D3G_TRY(set_split.alloc(size_t(nsets), s));
-    D3G_TRY(nworkers.alloc(1, s));
-    D3G_CUDA(cudaMemsetAsync(set_ins.p, 0, sizeof(int) * size_t(nsets), s));
-    SplitState SS{set_p0.p, set_ins.p, set_w.p, set_split.p, nworkers.p, maxw};
-    D3G_TRY(wlast.alloc(size_t(wcap), s));
-    D3G_TRY(wguide.alloc(size_t(wcap), s));
-    D3G_TRY(wstate.alloc(size_t(wcap), s));
-    D3G_TRY(wncav.alloc(size_t(wcap), s));
-    D3G_TRY(wnfac.alloc(size_t(wcap), s));
-    D3G_TRY(wcav.alloc(size_t(wslots) * W.cav_cap, s));
-    D3G_TRY(wfac.alloc(size_t(wslots) * W.fac_cap, s));
-    D3G_TRY(wsv.alloc(size_t(wslots) * W.fac_cap, s));
-    D3G_TRY(wsn.alloc(size_t(wslots) * W.fac_cap, s));
-    D3G_TRY(counters.alloc(4, s));
-    DevBuf<unsigned long long> sums, totals, steps;
+    // ---- counters and status ----
+    Round Rd;
+    DevBuf<int> counters;
+    DevBuf<unsigned long long> sums, totals, steps, pstats, astats;
     DevBuf<unsigned> dround;
+    D3G_TRY(counters.alloc(4, s));
     D3G_TRY(sums.alloc(2, s));
     D3G_TRY(steps.alloc(2, s));
-    D3G_CUDA(cudaMemsetAsync(steps.p, 0, 2 * sizeof(unsigned long long), s));
     D3G_TRY(totals.alloc(6, s));
+    D3G_TRY(pstats.alloc(4, s));
+    D3G_TRY(astats.alloc(7, s));
     D3G_TRY(dround.alloc(1, s));
+    D3G_CUDA(cudaMemsetAsync(steps.p, 0, 2 * sizeof(unsigned long long), s));
     D3G_CUDA(cudaMemsetAsync(sums.p, 0, 2 * sizeof(unsigned long long), s));
     D3G_CUDA(cudaMemsetAsync(totals.p, 0, 6 * sizeof(unsigned long long), s));
+    D3G_CUDA(cudaMemsetAsync(pstats.p, 0, 4 * sizeof(unsigned long long), s));
+    D3G_CUDA(cudaMemsetAsync(astats.p, 0, 7 * sizeof(unsigned long long), s));
     D3G_CUDA(cudaMemsetAsync(dround.p, 0, sizeof(unsigned), s));
-    W.cur = wcur.p;
-    W.end = wend.p;
-    W.beg = wbeg.p;
-    W.list = nullptr;
-    W.parked = wparked.p;
-    W.wset = wset.p;
-    W.skips = skips.p;
-    W.set_exact = set_exact.p;
-    W.pos = wpos.p;
-    W.left = wleft.p;
-    W.nwon = wnwon.p;
-    W.last = wlast.p;
-    W.guide = wguide.p;
-    W.state = wstate.p;
-    W.ncav = wncav.p;
-    W.nfac = wnfac.p;
-    W.cav = wcav.p;
-    W.fac = wfac.p;
-    W.st_v = wsv.p;
-    W.st_n = wsn.p;
-
-    Round Rd;
     Rd.counters = counters.p;
     Rd.sums = sums.p;
     Rd.totals = totals.p;
     Rd.steps = opt.timing ? steps.p : nullptr;
     Rd.round = dround.p;
     Rd.status = status.p;
-    DevBuf<unsigned long long> pstats;
-    D3G_TRY(pstats.alloc(4, s));
-    D3G_CUDA(cudaMemsetAsync(pstats.p, 0, 4 * sizeof(unsigned long long), s));
     Rd.pstats = pstats.p;
     const int max_rounds = opt.max_rounds > 0 ? opt.max_rounds : (1 << 20);
     int round = 0;
-    DevBuf<int> alock, anext, aleft, aleft2, anleft;
-    DevBuf<unsigned long long> astats, aekey;
-    if (use_async) {
-        D3G_TRY(aekey.alloc(size_t(std::min(wslots, kAsyncWarps)) * 3 * size_t(W.fac_cap), s));
-        D3G_TRY(alock.alloc(size_t(T.cap), s));
-        D3G_TRY(anext.alloc(1, s));
-        D3G_TRY(aleft.alloc(size_t(nv), s));
-        D3G_TRY(aleft2.alloc(size_t(nv), s));
-        D3G_TRY(anleft.alloc(2, s));
-        D3G_TRY(astats.alloc(7, s));
-        D3G_CUDA(cudaMemsetAsync(alock.p, 0, sizeof(int) * size_t(T.cap), s));
-        D3G_CUDA(cudaMemsetAsync(astats.p, 0, 7 * sizeof(unsigned long long), s));
-    }
+    long long to_rounds = 0;   // points the asynchronous passes left to the rounds
     // Structural self-check after each level (opt.validate): k_validate over
     // every tet slot and vertex; the first broken invariant ends the build.
     DevBuf<unsigned long long> vfail;
@@ -2623,7 +2580,7 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
         D3G_CUDA(cudaMemcpyAsync(&ntet_now, tet_count.p, sizeof ntet_now, cudaMemcpyDeviceToHost, s));
         D3G_CUDA(cudaStreamSynchronize(s));
         const int64_t threads = int64_t(ntet_now) + nv;
-        k_validate<<<grid_for(threads, 256, 1 << 30), 256, 0, s>>>(T, use_async ? alock.p : nullptr, ntet_now, nv,
+        k_validate<<<grid_for(threads, 256, 1 << 30), 256, 0, s>>>(T, alock.p, ntet_now, nv,
                                                                    status.p, vfail.p);
         D3G_CUDA(cudaGetLastError());
         unsigned long long rec = ~0ull;
@@ -2652,11 +2609,75 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
                 if (e[i]) cudaEventDestroy(e[i]);
         }
     } ev_guard{kev};
+    // ---- workers of the lockstep rounds and of the full variant ----
+    // Allocated when first needed: a build whose points all go in through
+    // k_insert_groups has none.
+    constexpr int kAsyncWarps = kNumSMs * 32;   // resident at 64 registers a thread
+    Workers W{};
+    Workers WB{};
+    // Conflict-region scratch per worker (normal rounds and the full variant) and
+    // per big-round slot; a caller's cavity_capacity lowers both.
+    const int cav_normal = opt.cavity_capacity > 0 ? std::min(kCavCap, int(opt.cavity_capacity)) : kCavCap;
+    const int cav_big = opt.cavity_capacity > 0 ? std::min(kBigCav, int(opt.cavity_capacity)) : kBigCav;
+    int maxw = 0, wcap = 0, wslots = 0;
+    DevBuf<int> wcur, wbeg, wend, wpos, wleft, wnwon, wlast, wguide, wstate, wncav, wnfac, wcav, wfac, wparked, wset;
+    DevBuf<int4> wsv, wsn;
+    DevBuf<unsigned long long> aekey;
+    // Records for `cap` workers; per-slot scratch for `slots` of them at a time.
+    auto alloc_workers = [&](int cap, int slots) -> int {
+        if (cap <= wcap && slots <= wslots) return D3G_OK;
+        wcap = std::max(wcap, cap);
+        wslots = std::max(wslots, slots);
+        W.cav_cap = cav_normal;
+        W.fac_cap = 2 * cav_normal;
+        DevBuf<int>* per_worker[] = {&wcur, &wbeg, &wend, &wpos, &wleft, &wnwon, &wlast, &wguide,
+                                     &wstate, &wncav, &wnfac, &wparked, &wset};
+        for (DevBuf<int>* d : per_worker) D3G_TRY(d->alloc(size_t(wcap), s));
+        D3G_TRY(wcav.alloc(size_t(wslots) * W.cav_cap, s));
+        D3G_TRY(wfac.alloc(size_t(wslots) * W.fac_cap, s));
+        D3G_TRY(wsv.alloc(size_t(wslots) * W.fac_cap, s));
+        D3G_TRY(wsn.alloc(size_t(wslots) * W.fac_cap, s));
+        if (use_async) D3G_TRY(aekey.alloc(size_t(std::min(wslots, kAsyncWarps)) * 3 * size_t(W.fac_cap), s));
+        W.cur = wcur.p;
+        W.end = wend.p;
+        W.beg = wbeg.p;
+        W.list = nullptr;
+        W.parked = wparked.p;
+        W.wset = wset.p;
+        W.skips = skips.p;
+        W.set_exact = set_exact.p;
+        W.pos = wpos.p;
+        W.left = wleft.p;
+        W.nwon = wnwon.p;
+        W.last = wlast.p;
+        W.guide = wguide.p;
+        W.state = wstate.p;
+        W.ncav = wncav.p;
+        W.nfac = wnfac.p;
+        W.cav = wcav.p;
+        W.fac = wfac.p;
+        W.st_v = wsv.p;
+        W.st_n = wsn.p;
+        return D3G_OK;
+    };
+    // The rounds' claims and restar scratch, likewise.
+    auto alloc_rounds = [&]() -> int {
+        if (claim.p) return D3G_OK;
+        D3G_TRY(claim.alloc(size_t(T.cap), s));
+        D3G_TRY(fnew.alloc(size_t(T.cap) * 4, s));
+        D3G_CUDA(cudaMemsetAsync(claim.p, 0xFF, sizeof(unsigned long long) * size_t(T.cap), s));
+        T.claim = claim.p;
+        T.fnew = fnew.p;
+        return D3G_OK;
+    };
+    DevBuf<int> set_p0, set_ins, set_w, set_split, nworkers;
+    SplitState SS{};
+    DevBuf<int> blist, bcount, bcav, bfac;
+    DevBuf<int4> bsv, bsn;
     // Big rounds: workers whose conflict region outgrew the normal scratch.
-    Workers WB = W;
     auto big_rounds = [&]() -> int {
-        if (!blist.p) {
-            D3G_TRY(blist.alloc(size_t(maxw), s));
+        if (blist.n < size_t(wcap)) D3G_TRY(blist.alloc(size_t(wcap), s));
+        if (!bcount.p) {
             D3G_TRY(bcount.alloc(1, s));
             D3G_TRY(bcav.alloc(size_t(kBigSlots) * cav_big, s));
             D3G_TRY(bfac.alloc(size_t(kBigSlots) * 2 * cav_big, s));
@@ -2710,256 +2731,402 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
             }
         }
     };
-    std::vector<LevelDesc> descs;
-    std::vector<int> hp0(static_cast<size_t>(nsets)), hw(static_cast<size_t>(nsets));
-    for (int lev = 0; lev < nlev; ++lev) {
-        const double alpha_eff = level_alpha(lev);
-        W.n = level_descs(lev, alpha_eff, descs);
-        if (W.n == 0) continue;
-        char level_name[32];
-        std::snprintf(level_name, sizeof level_name, "d3g.level %d", lev);
-        NvtxRange nvtx_level(level_name);
-        std::fill(hp0.begin(), hp0.end(), 0);
-        std::fill(hw.begin(), hw.end(), 0);
-        for (size_t i = 0; i < descs.size(); ++i) {
-            const LevelDesc& d = descs[i];
-            hp0[size_t(d.set)] = d.lb - hvoff[size_t(d.set)];
-            hw[size_t(d.set)] = (i + 1 < descs.size() ? descs[i + 1].w0 : W.n) - d.w0;
+    double split_alpha = alpha;
+    int lanes = opt.lanes > 0 ? opt.lanes : 32;
+    auto one_round = [&](bool timed) {
+        k_round_begin<<<1, 1, 0, s>>>(Rd);
+        if (timed) cudaEventRecord(kev[0], s);
+        launch_insertion(lanes, 0, T, W, Rd, vx.p, s);
+        if (timed) cudaEventRecord(kev[1], s);
+        launch_insertion(lanes, 1, T, W, Rd, vx.p, s);
+        if (timed) cudaEventRecord(kev[2], s);
+        launch_insertion(lanes, 2, T, W, Rd, vx.p, s);
+        if (timed) cudaEventRecord(kev[3], s);
+        k_round_end<<<1, 1, 0, s>>>(Rd);
+    };
+    // Rounds go out in batches captured as one CUDA graph; the host looks at
+    // the counters once per batch.  Rounds after the level is done find no
+    // active worker and return at once.
+    cudaGraphExec_t gexec = nullptr;
+    struct GraphGuard {
+        cudaGraphExec_t* g;
+        ~GraphGuard() {
+            if (*g) cudaGraphExecDestroy(*g);
         }
-        D3G_CUDA(cudaMemcpyAsync(set_p0.p, hp0.data(), sizeof(int) * size_t(nsets), cudaMemcpyHostToDevice, s));
-        D3G_CUDA(cudaMemcpyAsync(set_w.p, hw.data(), sizeof(int) * size_t(nsets), cudaMemcpyHostToDevice, s));
-        k_set_int<<<1, 1, 0, s>>>(nworkers.p, W.n);
-        const int round0 = round;
-        long long won = 0, attempts = 0;
-        long long won_before = 0, att_before = 0;
-        {
-            unsigned long long ht0[2];
-            D3G_CUDA(cudaMemcpyAsync(ht0, totals.p, sizeof ht0, cudaMemcpyDeviceToHost, s));
-            D3G_CUDA(cudaStreamSynchronize(s));
-            won_before = (long long)ht0[0];
-            att_before = (long long)ht0[1];
+    } graph_guard{&gexec};
+    auto capture = [&]() -> int {
+        if (gexec) cudaGraphExecDestroy(gexec);
+        gexec = nullptr;
+        if (opt.timing) return D3G_OK;
+        cudaGraph_t graph = nullptr;
+        D3G_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+        for (int r = 0; r < kRoundsPerBatch; ++r) one_round(false);
+        D3G_CUDA(cudaStreamEndCapture(s, &graph));
+        const cudaError_t ge = cudaGraphInstantiate(&gexec, graph, 0);
+        cudaGraphDestroy(graph);
+        if (ge != cudaSuccess) {
+            set_error(std::string("cudaGraphInstantiate: ") + cudaGetErrorString(ge));
+            return D3G_ERR_CUDA;
         }
-        cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-        if (trace) {
-            cudaEventCreate(&ev0);
-            cudaEventCreate(&ev1);
-            cudaEventRecord(ev0, s);
+        return D3G_OK;
+    };
+    auto run_rounds = [&]() -> int {
+    D3G_TRY(capture());
+    for (;;) {
+        const int batch = opt.timing ? 1 : kRoundsPerBatch;
+        round += batch;
+        if (round > max_rounds) {
+            set_error("d3g_build: insertion round limit reached");
+            return D3G_ERR_ROUND_LIMIT;
         }
-        DevBuf<LevelDesc> ddesc;
-        D3G_TRY(ddesc.alloc(descs.size(), s));
-        D3G_CUDA(cudaMemcpyAsync(ddesc.p, descs.data(), sizeof(LevelDesc) * descs.size(), cudaMemcpyHostToDevice, s));
-        k_setup_level<<<grid_for(W.n, 128, 1 << 30), 128, 0, s>>>(W, ddesc.p, int(descs.size()));
-        int lanes = opt.lanes > 0 ? opt.lanes : 32;
-        auto one_round = [&](bool timed) {
-            k_round_begin<<<1, 1, 0, s>>>(Rd);
-            if (timed) cudaEventRecord(kev[0], s);
-            launch_insertion(lanes, 0, T, W, Rd, vx.p, s);
-            if (timed) cudaEventRecord(kev[1], s);
-            launch_insertion(lanes, 1, T, W, Rd, vx.p, s);
-            if (timed) cudaEventRecord(kev[2], s);
-            launch_insertion(lanes, 2, T, W, Rd, vx.p, s);
-            if (timed) cudaEventRecord(kev[3], s);
-            k_round_end<<<1, 1, 0, s>>>(Rd);
-        };
-        // Rounds go out in batches captured as one CUDA graph; the host looks at
-        // the counters once per batch.  Rounds after the level is done find no
-        // active worker and return at once.
-        cudaGraphExec_t gexec = nullptr;
-        struct GraphGuard {
-            cudaGraphExec_t* g;
-            ~GraphGuard() {
-                if (*g) cudaGraphExecDestroy(*g);
+        if (opt.timing) one_round(true);
+        else D3G_CUDA(cudaGraphLaunch(gexec, s));
+        if (grow) {
+            D3G_CUDA(cudaMemsetAsync(set_ins.p, 0, sizeof(int) * size_t(nsets), s));
+            k_count_wins<<<grid_for(W.n, 128, 1 << 30), 128, 0, s>>>(W, SS);
+            k_plan_split<<<grid_for(nsets, 128), 128, 0, s>>>(SS, nsets, split_alpha);
+            k_split<<<grid_for(W.n, 128, 1 << 30), 128, 0, s>>>(W, SS, W.n);
+        }
+        unsigned long long ht[6];
+        uint32_t hs = 0;
+        int hn = W.n;
+        D3G_CUDA(cudaMemcpyAsync(ht, totals.p, sizeof ht, cudaMemcpyDeviceToHost, s));
+        D3G_CUDA(cudaMemcpyAsync(&hs, status.p, sizeof hs, cudaMemcpyDeviceToHost, s));
+        if (grow) D3G_CUDA(cudaMemcpyAsync(&hn, nworkers.p, sizeof hn, cudaMemcpyDeviceToHost, s));
+        D3G_CUDA(cudaStreamSynchronize(s));
+        hn = std::min(hn, maxw);
+        if (hn != W.n) {
+            // The pool grew: the next batches serve the new workers too.
+            W.n = hn;
+            k_set_int<<<1, 1, 0, s>>>(nworkers.p, W.n);
+            D3G_TRY(capture());
+        }
+        if (hs != 0) {
+            const int st = status_from_bits(hs);
+            if (st == D3G_ERR_OOM) set_error("d3g_build: tet table full");
+            return st;
+        }
+        if (ht[4]) {
+            set_error("d3g_build: an insertion round made no progress");
+            return D3G_ERR_INTERNAL;
+        }
+        if (opt.timing) {
+            float a = 0.f, b2 = 0.f, c = 0.f;
+            cudaEventElapsedTime(&a, kev[0], kev[1]);
+            cudaEventElapsedTime(&b2, kev[1], kev[2]);
+            cudaEventElapsedTime(&c, kev[2], kev[3]);
+            R.stats.ms_cavity += a;
+            R.stats.ms_check += b2;
+            R.stats.ms_restar += c;
+            R.stats.launches_cavity += 1;
+        }
+        if (ht[5] != 0) continue;
+        if (ht[3] == 0) break;
+        // Only parked workers are left: serve them in big rounds, up to
+        // kBigSlots at a time, each until its point is in.
+        D3G_TRY(big_rounds());
+    }
+    return D3G_OK;
+    };
+    // Lockstep rounds over every level (schedule = 1, or a pool that grows within
+    // levels).
+    auto run_lockstep = [&]() -> int {
+        std::vector<LevelDesc> descs;
+        maxw = 1;
+        for (int lev = 0; lev < nlev; ++lev) maxw = std::max(maxw, level_descs(lev, level_alpha(lev), descs));
+        // Room for the pool to grow within levels (at most one worker per 16 points).
+        if (grow) maxw = std::max<int>(maxw, int(std::min<int64_t>(int64_t(nv) / 16, int64_t(1) << 18)));
+        D3G_TRY(alloc_workers(maxw, maxw));
+        D3G_TRY(alloc_rounds());
+        D3G_TRY(set_p0.alloc(size_t(nsets), s));
+        D3G_TRY(set_ins.alloc(size_t(nsets), s));
+        D3G_TRY(set_w.alloc(size_t(nsets), s));
+        D3G_TRY(set_split.alloc(size_t(nsets), s));
+        D3G_TRY(nworkers.alloc(1, s));
+        D3G_CUDA(cudaMemsetAsync(set_ins.p, 0, sizeof(int) * size_t(nsets), s));
+        SS = SplitState{set_p0.p, set_ins.p, set_w.p, set_split.p, nworkers.p, maxw};
+        std::vector<int> hp0(static_cast<size_t>(nsets)), hw(static_cast<size_t>(nsets));
+        for (int lev = 0; lev < nlev; ++lev) {
+            split_alpha = level_alpha(lev);
+            W.n = level_descs(lev, split_alpha, descs);
+            if (W.n == 0) continue;
+            char level_name[32];
+            std::snprintf(level_name, sizeof level_name, "d3g.level %d", lev);
+            NvtxRange nvtx_level(level_name);
+            std::fill(hp0.begin(), hp0.end(), 0);
+            std::fill(hw.begin(), hw.end(), 0);
+            for (size_t i = 0; i < descs.size(); ++i) {
+                const LevelDesc& d = descs[i];
+                hp0[size_t(d.set)] = d.lb - hvoff[size_t(d.set)];
+                hw[size_t(d.set)] = (i + 1 < descs.size() ? descs[i + 1].w0 : W.n) - d.w0;
             }
-        } graph_guard{&gexec};
-        auto capture = [&]() -> int {
-            if (gexec) cudaGraphExecDestroy(gexec);
-            gexec = nullptr;
-            if (opt.timing) return D3G_OK;
-            cudaGraph_t graph = nullptr;
-            D3G_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-            for (int r = 0; r < kRoundsPerBatch; ++r) one_round(false);
-            D3G_CUDA(cudaStreamEndCapture(s, &graph));
-            const cudaError_t ge = cudaGraphInstantiate(&gexec, graph, 0);
-            cudaGraphDestroy(graph);
-            if (ge != cudaSuccess) {
-                set_error(std::string("cudaGraphInstantiate: ") + cudaGetErrorString(ge));
-                return D3G_ERR_CUDA;
+            D3G_CUDA(cudaMemcpyAsync(set_p0.p, hp0.data(), sizeof(int) * size_t(nsets), cudaMemcpyHostToDevice, s));
+            D3G_CUDA(cudaMemcpyAsync(set_w.p, hw.data(), sizeof(int) * size_t(nsets), cudaMemcpyHostToDevice, s));
+            k_set_int<<<1, 1, 0, s>>>(nworkers.p, W.n);
+            DevBuf<LevelDesc> ddesc;
+            D3G_TRY(ddesc.alloc(descs.size(), s));
+            D3G_CUDA(cudaMemcpyAsync(ddesc.p, descs.data(), sizeof(LevelDesc) * descs.size(),
+                                     cudaMemcpyHostToDevice, s));
+            k_setup_level<<<grid_for(W.n, 128, 1 << 30), 128, 0, s>>>(W, ddesc.p, int(descs.size()));
+            D3G_TRY(run_rounds());
+            if (opt.validate) D3G_TRY(validate_tables("after", lev));
+            if (trace) fprintf(stderr, "d3g level %d sets %zu workers %d rounds so far %d\n", lev, descs.size(), W.n, round);
+        }
+        return D3G_OK;
+    };
+    // The points k_insert_groups left (tests its filters cannot decide, regions
+    // beyond its scratch, persistent conflicts) through the full variant, one
+    // worker per point, all of them at once, again while a pass inserts at least a
+    // quarter of its points; what that leaves through the rounds.
+    DevBuf<int> aleft, aleft2, actl;
+    auto finish_points = [&](int* list, int count) -> int {
+        if (count <= 0) return D3G_OK;
+        D3G_TRY(alloc_workers(std::min(count, 1 << 20), std::min(count, kAsyncWarps)));
+        if (!aleft.p) {
+            D3G_TRY(aleft.alloc(size_t(nv), s));
+            D3G_TRY(aleft2.alloc(size_t(nv), s));
+            D3G_TRY(actl.alloc(2, s));
+        }
+        int* cur = list;
+        int* nxt = aleft.p;
+        int ncur = count;
+        for (int pass = 0; ncur > 0 && pass < kLeftPasses; ++pass) {
+            int nnext = 0;
+            D3G_CUDA(cudaMemsetAsync(actl.p + 1, 0, sizeof(int), s));
+            for (int off = 0; off < ncur; off += wcap) {
+                W.n = std::min(wcap, ncur - off);
+                k_setup_list<<<grid_for(W.n, 128, 1 << 30), 128, 0, s>>>(W, cur + off, W.n, vset.p, voff.p, T.vert_tet);
+                // Workers go out in a scattered order (stride coprime with their count,
+                // near its golden ratio), so that those taken at the same time lie far
+                // apart along the curve.
+                int64_t stride = std::max<int64_t>(1, int64_t(double(W.n) * 0.6180339887));
+                while (std::gcd(stride, int64_t(W.n)) != 1) ++stride;
+                D3G_CUDA(cudaMemsetAsync(actl.p, 0, sizeof(int), s));
+                const int warps = std::min(W.n, kAsyncWarps);
+                if (warps > wslots) {
+                    set_error("d3g_build: asynchronous pass wider than its scratch");
+                    return D3G_ERR_INTERNAL;
+                }
+                AsyncCtx A{alock.p, actl.p, nxt, actl.p + 1, stride, W.n, aekey.p, astats.p};
+                k_insert_full<<<unsigned((int64_t(warps) * 32 + 127) / 128), 128, 0, s>>>(T, W, A, Rd, vx.p, warps);
+                D3G_CUDA(cudaGetLastError());
+                R.stats.launches_async += 1;
             }
-            return D3G_OK;
-        };
-        auto run_rounds = [&]() -> int {
-        D3G_TRY(capture());
-        for (;;) {
-            const int batch = opt.timing ? 1 : kRoundsPerBatch;
-            round += batch;
-            if (round > max_rounds) {
-                set_error("d3g_build: insertion round limit reached");
-                return D3G_ERR_ROUND_LIMIT;
-            }
-            if (opt.timing) one_round(true);
-            else D3G_CUDA(cudaGraphLaunch(gexec, s));
-            if (grow) {
-                D3G_CUDA(cudaMemsetAsync(set_ins.p, 0, sizeof(int) * size_t(nsets), s));
-                k_count_wins<<<grid_for(W.n, 128, 1 << 30), 128, 0, s>>>(W, SS);
-                k_plan_split<<<grid_for(nsets, 128), 128, 0, s>>>(SS, nsets, alpha_eff);
-                k_split<<<grid_for(W.n, 128, 1 << 30), 128, 0, s>>>(W, SS, W.n);
-            }
-            unsigned long long ht[6];
             uint32_t hs = 0;
-            int hn = W.n;
-            D3G_CUDA(cudaMemcpyAsync(ht, totals.p, sizeof ht, cudaMemcpyDeviceToHost, s));
+            D3G_CUDA(cudaMemcpyAsync(&nnext, actl.p + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
             D3G_CUDA(cudaMemcpyAsync(&hs, status.p, sizeof hs, cudaMemcpyDeviceToHost, s));
-            if (grow) D3G_CUDA(cudaMemcpyAsync(&hn, nworkers.p, sizeof hn, cudaMemcpyDeviceToHost, s));
             D3G_CUDA(cudaStreamSynchronize(s));
-            hn = std::min(hn, maxw);
-            if (hn != W.n) {
-                // The pool grew: the next batches serve the new workers too.
-                W.n = hn;
-                k_set_int<<<1, 1, 0, s>>>(nworkers.p, W.n);
-                D3G_TRY(capture());
-            }
+            if (trace) fprintf(stderr, "d3g full pass over %d points left %d\n", ncur, nnext);
             if (hs != 0) {
                 const int st = status_from_bits(hs);
                 if (st == D3G_ERR_OOM) set_error("d3g_build: tet table full");
                 return st;
             }
-            if (ht[4]) {
-                set_error("d3g_build: an insertion round made no progress");
-                return D3G_ERR_INTERNAL;
-            }
-            if (opt.timing) {
-                float a = 0.f, b2 = 0.f, c = 0.f;
-                cudaEventElapsedTime(&a, kev[0], kev[1]);
-                cudaEventElapsedTime(&b2, kev[1], kev[2]);
-                cudaEventElapsedTime(&c, kev[2], kev[3]);
-                R.stats.ms_cavity += a;
-                R.stats.ms_check += b2;
-                R.stats.ms_restar += c;
-                R.stats.launches_cavity += 1;
-            }
-            won = (long long)ht[0] - won_before;
-            attempts = (long long)ht[1] - att_before;
-            if (ht[5] != 0) continue;
-            if (ht[3] == 0) break;
-            // Only parked workers are left: serve them in big rounds, up to
-            // kBigSlots at a time, each until its point is in.
-            D3G_TRY(big_rounds());
+            const bool slow = int64_t(ncur - nnext) * 4 < int64_t(ncur);
+            cur = nxt;
+            nxt = cur == aleft.p ? aleft2.p : aleft.p;
+            ncur = nnext;
+            if (slow) break;
+        }
+        if (ncur > 0) D3G_TRY(alloc_rounds());
+        to_rounds += ncur;
+        for (int off = 0; off < ncur; off += wslots) {
+            maxw = W.n = std::min(wslots, ncur - off);
+            k_setup_list<<<grid_for(W.n, 128, 1 << 30), 128, 0, s>>>(W, cur + off, W.n, vset.p, voff.p, T.vert_tet);
+            D3G_TRY(run_rounds());
         }
         return D3G_OK;
+    };
+    // Every level through k_insert_groups, launched one after another with no
+    // look at the results in between: what a level leaves goes in at the end (the
+    // order of insertions does not matter).
+    auto run_async = [&]() -> int {
+        // Items: level by level, each set's vertices of the level together.
+        std::vector<int> ctl(size_t(2) * size_t(nlev) + size_t(nlev) * size_t(nsets), 0);
+        int* m_of = ctl.data();
+        int* first_of = ctl.data() + nlev;
+        int* base = ctl.data() + 2 * nlev;
+        int total = 0;
+        std::vector<int64_t> groups_of(static_cast<size_t>(nlev), 0);
+        std::vector<int> sets_of(static_cast<size_t>(nlev), 0);
+        for (int lev = 0; lev < nlev; ++lev) {
+            const double alpha_eff = level_alpha(lev);
+            first_of[lev] = total;
+            for (int st = 0; st < nsets; ++st) {
+                const std::vector<int>& L = levels[size_t(st)];
+                if (int(L.size()) - 1 <= lev) continue;
+                const int cnt = L[size_t(lev) + 1] - L[size_t(lev)];
+                base[size_t(lev) * size_t(nsets) + size_t(st)] = total;
+                total += cnt;
+                if (cnt <= 0) continue;
+                sets_of[size_t(lev)] += 1;
+                const int64_t w = opt.chunk > 0 ? (cnt + opt.chunk - 1) / opt.chunk
+                                                : std::max<int64_t>(1, int64_t(double(L[size_t(lev)]) / alpha_eff));
+                groups_of[size_t(lev)] += std::min<int64_t>(w, cnt);
+            }
+            m_of[lev] = total - first_of[lev];
+        }
+        DevBuf<int> dctl, items, guide, hint, lstart, defer, left[2], cnt;
+        DevBuf<int4> pool;
+        D3G_TRY(dctl.alloc(ctl.size(), s));
+        D3G_TRY(items.alloc(size_t(std::max(total, 1)), s));
+        D3G_TRY(guide.alloc(size_t(nv), s));
+        D3G_TRY(hint.alloc(size_t(nv), s));
+        D3G_CUDA(cudaMemsetAsync(hint.p, 0xFF, sizeof(int) * size_t(nv), s));
+        D3G_TRY(defer.alloc(size_t(nv), s));
+        for (auto& l : left) D3G_TRY(l.alloc(size_t(nv), s));
+        D3G_TRY(pool.alloc(size_t(kMaxGroups), s));
+        D3G_TRY(cnt.alloc(size_t(4) * size_t(nlev + kLastPasses + 1) + 1, s));
+        D3G_CUDA(cudaMemcpyAsync(dctl.p, ctl.data(), sizeof(int) * ctl.size(), cudaMemcpyHostToDevice, s));
+        D3G_CUDA(cudaMemsetAsync(pool.p, 0, sizeof(int4) * size_t(kMaxGroups), s));
+        D3G_CUDA(cudaMemsetAsync(cnt.p, 0, sizeof(int) * cnt.n, s));
+        const int* starts = own.level_start.p;
+        int start_stride = own.levels;
+        std::vector<int> hstart;
+        if (!own.ok) {
+            start_stride = nlev;
+            hstart.resize(size_t(nsets) * size_t(nlev) + 1);
+            for (int st = 0; st < nsets; ++st)
+                for (int lev = 0; lev < nlev; ++lev) {
+                    const std::vector<int>& L = levels[size_t(st)];
+                    const int k = std::min(lev, std::max(int(L.size()) - 1, 0));
+                    hstart[size_t(st) * size_t(nlev) + size_t(lev)] = hvoff[size_t(st)] + (L.empty() ? 0 : L[size_t(k)]);
+                }
+            hstart.back() = nv;
+            D3G_TRY(lstart.alloc(hstart.size(), s));
+            D3G_CUDA(cudaMemcpyAsync(lstart.p, hstart.data(), sizeof(int) * hstart.size(), cudaMemcpyHostToDevice, s));
+            starts = lstart.p;
+        }
+        k_level_items<<<grid_for(nv, 256), 256, 0, s>>>(vset.p, skips.p, starts, start_stride, dctl.p + 2 * nlev, nsets,
+                                                        own.ok ? own.keys.p : nullptr, own.curve_bits, vx.p, nv,
+                                                        items.p, guide.p);
+        own.keys.release();
+        // Per level: the queue head, the points left, the head of the pass over those.
+        auto head_of = [&](int lev) { return cnt.p + 4 * lev; };
+        auto n_left_of = [&](int lev) { return cnt.p + 4 * lev + 1; };
+        auto left_of = [&](int lev) { return left[lev & 1].p; };
+        int* n_defer = cnt.p + (cnt.n - 1);
+        GroupArgs A{};
+        A.lock = alock.p;
+        A.guide = guide.p;
+        A.hint = hint.p;
+        A.defer = defer.p;
+        A.n_defer = n_defer;
+        A.pool = pool.p;
+        A.skips = skips.p;
+        A.set_exact = set_exact.p;
+        A.voff = voff.p;
+        A.stats = astats.p;
+        A.cavity = cav_normal;
+        auto launch = [&](int G, int ngroups) {
+            // At most one group per kPoolSlots vertices, so that the slots groups hold
+            // without using them stay within the table's room for them.
+            A.ngroups = std::max(1, std::min({ngroups, kNumSMs * kGroupBlocks * (kGroupThreads / G), nv / kPoolSlots}));
+            const unsigned grid = unsigned((A.ngroups + kGroupThreads / G - 1) / (kGroupThreads / G));
+            if (G == 8) k_insert_groups<8><<<grid, kGroupThreads, 0, s>>>(T, A, Rd, vx.p);
+            else if (G == 16) k_insert_groups<16><<<grid, kGroupThreads, 0, s>>>(T, A, Rd, vx.p);
+            else k_insert_groups<32><<<grid, kGroupThreads, 0, s>>>(T, A, Rd, vx.p);
+            R.stats.launches_async += 1;
         };
-        long long async_left = -1, deferred = -1;
-        if (use_async) {
-            // One asynchronous pass: a persistent grid over the workers W
-            // (level chunks, or one leftover point each), writing the points it
-            // leaves to `left` / `nleft_d`; their count goes to *nleft_out.
-            auto async_pass = [&](bool fast, int nw, int* left, int* nleft_d,
-                                  int* nleft_out) -> int {
-                // The chunks go out in a scattered order (stride coprime with the
-                // chunk count, near the golden ratio of it), so that chunks taken
-                // at the same time lie far apart along the curve.
-                int64_t stride = std::max<int64_t>(1, int64_t(double(nw) * 0.6180339887));
-                while (std::gcd(stride, int64_t(nw)) != 1) ++stride;
-                D3G_CUDA(cudaMemsetAsync(anext.p, 0, sizeof(int), s));
-                AsyncCtx A{alock.p, anext.p, left, nleft_d, stride, nw, aekey.p, astats.p};
-                const int warps = std::min(nw, kAsyncWarps);
-                if (warps > wslots) {
-                    set_error("d3g_build: asynchronous pass wider than its scratch");
-                    return D3G_ERR_INTERNAL;
+        auto left_pass = [&](int lev, int ngroups) {
+            A.items = left_of(lev);
+            A.n_items = n_left_of(lev);
+            A.next = head_of(lev) + 2;
+            A.left = left_of(lev + 1);
+            A.n_left = n_left_of(lev + 1);
+            launch(32, ngroups);
+        };
+        if (opt.timing) cudaEventRecord(kev[0], s);
+        for (int lev = 0; lev < nlev; ++lev) {
+            char level_name[32];
+            std::snprintf(level_name, sizeof level_name, "d3g.level %d", lev);
+            NvtxRange nvtx_level(level_name);
+            cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+            if (trace) {
+                cudaEventCreate(&ev0);
+                cudaEventCreate(&ev1);
+                cudaEventRecord(ev0, s);
+            }
+            const int G = group_lanes(groups_of[size_t(lev)]);
+            A.items = items.p + first_of[lev];
+            A.n_items = dctl.p + lev;
+            A.next = head_of(lev);
+            // What narrower groups leave goes to wider ones at once; what those leave
+            // (points in each other's way) waits for the next level's pass.
+            A.left = left_of(G < 32 ? lev : lev + 1);
+            A.n_left = n_left_of(G < 32 ? lev : lev + 1);
+            // (The first level grows from one tet: there the guides are nearer.)
+            if (lev > 0) k_locate<<<grid_for(m_of[lev], 128), 128, 0, s>>>(T, A, vx.p);
+            launch(G, int(std::min<int64_t>(groups_of[size_t(lev)], 1 << 24)));
+            if (lev > 0 || G < 32) left_pass(lev, kNumSMs * (kGroupThreads / 32));
+            D3G_CUDA(cudaGetLastError());
+            if (trace) {
+                cudaEventRecord(ev1, s);
+                cudaEventSynchronize(ev1);
+                float ms = 0.f;
+                cudaEventElapsedTime(&ms, ev0, ev1);
+                int c[4] = {0, 0, 0, 0}, nd = 0;
+                unsigned long long as[7], ht[2];
+                cudaMemcpy(c, cnt.p + 4 * lev, sizeof c, cudaMemcpyDeviceToHost);
+                cudaMemcpy(&nd, n_defer, sizeof nd, cudaMemcpyDeviceToHost);
+                cudaMemcpy(as, astats.p, sizeof as, cudaMemcpyDeviceToHost);
+                cudaMemcpy(ht, totals.p, sizeof ht, cudaMemcpyDeviceToHost);
+                fprintf(stderr, "d3g level %d sets %d points %d groups %d of %d lanes: left to wider groups %d, "
+                        "deferred so far %d, %.3f ms | inserted %llu attempts %llu lock-conflicts %llu walk-restarts %llu "
+                        "bad-seeds %llu too-big %llu left %llu undecided %llu\n",
+                        lev, sets_of[size_t(lev)], m_of[lev], int(std::min<int64_t>(groups_of[size_t(lev)], kMaxGroups)),
+                        G, c[1], nd, ms, ht[0], ht[1], as[0], as[1], as[2], as[3], as[4], as[6]);
+                cudaEventDestroy(ev0);
+                cudaEventDestroy(ev1);
+            }
+            if (lev == nlev - 1) {
+                // The points still left, with fewer and fewer groups in the way of one another;
+                // the last pass hands what remains to the full variant.
+                for (int k = 0; k < kLastPasses; ++k) {
+                    if (k == kLastPasses - 1) break;
+                    left_pass(nlev + k, kNumSMs * (kGroupThreads / 32) >> (2 * k));
                 }
-                const unsigned grid = unsigned((int64_t(warps) * 32 + 127) / 128);
-                unsigned long long won0 = 0;
-                D3G_CUDA(cudaMemcpyAsync(&won0, totals.p, sizeof won0, cudaMemcpyDeviceToHost, s));
-                if (opt.timing) cudaEventRecord(kev[0], s);
-                if (fast) k_insert_async<true><<<grid, 128, 0, s>>>(T, W, A, Rd, vx.p, warps);
-                else k_insert_async<false><<<grid, 128, 0, s>>>(T, W, A, Rd, vx.p, warps);
-                D3G_CUDA(cudaGetLastError());
-                if (opt.timing) cudaEventRecord(kev[1], s);
+                A.items = left_of(nlev + kLastPasses - 1);
+                A.n_items = n_left_of(nlev + kLastPasses - 1);
+                A.next = head_of(nlev + kLastPasses - 1) + 2;
+                A.left = defer.p;
+                A.n_left = n_defer;
+                launch(32, 16);   // few in the way of one another
+            }
+            if (opt.validate || lev == nlev - 1) {
+                int nd = 0;
                 uint32_t hs = 0;
-                unsigned long long won1 = 0;
-                D3G_CUDA(cudaMemcpyAsync(nleft_out, nleft_d, sizeof(int), cudaMemcpyDeviceToHost, s));
+                if (opt.timing) cudaEventRecord(kev[1], s);
+                D3G_CUDA(cudaMemcpyAsync(&nd, n_defer, sizeof nd, cudaMemcpyDeviceToHost, s));
                 D3G_CUDA(cudaMemcpyAsync(&hs, status.p, sizeof hs, cudaMemcpyDeviceToHost, s));
-                D3G_CUDA(cudaMemcpyAsync(&won1, totals.p, sizeof won1, cudaMemcpyDeviceToHost, s));
                 D3G_CUDA(cudaStreamSynchronize(s));
-                R.stats.launches_async += 1;
-                R.stats.async_inserted += int64_t(won1 - won0);
-                if (trace)
-                    fprintf(stderr, "d3g level %d async pass %s chunks-or-points %d inserted %llu left %d\n", lev,
-                            fast ? "fast" : "full", nw, won1 - won0, *nleft_out);
-                if (opt.timing) {
-                    float am = 0.f;
-                    cudaEventElapsedTime(&am, kev[0], kev[1]);
-                    R.stats.ms_async += am;
-                }
                 if (hs != 0) {
                     const int st = status_from_bits(hs);
                     if (st == D3G_ERR_OOM) set_error("d3g_build: tet table full");
                     return st;
                 }
-                return D3G_OK;
-            };
-            // The level's chunks through the fast variant; what it deferred or
-            // left (undecided tests, lock conflicts, regions too big) through
-            // the full variant, one worker per point, all of them at once,
-            // again while a pass inserts at least a quarter of its points; what
-            // that leaves through the rounds, maxw points at a time.
-            int nleft = 0;
-            D3G_CUDA(cudaMemsetAsync(anleft.p, 0, 2 * sizeof(int), s));
-            D3G_TRY(async_pass(true, W.n, aleft.p, anleft.p, &nleft));
-            deferred = nleft;
-            int* cur = aleft.p;
-            int* nxt = aleft2.p;
-            int ncur = nleft;
-            for (int pass = 0; ncur > 0 && pass < kLeftPasses; ++pass) {
-                int nnext = 0;
-                D3G_CUDA(cudaMemsetAsync(anleft.p + 1, 0, sizeof(int), s));
-                for (int off = 0; off < ncur; off += wcap) {
-                    W.n = std::min(wcap, ncur - off);
-                    k_setup_list<<<grid_for(W.n, 128, 1 << 30), 128, 0, s>>>(W, cur + off, W.n, vset.p, voff.p,
-                                                                            T.vert_tet);
-                    D3G_TRY(async_pass(false, W.n, nxt, anleft.p + 1, &nnext));
+                if (opt.timing) {
+                    float am = 0.f;
+                    cudaEventElapsedTime(&am, kev[0], kev[1]);
+                    R.stats.ms_async += am;
                 }
-                const bool slow = int64_t(ncur - nnext) * 4 < int64_t(ncur);
-                std::swap(cur, nxt);
-                ncur = nnext;
-                if (slow) break;
+                D3G_TRY(finish_points(defer.p, nd));
+                D3G_CUDA(cudaMemsetAsync(n_defer, 0, sizeof(int), s));
+                if (opt.validate) D3G_TRY(validate_tables("after", lev));
+                if (opt.timing) cudaEventRecord(kev[0], s);
             }
-            async_left = ncur;
-            for (int off = 0; off < ncur; off += maxw) {
-                W.n = std::min(maxw, ncur - off);
-                k_setup_list<<<grid_for(W.n, 128, 1 << 30), 128, 0, s>>>(W, cur + off, W.n, vset.p, voff.p,
-                                                                        T.vert_tet);
-                D3G_TRY(run_rounds());
-            }
-        } else {
-            D3G_TRY(run_rounds());
         }
-        if (opt.validate) D3G_TRY(validate_tables("after", lev));
-        if (trace) {
-            cudaEventRecord(ev1, s);
-            cudaEventSynchronize(ev1);
-            float ms = 0.f;
-            cudaEventElapsedTime(&ms, ev0, ev1);
-            {
-                unsigned long long ht1[2];
-                cudaMemcpy(ht1, totals.p, sizeof ht1, cudaMemcpyDeviceToHost);
-                won = (long long)ht1[0] - won_before;
-                attempts = (long long)ht1[1] - att_before;
-            }
-            unsigned long long as[7] = {0, 0, 0, 0, 0, 0, 0};
-            if (use_async) cudaMemcpy(as, astats.p, sizeof as, cudaMemcpyDeviceToHost);
-            fprintf(stderr, "d3g level %d sets %zu workers %d rounds %d inserted %lld attempts %lld "
-                    "left-by-fast-pass %lld left-by-async %lld ms %.2f | async totals: lock-conflicts %llu "
-                    "walk-restarts %llu bad-seeds %llu too-big %llu left %llu first-left %llu deferred %llu\n",
-                    lev, descs.size(), W.n, round - round0, won, attempts, deferred, async_left, ms, as[0],
-                    as[1], as[2], as[3], as[4], as[5], as[6]);
-            cudaEventDestroy(ev0);
-            cudaEventDestroy(ev1);
-        }
+        return D3G_OK;
+    };
+    if (use_async) {
+        D3G_TRY(run_async());
+    } else {
+        D3G_TRY(run_lockstep());
     }
     {
         unsigned long long hs2[2] = {0, 0}, ht[6], hst[2] = {0, 0}, hp[4] = {0, 0, 0, 0}, ha[7] = {};
         D3G_CUDA(cudaMemcpyAsync(hp, pstats.p, sizeof hp, cudaMemcpyDeviceToHost, s));
-        if (use_async) D3G_CUDA(cudaMemcpyAsync(ha, astats.p, sizeof ha, cudaMemcpyDeviceToHost, s));
+        D3G_CUDA(cudaMemcpyAsync(ha, astats.p, sizeof ha, cudaMemcpyDeviceToHost, s));
         D3G_CUDA(cudaMemcpyAsync(hs2, sums.p, sizeof hs2, cudaMemcpyDeviceToHost, s));
         D3G_CUDA(cudaMemcpyAsync(hst, steps.p, sizeof hst, cudaMemcpyDeviceToHost, s));
         D3G_CUDA(cudaMemcpyAsync(ht, totals.p, sizeof ht, cudaMemcpyDeviceToHost, s));
@@ -2975,12 +3142,14 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
         R.stats.tie_breaks = int64_t(hp[2]);
         R.stats.max_region_tets = int64_t(hp[3]);
         R.stats.deferred_points = int64_t(ha[6]);
+        if (use_async) R.stats.async_inserted = int64_t(ht[0]) - to_rounds;
     }
     // Release round scratch before the output stage.
     wcav.release();
     wfac.release();
     wsv.release();
     wsn.release();
+    alock.release();
     claim.release();
     fnew.release();
 

@@ -354,6 +354,8 @@ int own_order_sets(const double* d_xyz, const int64_t* h_off, const int64_t* d_o
         O.vert.swap(idx);
     }
     D3G_CUDA(cudaGetLastError());
+    O.keys.swap(hflags[0] > 0 ? keys2 : keys);
+    O.curve_bits = shift;
     O.ok = true;
     return D3G_OK;
 }

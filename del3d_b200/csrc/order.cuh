@@ -38,6 +38,8 @@ struct OwnOrder {
     DevBuf<int32_t> vert;        // per vertex: the global index of its first copy
     DevBuf<int32_t> rep;         // with repeated points: per vertex the local index it is reported under
     DevBuf<int32_t> level_start; // nsets * levels + 1: first vertex of each (set, level)
+    DevBuf<unsigned long long> keys;   // per vertex its sorted key, the Hilbert index in the low curve_bits
+    int curve_bits = 0;
     int64_t nv = 0;              // distinct points
     int levels = 0;              // levels per set in level_start
     bool ok = false;             // false: the keys cannot tell the points apart (use the spatial sort)
