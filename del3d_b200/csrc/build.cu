@@ -136,7 +136,7 @@ struct Workers {
     int4* st_n;   // ... and neighbours
     int* wset;        // set of each worker
     const int4* skips; // per set: its first tet's vertices (inserted before the rounds)
-    const uint8_t* set_exact;  // per set: 1 if its coordinates make the filters exact
+    const uint8_t* set_exact;  // per set: EX_*, what its coordinates make exact
     int cav_cap;
     int fac_cap;
     int n;
@@ -256,6 +256,9 @@ __device__ __noinline__ int hull_in_circle(double ax, double ay, double az, doub
 /// perturbation, or the hull in-circle test); and, for the fast variant only,
 /// undecided (left to the full variant).
 enum : int { CT_IN = 1, CT_UNCERTAIN = 2, CT_TIE = 4, CT_UNDECIDED = 8 };
+
+/// What a set's coordinates make exact (k_set_exact).
+enum : int { EX_ORIENT = 1, EX_SPHERE = 2, EX_BOTH = 3, EX_GRID = 4 };
 
 /// in_sphere's exact sign for a set whose filter is not exact and, when it is
 /// zero, the reference's tie-break (src/predicates.cpp:206-232): the sign, plus
@@ -446,7 +449,7 @@ __global__ void __launch_bounds__(128, 8) k_cavity(Tables T, Workers W, Round R,
     }
     if (!__any_sync(kFull, live)) return;
     const Pt p = live ? vpt(vx, v) : Pt{0.0, 0.0, 0.0};
-    const bool ex = live && W.set_exact[W.wset[w]] != 0;
+    const bool ex = live && (W.set_exact[W.wset[w]] & EX_BOTH) == EX_BOTH;
     int start = 0;
     if (live) start = T.vert_tet[W.last[w] >= 0 ? W.last[w] : W.guide[w]];
     int wsteps = 0;
@@ -1040,20 +1043,54 @@ __device__ __forceinline__ int in_circle_tiebreak_ex(int va, int vb, int vd, int
     return -local;
 }
 
+/// in_sphere of tet t and vertex pid in 64-bit integers, for points of a set
+/// whose coordinates are multiples of 1 / inv: exact where no difference exceeds
+/// kNearSteps steps (72 kNearSteps^5 < 2^63).  Returns its sign, or 2 where the
+/// points are too far apart or the set has no such grid.  Points are read again,
+/// as in in_sphere_tiebreak_ex.
+constexpr double kNearSteps = 2600.0;
+__device__ __forceinline__ int in_sphere_near(const int4 t, int pid, const double* __restrict__ vx, double inv) {
+    const Pt e = ld_vertex(vx, pid);
+    bool near = inv > 0.0;
+    auto steps = [&](int v, long long& x, long long& y, long long& z) {
+        const Pt p = ld_vertex(vx, v);
+        const double dx = fmul(fsub(p.x, e.x), inv), dy = fmul(fsub(p.y, e.y), inv), dz = fmul(fsub(p.z, e.z), inv);
+        near = near && fabs_(dx) <= kNearSteps && fabs_(dy) <= kNearSteps && fabs_(dz) <= kNearSteps;
+        x = (long long)dx;
+        y = (long long)dy;
+        z = (long long)dz;
+    };
+    long long ax, ay, az, bx, by, bz, cx, cy, cz, dx, dy, dz;
+    steps(t.x, ax, ay, az);
+    steps(t.y, bx, by, bz);
+    steps(t.z, cx, cy, cz);
+    steps(t.w, dx, dy, dz);
+    if (!near) return 2;
+    const long long ab = ax * by - bx * ay, bc = bx * cy - cx * by, cd = cx * dy - dx * cy, da = dx * ay - ax * dy,
+                    ac = ax * cy - cx * ay, bd = bx * dy - dx * by;
+    const long long abc = az * bc - bz * ac + cz * ab, bcd = bz * cd - cz * bd + dz * bc,
+                    cda = cz * da + dz * ac + az * cd, dab = dz * ab + az * bd + bz * da;
+    const long long det = ((dx * dx + dy * dy + dz * dz) * abc - (cx * cx + cy * cy + cz * cz) * dab) +
+                          ((bx * bx + by * by + bz * bz) * cda - (ax * ax + ay * ay + az * az) * bcd);
+    return det > 0 ? -1 : (det < 0 ? 1 : 0);   // in_sphere = -sign(det)
+}
+
 /// The hull in-circle test (reference src/triangulation.cpp:588-602, a point
 /// in the plane of the hull facet (va, vb, vd) of infinite tet `tet`: in
 /// conflict iff inside the facet's circumcircle, a tie by the cocircular
-/// perturbation) for a set whose coordinates make the filters exact, without
+/// perturbation) for a set whose coordinates make orient3d exact, without
 /// the in-circle determinant: the sphere through va, vb, vd and the apex x of
 /// the finite tet across the facet cuts the facet's plane in the facet's
 /// circumcircle, and a point of that plane has the same power with respect
 /// to both, so sign in_circle(va, vb, vd, p) = sign det_in_sphere(va, vb, vd,
-/// x, p) * sign det_orient3d(va, vb, vd, x), both exact here.  The caller
+/// x, p) * sign det_orient3d(va, vb, vd, x); the first is exact in double
+/// (`sphere`: the set's coordinates make it so) or in 64 bits (in_sphere_near).  The caller
 /// holds the lock of `tet`, so the finite tet across its facet is not being
 /// rewritten.  Returns 1 (inside), -1 (outside), or 0 if the apex is unusable
 /// (the caller then leaves the test undecided).
+template <bool kNear>
 __device__ __forceinline__ int hull_in_circle_ex(const Tables& T, int tet, int ip, int va, int vb, int vd, int pid,
-                                                 const double* __restrict__ vx) {
+                                                 const double* __restrict__ vx, bool sphere, double inv) {
     const int f = at(ld4(&T.tn(tet)), ip) >> 2;
     const int4 fv = ld4(&T.tv(f));
     int x = -1;
@@ -1066,20 +1103,25 @@ __device__ __forceinline__ int hull_in_circle_ex(const Tables& T, int tet, int i
     const Pt a = ld_vertex(vx, va), b = ld_vertex(vx, vb), d = ld_vertex(vx, vd), xp = ld_vertex(vx, x);
     const int so = sign_of(orient3d_filter(a, b, d, xp).det);
     if (so == 0) return 0;
-    const int ss = sign_of(in_sphere_filter_lean(a, b, d, xp, ld_vertex(vx, pid)).det);
+    if (!kNear && !sphere) return 0;
+    const int ss = sphere ? sign_of(in_sphere_filter_lean(a, b, d, xp, ld_vertex(vx, pid)).det)
+                          : -in_sphere_near(make_int4(va, vb, vd, x), pid, vx, inv);
+    if (ss == -2) return 0;
     if (ss != 0) return ss * so;
     return in_circle_tiebreak_ex(va, vb, vd, pid, vx);
 }
 
 /// The conflict test of the fast variant (reference src/triangulation.cpp:588-602,
 /// as conflict_test) of tet `tet` = t, with its outcome bits; CT_UNDECIDED when
-/// the filter cannot decide and the exact stage is needed, or the point lies in
-/// the plane of a hull facet (the coplanar in-circle test) of a set whose
-/// filters are not exact.  Call-free: on a set whose coordinates make the
-/// filters exact, an exactly cospherical call gets its tie-break inline, and
-/// a point in the plane of a hull facet its in-circle test.
+/// the filter cannot decide and the exact stage is needed.  Call-free: where the
+/// set's coordinates make the filters exact (`ex`: EX_*), or (kNear) the points
+/// lie near enough on its grid, an undecided call is settled inline, an exactly
+/// cospherical one by its tie-break and a point in the plane of a hull facet by
+/// its in-circle test.
+template <bool kNear>
 __device__ __forceinline__ int in_conflict_fast(const Tables& T, int tet, const int4 t, const Pt& p, int pid,
-                                                const double* __restrict__ vx, bool ex) {
+                                                const double* __restrict__ vx, int ex,
+                                                const double* __restrict__ inv_grid) {
     const int ip = inf_pos(t);
     if (ip >= 0) {
         const int o0 = ip == 0 ? 2 : (ip == 1 ? 2 : (ip == 2 ? 1 : 0));
@@ -1088,9 +1130,10 @@ __device__ __forceinline__ int in_conflict_fast(const Tables& T, int tet, const 
         const Pt a = vpt(vx, at(t, o0)), b = vpt(vx, at(t, o1)), d = vpt(vx, at(t, o2));
         const Orient3dFilter f = orient3d_filter(a, b, d, p);
         if (f.certain) return f.det < 0.0 ? CT_IN : 0;   // orient3d = -sign(det)
-        if (ex && f.det != 0.0) return (f.det < 0.0 ? CT_IN : 0) | CT_UNCERTAIN;
-        if (ex) {
-            const int h = hull_in_circle_ex(T, tet, ip, at(t, o0), at(t, o1), at(t, o2), pid, vx);
+        if ((ex & EX_ORIENT) && f.det != 0.0) return (f.det < 0.0 ? CT_IN : 0) | CT_UNCERTAIN;
+        if (ex & EX_ORIENT) {
+            const int h = hull_in_circle_ex<kNear>(T, tet, ip, at(t, o0), at(t, o1), at(t, o2), pid, vx, ex & EX_SPHERE,
+                                                   kNear ? inv_grid[T.vset[pid]] : 0.0);
             if (h != 0) return (h > 0 ? CT_IN : 0) | CT_UNCERTAIN | CT_TIE;
         }
         return CT_UNDECIDED;
@@ -1098,9 +1141,12 @@ __device__ __forceinline__ int in_conflict_fast(const Tables& T, int tet, const 
     const Pt a = vpt(vx, t.x), b = vpt(vx, t.y), c = vpt(vx, t.z), d = vpt(vx, t.w);
     const InSphereFilter f = in_sphere_filter_lean(a, b, c, d, p);
     if (f.certain) return f.det < 0.0 ? CT_IN : 0;   // in_sphere = -sign(det)
-    if (ex && f.det != 0.0) return (f.det < 0.0 ? CT_IN : 0) | CT_UNCERTAIN;
-    if (ex) return (in_sphere_tiebreak_ex(t, pid, vx) > 0 ? CT_IN : 0) | CT_UNCERTAIN | CT_TIE;
-    return CT_UNDECIDED;
+    int s = 0;
+    if (ex & EX_SPHERE) s = -sign_of(f.det);
+    else s = kNear ? in_sphere_near(t, pid, vx, inv_grid[T.vset[pid]]) : 2;
+    if (s == 2) return CT_UNDECIDED;
+    if (s != 0) return (s > 0 ? CT_IN : 0) | CT_UNCERTAIN;
+    return (in_sphere_tiebreak_ex(t, pid, vx) > 0 ? CT_IN : 0) | CT_UNCERTAIN | CT_TIE;
 }
 
 enum : int { AI_DONE = 0, AI_RETRY = 1, AI_LEAVE = 2, AI_DEFER = 3 };
@@ -1378,7 +1424,7 @@ __global__ void __launch_bounds__(128, 8) k_insert_full(Tables T, Workers W, Asy
         q = __shfl_sync(kFull, q, 0);
         if (q >= A.nw) break;
         const int w = int((int64_t(q) * A.stride) % A.nw);
-        const bool ex = W.set_exact[W.wset[w]] != 0;
+        const bool ex = (W.set_exact[W.wset[w]] & EX_BOTH) == EX_BOTH;
         const int b = W.beg[w], len = W.end[w] - b;
         const int4 sk = W.skips[W.wset[w]];
         int pos = W.pos[w], left = W.left[w];
@@ -1546,15 +1592,36 @@ __global__ void k_setup_list(Workers W, const int* __restrict__ list, int n, con
     W.state[w] = WS_DONE;
 }
 
-/// A set whose span makes the orient3d and in_sphere filters exact.
-__global__ void k_set_exact(const int* __restrict__ smin, const int* __restrict__ stop, int nsets,
-                            uint8_t* __restrict__ ex) {
+/// What a set's coordinates say of its filters.  All are multiples of grid = 2^emin
+/// and lie in a box of longest side D grid steps, so every difference a filter
+/// takes is a whole number of steps, at most D: exact in double, and with it
+/// every product and sum of the determinants while these stay below 2^53.
+/// orient3d sums 6 products of 3 differences (6 D^3), in_sphere 72 of 5 (72 D^5).
+/// Bit 0: orient3d's filter value is exact for any points of the set, bit 1:
+/// in_sphere's; bit 2: a grid of few enough steps that its points often are
+/// cospherical, but too many for bit 1.  `inv_grid` is 1 / grid, for the tests whose five points are near
+/// enough to be exact in 64 bits by themselves (in_sphere_near); 0 where the
+/// scale leaves the range in which nothing can over- or underflow.
+constexpr double kGridSteps = 1048576.0;
+__global__ void k_set_exact(const int* __restrict__ span, const unsigned long long* __restrict__ box, int nsets,
+                            uint8_t* __restrict__ ex, double* __restrict__ inv_grid) {
     const int s = int(blockIdx.x) * blockDim.x + threadIdx.x;
     if (s >= nsets) return;
-    Span sp;
-    sp.emin = smin[s];
-    sp.top = stop[s];
-    ex[s] = (sp.exact_in_double(5, 7) && sp.exact_in_double(3, 3)) ? 1 : 0;
+    const int emin = span[s], top = span[nsets + s];
+    int r = 0;
+    double inv = 0.0;
+    if (top < emin) {   // no coordinate but zeros
+        r = EX_ORIENT | EX_SPHERE;
+    } else if (emin >= -200 && emin <= 190) {
+        inv = scalbn(1.0, -emin);
+        double side = 0.0;
+        for (int k = 0; k < 3; ++k)
+            side = fmax(side, dbl_from_order_key(box[6 * int64_t(s) + 3 + k]) - dbl_from_order_key(box[6 * int64_t(s) + k]));
+        const double steps = side * inv;
+        r = (steps <= 110000.0 ? EX_ORIENT : 0) | (steps <= 659.0 ? EX_SPHERE : (steps <= kGridSteps ? EX_GRID : 0));
+    }
+    ex[s] = uint8_t(r);
+    inv_grid[s] = inv;
 }
 
 /// Puts every vertex but the first tets' in its level's list (items), and gives
@@ -2306,16 +2373,20 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
     int growth = opt.level_growth;
     SetScan scan;
     D3G_TRY(scan_sets(d_xyz, d_off.p, nsets, n, scan, status.p + 1, s));
+    // Sets whose coordinates span few grid steps (integer lattices, coarse grids):
+    // their filters are exact, so their degenerate queries skip the exact stage.
+    DevBuf<uint8_t> set_exact;
+    DevBuf<double> inv_grid;
+    D3G_TRY(set_exact.alloc(size_t(nsets), s));
+    D3G_TRY(inv_grid.alloc(size_t(nsets), s));
+    k_set_exact<<<grid_for(nsets, 128), 128, 0, s>>>(scan.span.p, scan.box.p, nsets, set_exact.p, inv_grid.p);
     if (growth == 0 && use_async) growth = kGroupGrowth;
     if (growth == 0) {
-        DevBuf<uint8_t> ex;
-        D3G_TRY(ex.alloc(size_t(nsets), s));
-        k_set_exact<<<grid_for(nsets, 128), 128, 0, s>>>(scan.span.p, scan.span.p + nsets, nsets, ex.p);
         std::vector<uint8_t> hex(static_cast<size_t>(nsets));
-        D3G_CUDA(cudaMemcpyAsync(hex.data(), ex.p, size_t(nsets), cudaMemcpyDeviceToHost, s));
+        D3G_CUDA(cudaMemcpyAsync(hex.data(), set_exact.p, size_t(nsets), cudaMemcpyDeviceToHost, s));
         D3G_CUDA(cudaStreamSynchronize(s));
         growth = n < kSmallBuildPoints ? kExactSetGrowth : 8;
-        for (const uint8_t e : hex) growth = e ? kExactSetGrowth : growth;
+        for (const uint8_t e : hex) growth = (e & EX_BOTH) == EX_BOTH ? kExactSetGrowth : growth;
     }
     DevBuf<double> vx;
     DevBuf<int32_t> vert_point, vset, voff;
@@ -2392,6 +2463,8 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
     std::vector<int32_t> hvoff(size_t(nsets) + 1);
     D3G_CUDA(cudaMemcpyAsync(hvoff.data(), voff.p, sizeof(int32_t) * hvoff.size(), cudaMemcpyDeviceToHost, s));
 
+    std::vector<uint8_t> hexact(static_cast<size_t>(nsets));
+    D3G_CUDA(cudaMemcpyAsync(hexact.data(), set_exact.p, size_t(nsets), cudaMemcpyDeviceToHost, s));
     uint32_t hst[2] = {0, 0};
     D3G_CUDA(cudaMemcpyAsync(hst, status.p, sizeof hst, cudaMemcpyDeviceToHost, s));
     D3G_CUDA(cudaStreamSynchronize(s));
@@ -2469,12 +2542,6 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
     T.vset = vset.p;
     k_set_int<<<1, 1, 0, s>>>(tet_count.p, 5 * nsets);
     k_init_tets<<<grid_for(nsets, 64), 64, 0, s>>>(T, vx.p, skips.p, nsets, status.p);
-    // Sets whose coordinates span few bits (integer lattices, coarse grids):
-    // their filters are exact, so their degenerate queries skip the exact stage.
-    DevBuf<uint8_t> set_exact;
-    D3G_TRY(set_exact.alloc(size_t(nsets), s));
-    k_set_exact<<<grid_for(nsets, 128), 128, 0, s>>>(scan.span.p, scan.span.p + nsets, nsets, set_exact.p);
-
     // ---- levels ----
     // A level of s points goes into a triangulation of p earlier points.  Two
     // insertions collide when their regions (about 20 tets and their ring)
@@ -3015,26 +3082,37 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
         A.pool = pool.p;
         A.skips = skips.p;
         A.set_exact = set_exact.p;
+        A.inv_grid = inv_grid.p;
         A.voff = voff.p;
         A.stats = astats.p;
         A.cavity = cav_normal;
-        auto launch = [&](int G, int ngroups) {
+        auto launch = [&](int G, int ngroups, bool near) {
             // At most one group per kPoolSlots vertices, so that the slots groups hold
             // without using them stay within the table's room for them.
             A.ngroups = std::max(1, std::min({ngroups, kNumSMs * kGroupBlocks * (kGroupThreads / G), nv / kPoolSlots}));
             const unsigned grid = unsigned((A.ngroups + kGroupThreads / G - 1) / (kGroupThreads / G));
-            if (G == 8) k_insert_groups<8><<<grid, kGroupThreads, 0, s>>>(T, A, Rd, vx.p);
-            else if (G == 16) k_insert_groups<16><<<grid, kGroupThreads, 0, s>>>(T, A, Rd, vx.p);
-            else k_insert_groups<32><<<grid, kGroupThreads, 0, s>>>(T, A, Rd, vx.p);
+            auto* kernel = G == 8 ? (near ? k_insert_groups<8, true> : k_insert_groups<8, false>)
+                                  : (G == 16 ? (near ? k_insert_groups<16, true> : k_insert_groups<16, false>)
+                                             : (near ? k_insert_groups<32, true> : k_insert_groups<32, false>));
+            kernel<<<grid, kGroupThreads, 0, s>>>(T, A, Rd, vx.p);
             R.stats.launches_async += 1;
         };
+        // The variant that settles undecided tests of near points in 64 bits needs more
+        // registers (36 bytes of spills at 96): 10^7 uniform points 107 -> 114 ms, 4096
+        // mixed sets 410 -> 437, but the 10^6 sphere on a 2^-10 grid 79 -> 27.  So it takes
+        // the levels of a build most of whose points lie on such grids, and elsewhere
+        // only what the plain one leaves.
+        int64_t on_grid = 0;
+        for (int st = 0; st < nsets; ++st)
+            if (hexact[size_t(st)] & EX_GRID) on_grid += R.set_nv[size_t(st)];
+        const bool near_main = 2 * on_grid > nv;
         auto left_pass = [&](int lev, int ngroups) {
             A.items = left_of(lev);
             A.n_items = n_left_of(lev);
             A.next = head_of(lev) + 2;
             A.left = left_of(lev + 1);
             A.n_left = n_left_of(lev + 1);
-            launch(32, ngroups);
+            launch(32, ngroups, true);
         };
         if (opt.timing) cudaEventRecord(kev[0], s);
         for (int lev = 0; lev < nlev; ++lev) {
@@ -3055,9 +3133,10 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
             // (points in each other's way) waits for the next level's pass.
             A.left = left_of(G < 32 ? lev : lev + 1);
             A.n_left = n_left_of(G < 32 ? lev : lev + 1);
-            // (The first level grows from one tet: there the guides are nearer.)
-            if (lev > 0) k_locate<<<grid_for(m_of[lev], 128), 128, 0, s>>>(T, A, vx.p);
-            launch(G, int(std::min<int64_t>(groups_of[size_t(lev)], 1 << 24)));
+            // (The first level grows from one tet: there the guides are nearer.  A caller's
+            // walk limit holds for an insertion's whole walk.)
+            if (lev > 0 && opt.walk_limit <= 0) k_locate<<<grid_for(m_of[lev], 128), 128, 0, s>>>(T, A, vx.p);
+            launch(G, int(std::min<int64_t>(groups_of[size_t(lev)], 1 << 24)), near_main);
             if (lev > 0 || G < 32) left_pass(lev, kNumSMs * (kGroupThreads / 32));
             D3G_CUDA(cudaGetLastError());
             if (trace) {
@@ -3091,7 +3170,7 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
                 A.next = head_of(nlev + kLastPasses - 1) + 2;
                 A.left = defer.p;
                 A.n_left = n_defer;
-                launch(32, 16);   // few in the way of one another
+                launch(32, 16, true);   // few in the way of one another
             }
             if (opt.validate || lev == nlev - 1) {
                 int nd = 0;

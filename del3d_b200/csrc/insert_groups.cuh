@@ -61,13 +61,15 @@ struct GroupArgs {
     const int* n_items;      // how many
     int* hint;               // per vertex: a tet near it (k_locate), -1: none
     int* next;               // queue head
-    int* left;               // points a wider group should try (regions too big, too many conflicts) ...
+    int* left;               // points to try again by wider groups or with kNear (regions too big, too many
+                             // conflicts, undecided tests) ...
     int* n_left;
     int* defer;              // ... and points for the full variant (a test the filters cannot decide)
     int* n_defer;
     int4* pool;              // per group: tet slots it holds (GroupScratch::pool)
     const int4* skips;       // per set: its first tet's vertices
-    const uint8_t* set_exact;
+    const uint8_t* set_exact;    // per set: EX_*
+    const double* inv_grid;      // per set: see in_sphere_near
     const int32_t* voff;     // per set: its vertices
     unsigned long long* stats;   // as AsyncCtx::stats
     int cavity;              // region tets at most (and twice as many boundary facets), if fewer than kCap
@@ -120,15 +122,16 @@ __device__ __forceinline__ int tet_near(const Tables& T, int guide, int vlo, int
 /// Locates a level's points, one thread each, in the mesh as it is before the
 /// level: the walk of an insertion, which has a group's lanes wait for one chain
 /// of reads, then starts a step or two from its end.  Reads may use L1, since
-/// nothing writes the mesh meanwhile.  A walk that the filter cannot decide, or a
-/// long one, ends where it is: the tet is only where the insertion starts.
+/// nothing writes the mesh meanwhile.  A facet the filter cannot decide is not
+/// crossed and a long walk ends where it is: the tet is only where the insertion
+/// starts.
 __global__ void __launch_bounds__(128) k_locate(Tables T, GroupArgs A, const double* __restrict__ vx) {
     const int n = *A.n_items;
     for (int k = int(blockIdx.x) * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         const int v = A.items[k];
         if (v < 0) continue;
         const int set = T.vset[v];
-        const bool ex = A.set_exact[set] != 0;
+        const bool ex = A.set_exact[set] & EX_ORIENT;
         const Pt p = vpt(vx, v);
         int t = tet_near(T, A.guide[v], A.voff[set], A.skips[set].x);
         int4 tv = T.tv(t);
@@ -144,15 +147,13 @@ __global__ void __launch_bounds__(128) k_locate(Tables T, GroupArgs A, const dou
             const Pt a = vpt(vx, tv.x), b = vpt(vx, tv.y), c = vpt(vx, tv.z), d = vpt(vx, tv.w);
             h = h * 1664525u + 1013904223u;
             int next = -1;
-            bool stop = false;
 #pragma unroll 1
-            for (int m = 0; m < 4 && next < 0 && !stop; ++m) {
+            for (int m = 0; m < 4 && next < 0; ++m) {
                 const int i = int((h >> 30) + unsigned(m)) & 3;
                 const int nb = at(tn, i) >> 2;
                 if (nb == prev) continue;
                 const int o = orient_replaced_filter(a, b, c, d, i, p, ex);
-                if (o == 2) stop = true;
-                else if (o < 0) next = nb;
+                if (o < 0) next = nb;
             }
             if (next < 0) break;
             prev = t;
@@ -164,7 +165,7 @@ __global__ void __launch_bounds__(128) k_locate(Tables T, GroupArgs A, const dou
     }
 }
 
-template <int G>
+template <int G, bool kNear>
 __global__ void __launch_bounds__(kGroupThreads, kGroupBlocks)
     k_insert_groups(Tables T, GroupArgs A, Round R, const double* __restrict__ vx) {
     typedef GroupScratch<G> Scratch;
@@ -239,7 +240,7 @@ __global__ void __launch_bounds__(kGroupThreads, kGroupBlocks)
         if (!__any_sync(kFull, live)) break;
         const int v = live ? S.item : 0;
         const Pt p = vpt(vx, v);
-        const bool ex = A.set_exact[T.vset[v]] != 0;
+        const int ex = A.set_exact[T.vset[v]];
         t = max(__shfl_sync(kFull, t, L.gbase), 0);
 
         // Slots for its new tets, asked for here so that the answer is there by the re-star.
@@ -249,7 +250,10 @@ __global__ void __launch_bounds__(kGroupThreads, kGroupBlocks)
 
         // ---- walk (see walk_async; lanes 0-3 test the facets, lanes 4-7 fetch the
         //      neighbours' records) ----
+        // A facet the filter cannot decide is not crossed: the seed is tested in any
+        // case, and if it fails the test the point is left to the full variant.
         int outcome = live ? AI_DONE : -1;
+        bool fuzzy = false;
         {
             int4 tv, tn;
             ld_rec(T, t, tv, tn);
@@ -276,7 +280,7 @@ __global__ void __launch_bounds__(kGroupThreads, kGroupBlocks)
                 if (walking && L.sub < 4 && (at(tn, L.sub) >> 2) != prev && tv.x != kInf && tv.y != kInf &&
                     tv.z != kInf && tv.w != kInf) {
                     const int o = orient_replaced_filter(vpt(vx, tv.x), vpt(vx, tv.y), vpt(vx, tv.z), vpt(vx, tv.w),
-                                                         L.sub, p, ex);
+                                                         L.sub, p, ex & EX_ORIENT);
                     undecided = o == 2;
                     neg = o < 0;
                 }
@@ -290,10 +294,8 @@ __global__ void __launch_bounds__(kGroupThreads, kGroupBlocks)
                 const int4 nn = make_int4(__shfl_sync(kFull, pn.x, src), __shfl_sync(kFull, pn.y, src),
                                           __shfl_sync(kFull, pn.z, src), __shfl_sync(kFull, pn.w, src));
                 if (!walking) continue;
-                if (und) {
-                    outcome = AI_DEFER;
-                    walking = false;
-                } else if (m == 0) {
+                fuzzy = fuzzy || und;
+                if (m == 0) {
                     walking = false;
                 } else {
                     const int next = at(tn, i) >> 2;
@@ -306,6 +308,7 @@ __global__ void __launch_bounds__(kGroupThreads, kGroupBlocks)
                     } else if (++step >= limit) {
                         outcome = AI_RETRY;
                         walking = false;
+                        t = -1;
                         if (L.sub == 0) atomicAdd(A.stats + 1, 1ull);
                     }
                 }
@@ -348,7 +351,7 @@ __global__ void __launch_bounds__(kGroupThreads, kGroupBlocks)
                 if (got) {
                     int r = 0;
                     for (;;) {
-                        r = in_conflict_fast(T, nb, guess, p, v, vx, ex);
+                        r = in_conflict_fast<kNear>(T, nb, guess, p, v, vx, ex, A.inv_grid);
                         if (guess.x == tv.x && guess.y == tv.y && guess.z == tv.z && guess.w == tv.w) break;
                         guess = tv;
                     }
@@ -402,7 +405,7 @@ __global__ void __launch_bounds__(kGroupThreads, kGroupBlocks)
                 }
                 for (int k = L.sub; k < nreg; k += G) set_lock(A.lock + S.reg[k], 0);
                 if (L.sub == 0) atomicAdd(A.stats + (ab ? 0 : (und ? 6 : (bad ? 2 : 3))), 1ull);
-                outcome = (ab || bad) && !und ? AI_RETRY : (und ? AI_DEFER : AI_LEAVE);
+                outcome = und || (bad && fuzzy) ? AI_DEFER : (ab || bad ? AI_RETRY : AI_LEAVE);
                 growing = false;
             }
             if (growing) {
@@ -564,12 +567,12 @@ __global__ void __launch_bounds__(kGroupThreads, kGroupBlocks)
             if (outcome == AI_RETRY && attempt < kGroupTries) {
                 S.stash[S.nstash] = v;
                 S.stash_tries[S.nstash++] = attempt;
-                A.hint[v] = t;
+                if (t >= 0) A.hint[v] = t;
                 idle = !S.open;
                 wait = min(attempt, 3);
             } else {
-                // Too big for the widest group, or undecided: the full variant.
-                const bool def = outcome == AI_DEFER || (outcome == AI_LEAVE && G == 32);
+                // Too big for the widest group, or undecided even so: the full variant.
+                const bool def = (outcome == AI_DEFER && kNear) || (outcome == AI_LEAVE && G == 32);
                 (def ? A.defer : A.left)[atomicAdd(def ? A.n_defer : A.n_left, 1)] = v;
                 atomicAdd(A.stats + 4, 1ull);
             }

@@ -58,3 +58,28 @@ def test_offset_lattice_and_caller_chunks(cuda):
     x = torch.from_numpy(pts).to(cuda)
     for kw in ({}, {"chunk": 7}, {"chunk": 100000}, {"chunk": -1, "alpha_small": 1}, {"chunk": -500}):
         assert np.array_equal(d3.build_device(x, **kw)[0].cpu().numpy(), want), kw
+
+
+def _grid_ball(radius, n, seed):
+    """n distinct integer points on a few concentric integer spheres and in the planes of their poles:
+    many exactly cospherical and cocircular groups, differences of up to 2 * radius."""
+    rng = np.random.default_rng(seed)
+    base = np.array([[radius, 0, 0], [radius * 3 // 5, radius * 4 // 5, 0], [radius // 3, radius * 2 // 3, radius * 2 // 3]])
+    v = base[rng.integers(0, 3, 4 * n)]
+    v = np.take_along_axis(v, rng.permuted(np.tile(np.arange(3), (4 * n, 1)), axis=1), 1) * rng.choice([-1, 1], (4 * n, 3))
+    v = v // rng.choice([1, 2], (4 * n, 1))
+    p = np.unique(np.concatenate([v, rng.integers(-radius, radius + 1, (n // 4, 3))]), axis=0)
+    return rng.permutation(p)[:n].astype(np.float64)
+
+
+@pytest.mark.parametrize("scale", [1.0, 2.0 ** -10, 2.0 ** 40, 2.0 ** -199, 2.0 ** 189, 2.0 ** -210])
+@pytest.mark.parametrize("radius", [315, 330, 1290, 1305, 5400, 60000])
+def test_exact_by_differences(cuda, radius, scale):
+    """Sets on either side of the lines up to which the filters are exact for the whole set (659 steps
+    across for in_sphere, 110000 for orient3d) and for one test (2600 steps), at both ends of the scales."""
+    pts = _grid_ball(radius, 300, radius) * scale
+    pts += np.array([7.0, -3.0, 11.0]) * radius * scale
+    want = oracle.orc_build(pts)
+    d = d3.Delaunay()
+    d.build(pts)
+    assert np.array_equal(d.finite_cells(), want["cells"]) and np.array_equal(d.all_cells(), want["all"])
