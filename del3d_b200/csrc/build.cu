@@ -803,14 +803,17 @@ __device__ __forceinline__ void unlock_if(int* lock, int t, int value) {
 
 __device__ __forceinline__ int4 ld4(const int4* p) { return __ldcg(p); }
 
-/// orient3d of tet (a, b, c, d) with vertex `i` replaced by p, from the filter
-/// alone: the sign when the filter decides it (or `ex`: the set's coordinates
-/// make the filter's value exact), else 2.  Selects, no calls and no local
-/// arrays, so that it adds nothing to the caller's live state.
-__device__ __forceinline__ int orient_replaced_filter(const Pt& a, const Pt& b, const Pt& c, const Pt& d, int i,
-                                                      const Pt& p, bool ex) {
-    const Pt A = i == 0 ? p : a, B = i == 1 ? p : b, C = i == 2 ? p : c, D = i == 3 ? p : d;
-    const Orient3dFilter f = orient3d_filter(A, B, C, D);
+/// orient3d of tet `t` with vertex i replaced by p, from the filter alone: the
+/// sign when the filter decides it (or `ex`: the set's coordinates make the
+/// filter's value exact), else 2.  An even permutation of that call puts p last,
+/// so only the facet's three vertices are read; choosing them by index costs a few
+/// selects where choosing among four points' coordinates costs 24.
+template <class M>
+__device__ __forceinline__ int orient_facet_filter(const M& m, const int4& t, int i, const Pt& p, bool ex) {
+    const int x = i == 0 ? t.z : (i == 2 ? t.y : t.x);
+    const int y = i == 0 ? t.y : (i == 1 ? t.z : (i == 2 ? t.x : t.y));
+    const int z = i == 3 ? t.z : t.w;
+    const Orient3dFilter f = orient3d_filter(m.point(x), m.point(y), m.point(z), p);
     if (f.certain || ex) return -sign_of(f.det);
     return 2;
 }
@@ -847,11 +850,8 @@ __device__ int walk_async(int t, const Pt& p, int pid, const Tables& T, const do
         if (lane < 4 && (at(tn, lane) >> 2) != prev && tv.x != kInf && tv.y != kInf && tv.z != kInf &&
             tv.w != kInf) {
             const Pt a = vpt(vx, tv.x), b = vpt(vx, tv.y), c = vpt(vx, tv.z), d = vpt(vx, tv.w);
-            int o = orient_replaced_filter(a, b, c, d, lane, p, ex);
-            if (o == 2) {
-                const Pt A = lane == 0 ? p : a, B = lane == 1 ? p : b, C = lane == 2 ? p : c, D = lane == 3 ? p : d;
-                o = orient3d(A, B, C, D, st);
-            }
+            const Pt A = lane == 0 ? p : a, B = lane == 1 ? p : b, C = lane == 2 ? p : c, D = lane == 3 ? p : d;
+            const int o = orient3d_x(A, B, C, D, ex, st);
             neg = o < 0;
         }
         const unsigned m = __ballot_sync(kFull, neg) & 0xFu;
@@ -892,7 +892,8 @@ __device__ __forceinline__ Pt ld_vertex(const double* __restrict__ vx, int v) {
 /// else the next largest, once more; else NEGATIVE.  Points are read again
 /// from memory each time they are needed, so the tie-break adds no live state
 /// to the loop around it.
-__device__ __forceinline__ int in_sphere_tiebreak_ex(const int4 t, int pid, const double* __restrict__ vx) {
+template <class M>
+__device__ __forceinline__ int in_sphere_tiebreak_ex(const M& m, const int4 t, int pid) {
     int skip = -1;
 #pragma unroll 1
     for (int r = 0; r < 2; ++r) {
@@ -901,16 +902,16 @@ __device__ __forceinline__ int in_sphere_tiebreak_ex(const int4 t, int pid, cons
 #pragma unroll 1
         for (int k = 0; k < 5; ++k) {
             if (k == skip) continue;
-            const Pt q = ld_vertex(vx, k < 4 ? at(t, k) : pid);
+            const Pt q = m.again(k < 4 ? at(t, k) : pid);
             if (best < 0 || lexico_less(bp, q)) {
                 best = k;
                 bp = q;
             }
         }
         if (best == 4) return -1;
-        const Pt pp = ld_vertex(vx, pid);
-        const Pt A = best == 0 ? pp : ld_vertex(vx, t.x), B = best == 1 ? pp : ld_vertex(vx, t.y),
-                 C = best == 2 ? pp : ld_vertex(vx, t.z), D = best == 3 ? pp : ld_vertex(vx, t.w);
+        const Pt pp = m.again(pid);
+        const Pt A = best == 0 ? pp : m.again(t.x), B = best == 1 ? pp : m.again(t.y),
+                 C = best == 2 ? pp : m.again(t.z), D = best == 3 ? pp : m.again(t.w);
         const int o = -sign_of(orient3d_filter(A, B, C, D).det);
         if (o != 0) return o;
         skip = best;
@@ -1015,9 +1016,9 @@ __device__ __forceinline__ int coplanar_orientation3_ex(const Pt& p, const Pt& q
 /// orientation gives it times the orientation of (va, vb, vd); else the
 /// opposite of that orientation.  Points are read again from memory, as in
 /// in_sphere_tiebreak_ex.
-__device__ __forceinline__ int in_circle_tiebreak_ex(int va, int vb, int vd, int pid,
-                                                     const double* __restrict__ vx) {
-    const int local = coplanar_orientation3_ex(ld_vertex(vx, va), ld_vertex(vx, vb), ld_vertex(vx, vd));
+template <class M>
+__device__ __forceinline__ int in_circle_tiebreak_ex(const M& m, int va, int vb, int vd, int pid) {
+    const int local = coplanar_orientation3_ex(m.again(va), m.again(vb), m.again(vd));
     unsigned excluded = 0;
 #pragma unroll 1
     for (int r = 0; r < 3; ++r) {
@@ -1026,7 +1027,7 @@ __device__ __forceinline__ int in_circle_tiebreak_ex(int va, int vb, int vd, int
 #pragma unroll 1
         for (int k = 0; k < 4; ++k) {
             if (excluded & (1u << k)) continue;
-            const Pt q = ld_vertex(vx, k == 0 ? va : (k == 1 ? vb : (k == 2 ? vd : pid)));
+            const Pt q = m.again(k == 0 ? va : (k == 1 ? vb : (k == 2 ? vd : pid)));
             if (best < 0 || !lexico_less(q, bp)) {   // a later slot wins ties
                 best = k;
                 bp = q;
@@ -1034,9 +1035,9 @@ __device__ __forceinline__ int in_circle_tiebreak_ex(int va, int vb, int vd, int
         }
         excluded |= 1u << best;
         if (best == 3) return -1;
-        const Pt pp = ld_vertex(vx, pid);
-        const Pt A = best == 0 ? pp : ld_vertex(vx, va), B = best == 1 ? pp : ld_vertex(vx, vb),
-                 C = best == 2 ? pp : ld_vertex(vx, vd);
+        const Pt pp = m.again(pid);
+        const Pt A = best == 0 ? pp : m.again(va), B = best == 1 ? pp : m.again(vb),
+                 C = best == 2 ? pp : m.again(vd);
         const int o = coplanar_orientation3_ex(A, B, C);
         if (o != 0) return o * local;
     }
@@ -1049,11 +1050,12 @@ __device__ __forceinline__ int in_circle_tiebreak_ex(int va, int vb, int vd, int
 /// points are too far apart or the set has no such grid.  Points are read again,
 /// as in in_sphere_tiebreak_ex.
 constexpr double kNearSteps = 2600.0;
-__device__ __forceinline__ int in_sphere_near(const int4 t, int pid, const double* __restrict__ vx, double inv) {
-    const Pt e = ld_vertex(vx, pid);
+template <class M>
+__device__ __forceinline__ int in_sphere_near(const M& m, const int4 t, int pid, double inv) {
+    const Pt e = m.again(pid);
     bool near = inv > 0.0;
     auto steps = [&](int v, long long& x, long long& y, long long& z) {
-        const Pt p = ld_vertex(vx, v);
+        const Pt p = m.again(v);
         const double dx = fmul(fsub(p.x, e.x), inv), dy = fmul(fsub(p.y, e.y), inv), dz = fmul(fsub(p.z, e.z), inv);
         near = near && fabs_(dx) <= kNearSteps && fabs_(dy) <= kNearSteps && fabs_(dz) <= kNearSteps;
         x = (long long)dx;
@@ -1088,11 +1090,11 @@ __device__ __forceinline__ int in_sphere_near(const int4 t, int pid, const doubl
 /// holds the lock of `tet`, so the finite tet across its facet is not being
 /// rewritten.  Returns 1 (inside), -1 (outside), or 0 if the apex is unusable
 /// (the caller then leaves the test undecided).
-template <bool kNear>
-__device__ __forceinline__ int hull_in_circle_ex(const Tables& T, int tet, int ip, int va, int vb, int vd, int pid,
-                                                 const double* __restrict__ vx, bool sphere, double inv) {
-    const int f = at(ld4(&T.tn(tet)), ip) >> 2;
-    const int4 fv = ld4(&T.tv(f));
+template <bool kNear, class M>
+__device__ __forceinline__ int hull_in_circle_ex(const M& m, int tet, int ip, int va, int vb, int vd, int pid,
+                                                 bool sphere) {
+    const int f = at(m.tn4(tet), ip) >> 2;
+    const int4 fv = m.tv4(f);
     int x = -1;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -1100,15 +1102,15 @@ __device__ __forceinline__ int hull_in_circle_ex(const Tables& T, int tet, int i
         if (w != va && w != vb && w != vd) x = w;
     }
     if (x < 0) return 0;   // kInf is negative
-    const Pt a = ld_vertex(vx, va), b = ld_vertex(vx, vb), d = ld_vertex(vx, vd), xp = ld_vertex(vx, x);
+    const Pt a = m.again(va), b = m.again(vb), d = m.again(vd), xp = m.again(x);
     const int so = sign_of(orient3d_filter(a, b, d, xp).det);
     if (so == 0) return 0;
     if (!kNear && !sphere) return 0;
-    const int ss = sphere ? sign_of(in_sphere_filter_lean(a, b, d, xp, ld_vertex(vx, pid)).det)
-                          : -in_sphere_near(make_int4(va, vb, vd, x), pid, vx, inv);
+    const int ss = sphere ? sign_of(in_sphere_filter_lean(a, b, d, xp, m.again(pid)).det)
+                          : -in_sphere_near(m, make_int4(va, vb, vd, x), pid, m.inv(pid));
     if (ss == -2) return 0;
     if (ss != 0) return ss * so;
-    return in_circle_tiebreak_ex(va, vb, vd, pid, vx);
+    return in_circle_tiebreak_ex(m, va, vb, vd, pid);
 }
 
 /// The conflict test of the fast variant (reference src/triangulation.cpp:588-602,
@@ -1118,35 +1120,32 @@ __device__ __forceinline__ int hull_in_circle_ex(const Tables& T, int tet, int i
 /// lie near enough on its grid, an undecided call is settled inline, an exactly
 /// cospherical one by its tie-break and a point in the plane of a hull facet by
 /// its in-circle test.
-template <bool kNear>
-__device__ __forceinline__ int in_conflict_fast(const Tables& T, int tet, const int4 t, const Pt& p, int pid,
-                                                const double* __restrict__ vx, int ex,
-                                                const double* __restrict__ inv_grid) {
+template <bool kNear, class M>
+__device__ __forceinline__ int in_conflict_fast(const M& m, int tet, const int4 t, const Pt& p, int pid, int ex) {
     const int ip = inf_pos(t);
     if (ip >= 0) {
         const int o0 = ip == 0 ? 2 : (ip == 1 ? 2 : (ip == 2 ? 1 : 0));
         const int o1 = ip == 0 ? 1 : (ip == 1 ? 3 : (ip == 2 ? 0 : 1));
         const int o2 = ip == 0 ? 3 : (ip == 1 ? 0 : (ip == 2 ? 3 : 2));
-        const Pt a = vpt(vx, at(t, o0)), b = vpt(vx, at(t, o1)), d = vpt(vx, at(t, o2));
+        const Pt a = m.point(at(t, o0)), b = m.point(at(t, o1)), d = m.point(at(t, o2));
         const Orient3dFilter f = orient3d_filter(a, b, d, p);
         if (f.certain) return f.det < 0.0 ? CT_IN : 0;   // orient3d = -sign(det)
         if ((ex & EX_ORIENT) && f.det != 0.0) return (f.det < 0.0 ? CT_IN : 0) | CT_UNCERTAIN;
         if (ex & EX_ORIENT) {
-            const int h = hull_in_circle_ex<kNear>(T, tet, ip, at(t, o0), at(t, o1), at(t, o2), pid, vx, ex & EX_SPHERE,
-                                                   kNear ? inv_grid[T.vset[pid]] : 0.0);
+            const int h = hull_in_circle_ex<kNear>(m, tet, ip, at(t, o0), at(t, o1), at(t, o2), pid, ex & EX_SPHERE);
             if (h != 0) return (h > 0 ? CT_IN : 0) | CT_UNCERTAIN | CT_TIE;
         }
         return CT_UNDECIDED;
     }
-    const Pt a = vpt(vx, t.x), b = vpt(vx, t.y), c = vpt(vx, t.z), d = vpt(vx, t.w);
+    const Pt a = m.point(t.x), b = m.point(t.y), c = m.point(t.z), d = m.point(t.w);
     const InSphereFilter f = in_sphere_filter_lean(a, b, c, d, p);
     if (f.certain) return f.det < 0.0 ? CT_IN : 0;   // in_sphere = -sign(det)
     int s = 0;
     if (ex & EX_SPHERE) s = -sign_of(f.det);
-    else s = kNear ? in_sphere_near(t, pid, vx, inv_grid[T.vset[pid]]) : 2;
+    else s = kNear ? in_sphere_near(m, t, pid, m.inv(pid)) : 2;
     if (s == 2) return CT_UNDECIDED;
     if (s != 0) return (s > 0 ? CT_IN : 0) | CT_UNCERTAIN;
-    return (in_sphere_tiebreak_ex(t, pid, vx) > 0 ? CT_IN : 0) | CT_UNCERTAIN | CT_TIE;
+    return (in_sphere_tiebreak_ex(m, t, pid) > 0 ? CT_IN : 0) | CT_UNCERTAIN | CT_TIE;
 }
 
 enum : int { AI_DONE = 0, AI_RETRY = 1, AI_LEAVE = 2, AI_DEFER = 3 };
@@ -1643,7 +1642,8 @@ __global__ void __launch_bounds__(256) k_level_items(const int32_t* __restrict__
         int lev = stride - 1;
         while (b[lev] > v) --lev;
         const bool first_tet = v == sk.x || v == sk.y || v == sk.z || v == sk.w;
-        items[base[int64_t(lev) * nsets + set] + (v - b[lev])] = first_tet ? -1 : v;
+        const int to = base[int64_t(lev) * nsets + set];   // < 0: k_coarse inserts the level
+        if (to >= 0) items[to + (v - b[lev])] = first_tet ? -1 : v;
         int lo = lev, hi = b[lev];
         while (lo > 0 && b[lo] == hi) --lo;   // the level before that has points: [b[lo], hi)
         int g;
@@ -3009,10 +3009,21 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
     // order of insertions does not matter).
     auto run_async = [&]() -> int {
         // Items: level by level, each set's vertices of the level together.
-        std::vector<int> ctl(size_t(2) * size_t(nlev) + size_t(nlev) * size_t(nsets), 0);
+        std::vector<int> ctl(size_t(2) * size_t(nlev) + size_t(nlev) * size_t(nsets) + size_t(nsets), 0);
         int* m_of = ctl.data();
         int* first_of = ctl.data() + nlev;
         int* base = ctl.data() + 2 * nlev;
+        int* coarse = base + size_t(nlev) * size_t(nsets);   // levels of each set that k_coarse inserts
+        // (Not under a caller's limits, which are on the tables and on a group's scratch.)
+        // Nor for more sets than the GPU has SMs: a block inserts slower than the GPU does
+        // when other sets keep it busy.
+        const bool use_coarse = own.ok && nsets <= kNumSMs && opt.walk_limit <= 0 && opt.cavity_capacity <= 0 && opt.tet_capacity <= 0;
+        for (int st = 0; use_coarse && st < nsets; ++st) {
+            const std::vector<int>& L = levels[size_t(st)];
+            int k = std::min(int(L.size()) - 1, coarse_levels(h_off[st + 1] - h_off[st], growth));
+            while (k > 0 && L[size_t(k)] > kCoarseCap) --k;
+            coarse[st] = k > 0 && L[size_t(k)] >= 8 ? k : 0;
+        }
         int total = 0;
         std::vector<int64_t> groups_of(static_cast<size_t>(nlev), 0);
         std::vector<int> sets_of(static_cast<size_t>(nlev), 0);
@@ -3022,6 +3033,10 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
             for (int st = 0; st < nsets; ++st) {
                 const std::vector<int>& L = levels[size_t(st)];
                 if (int(L.size()) - 1 <= lev) continue;
+                if (lev < coarse[st]) {
+                    base[size_t(lev) * size_t(nsets) + size_t(st)] = -1;
+                    continue;
+                }
                 const int cnt = L[size_t(lev) + 1] - L[size_t(lev)];
                 base[size_t(lev) * size_t(nsets) + size_t(st)] = total;
                 total += cnt;
@@ -3043,7 +3058,7 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
         D3G_TRY(defer.alloc(size_t(nv), s));
         for (auto& l : left) D3G_TRY(l.alloc(size_t(nv), s));
         D3G_TRY(pool.alloc(size_t(kMaxGroups), s));
-        D3G_TRY(cnt.alloc(size_t(4) * size_t(nlev + kLastPasses + 1) + 1, s));
+        D3G_TRY(cnt.alloc(size_t(4) * size_t(nlev + kLastPasses + 1) + 4, s));
         D3G_CUDA(cudaMemcpyAsync(dctl.p, ctl.data(), sizeof(int) * ctl.size(), cudaMemcpyHostToDevice, s));
         D3G_CUDA(cudaMemsetAsync(pool.p, 0, sizeof(int4) * size_t(kMaxGroups), s));
         D3G_CUDA(cudaMemsetAsync(cnt.p, 0, sizeof(int) * cnt.n, s));
@@ -3068,11 +3083,13 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
                                                         own.ok ? own.keys.p : nullptr, own.curve_bits, vx.p, nv,
                                                         items.p, guide.p);
         own.keys.release();
-        // Per level: the queue head, the points left, the head of the pass over those.
-        auto head_of = [&](int lev) { return cnt.p + 4 * lev; };
-        auto n_left_of = [&](int lev) { return cnt.p + 4 * lev + 1; };
-        auto left_of = [&](int lev) { return left[lev & 1].p; };
+        // Lists of points left, and per list the head of the queue whose points it gets, how
+        // many it has and the head of the pass over them.
+        auto head_of = [&](int k) { return cnt.p + 4 * k; };
+        auto n_left_of = [&](int k) { return cnt.p + 4 * k + 1; };
+        auto left_of = [&](int k) { return left[k & 1].p; };
         int* n_defer = cnt.p + (cnt.n - 1);
+        int list = 0;
         GroupArgs A{};
         A.lock = alock.p;
         A.guide = guide.p;
@@ -3091,10 +3108,12 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
             // without using them stay within the table's room for them.
             A.ngroups = std::max(1, std::min({ngroups, kNumSMs * kGroupBlocks * (kGroupThreads / G), nv / kPoolSlots}));
             const unsigned grid = unsigned((A.ngroups + kGroupThreads / G - 1) / (kGroupThreads / G));
-            auto* kernel = G == 8 ? (near ? k_insert_groups<8, true> : k_insert_groups<8, false>)
-                                  : (G == 16 ? (near ? k_insert_groups<16, true> : k_insert_groups<16, false>)
-                                             : (near ? k_insert_groups<32, true> : k_insert_groups<32, false>));
-            kernel<<<grid, kGroupThreads, 0, s>>>(T, A, Rd, vx.p);
+            auto* kernel = G == 8 ? (near ? k_insert_groups<8, true, 64, kGroupThreads> : k_insert_groups<8, false, 64, kGroupThreads>)
+                         : (G == 16 ? (near ? k_insert_groups<16, true, 128, kGroupThreads> : k_insert_groups<16, false, 128, kGroupThreads>)
+                                    : (near ? k_insert_groups<32, true, 256, kGroupThreads> : k_insert_groups<32, false, 256, kGroupThreads>));
+            const size_t scratch = G == 8 ? sizeof(GroupScratch<8, 64>) * 16
+                                          : (G == 16 ? sizeof(GroupScratch<16, 128>) * 8 : sizeof(GroupScratch<32, 256>) * 4);
+            kernel<<<grid, kGroupThreads, scratch, s>>>(T, A, Rd, vx.p);
             R.stats.launches_async += 1;
         };
         // The variant that settles undecided tests of near points in 64 bits needs more
@@ -3106,16 +3125,30 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
         for (int st = 0; st < nsets; ++st)
             if (hexact[size_t(st)] & EX_GRID) on_grid += R.set_nv[size_t(st)];
         const bool near_main = 2 * on_grid > nv;
-        auto left_pass = [&](int lev, int ngroups) {
-            A.items = left_of(lev);
-            A.n_items = n_left_of(lev);
-            A.next = head_of(lev) + 2;
-            A.left = left_of(lev + 1);
-            A.n_left = n_left_of(lev + 1);
+        // A pass of the widest groups over the current list; what it leaves is the next.
+        auto left_pass = [&](int ngroups, bool last = false) {
+            A.items = left_of(list);
+            A.n_items = n_left_of(list);
+            A.next = head_of(list) + 2;
+            ++list;
+            A.left = last ? defer.p : left_of(list);
+            A.n_left = last ? n_defer : n_left_of(list);
             launch(32, ngroups, true);
         };
         if (opt.timing) cudaEventRecord(kev[0], s);
+        if (use_coarse) {
+            NvtxRange nvtx_level("d3g.coarse");
+            A.left = left_of(list);
+            A.n_left = n_left_of(list);
+            const CoarseArgs K{starts, start_stride, dctl.p + (coarse - ctl.data()), nsets, n_defer - 1};
+            auto* kernel = near_main ? k_coarse<true> : k_coarse<false>;
+            D3G_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(CoarseShared))));
+            kernel<<<unsigned(std::min(nsets, kNumSMs)), kCoarseThreads, sizeof(CoarseShared), s>>>(T, A, K, Rd, vx.p);
+            D3G_CUDA(cudaGetLastError());
+            R.stats.launches_async += 1;
+        }
         for (int lev = 0; lev < nlev; ++lev) {
+            if (m_of[lev] == 0 && lev < nlev - 1 && !opt.validate) continue;
             char level_name[32];
             std::snprintf(level_name, sizeof level_name, "d3g.level %d", lev);
             NvtxRange nvtx_level(level_name);
@@ -3128,16 +3161,19 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
             const int G = group_lanes(groups_of[size_t(lev)]);
             A.items = items.p + first_of[lev];
             A.n_items = dctl.p + lev;
-            A.next = head_of(lev);
+            A.next = head_of(list);
             // What narrower groups leave goes to wider ones at once; what those leave
             // (points in each other's way) waits for the next level's pass.
-            A.left = left_of(G < 32 ? lev : lev + 1);
-            A.n_left = n_left_of(G < 32 ? lev : lev + 1);
-            // (The first level grows from one tet: there the guides are nearer.  A caller's
-            // walk limit holds for an insertion's whole walk.)
-            if (lev > 0 && opt.walk_limit <= 0) k_locate<<<grid_for(m_of[lev], 128), 128, 0, s>>>(T, A, vx.p);
-            launch(G, int(std::min<int64_t>(groups_of[size_t(lev)], 1 << 24)), near_main);
-            if (lev > 0 || G < 32) left_pass(lev, kNumSMs * (kGroupThreads / 32));
+            A.left = left_of(G < 32 ? list : list + 1);
+            A.n_left = n_left_of(G < 32 ? list : list + 1);
+            if (m_of[lev] > 0) {
+                // (The first level grows from one tet: there the guides are nearer.  A
+                // caller's walk limit holds for an insertion's whole walk.)
+                if ((lev > 0 || use_coarse) && opt.walk_limit <= 0)
+                    k_locate<<<grid_for(m_of[lev], 128), 128, 0, s>>>(T, A, vx.p);
+                launch(G, int(std::min<int64_t>(groups_of[size_t(lev)], 1 << 24)), near_main);
+                left_pass(kNumSMs * (kGroupThreads / 32));
+            }
             D3G_CUDA(cudaGetLastError());
             if (trace) {
                 cudaEventRecord(ev1, s);
@@ -3146,7 +3182,7 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
                 cudaEventElapsedTime(&ms, ev0, ev1);
                 int c[4] = {0, 0, 0, 0}, nd = 0;
                 unsigned long long as[7], ht[2];
-                cudaMemcpy(c, cnt.p + 4 * lev, sizeof c, cudaMemcpyDeviceToHost);
+                cudaMemcpy(c, cnt.p + 4 * std::max(list - 1, 0), sizeof c, cudaMemcpyDeviceToHost);
                 cudaMemcpy(&nd, n_defer, sizeof nd, cudaMemcpyDeviceToHost);
                 cudaMemcpy(as, astats.p, sizeof as, cudaMemcpyDeviceToHost);
                 cudaMemcpy(ht, totals.p, sizeof ht, cudaMemcpyDeviceToHost);
@@ -3161,22 +3197,31 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
             if (lev == nlev - 1) {
                 // The points still left, with fewer and fewer groups in the way of one another;
                 // the last pass hands what remains to the full variant.
-                for (int k = 0; k < kLastPasses; ++k) {
-                    if (k == kLastPasses - 1) break;
-                    left_pass(nlev + k, kNumSMs * (kGroupThreads / 32) >> (2 * k));
-                }
-                A.items = left_of(nlev + kLastPasses - 1);
-                A.n_items = n_left_of(nlev + kLastPasses - 1);
-                A.next = head_of(nlev + kLastPasses - 1) + 2;
-                A.left = defer.p;
-                A.n_left = n_defer;
-                launch(32, 16, true);   // few in the way of one another
+                for (int k = 0; k < kLastPasses; ++k)
+                    left_pass(std::max(kNumSMs * (kGroupThreads / 32) >> (3 * k), 16), k == kLastPasses - 1);
+            }
+            if (lev == nlev - 1) {
+                // Regions beyond that pass's scratch (and the odd undecided point) get one of
+                // kBigCapacity; what it leaves in turn is for the full variant.
+                auto* kernel = k_insert_groups<32, true, kBigCapacity, 32>;
+                D3G_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              int(sizeof(GroupScratch<32, kBigCapacity>))));
+                A.items = defer.p;
+                A.n_items = n_defer;
+                A.next = n_defer - 2;
+                A.left = A.defer = left_of(0);
+                A.n_left = A.n_defer = n_defer - 3;
+                A.cavity = opt.cavity_capacity > 0 ? cav_normal : kBigCapacity;
+                A.ngroups = std::min(16, std::max(1, nv / kPoolSlots));
+                kernel<<<unsigned(A.ngroups), 32, sizeof(GroupScratch<32, kBigCapacity>), s>>>(T, A, Rd, vx.p);
+                D3G_CUDA(cudaGetLastError());
+                R.stats.launches_async += 1;
             }
             if (opt.validate || lev == nlev - 1) {
                 int nd = 0;
                 uint32_t hs = 0;
                 if (opt.timing) cudaEventRecord(kev[1], s);
-                D3G_CUDA(cudaMemcpyAsync(&nd, n_defer, sizeof nd, cudaMemcpyDeviceToHost, s));
+                D3G_CUDA(cudaMemcpyAsync(&nd, A.n_defer, sizeof nd, cudaMemcpyDeviceToHost, s));
                 D3G_CUDA(cudaMemcpyAsync(&hs, status.p, sizeof hs, cudaMemcpyDeviceToHost, s));
                 D3G_CUDA(cudaStreamSynchronize(s));
                 if (hs != 0) {
@@ -3189,8 +3234,8 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
                     cudaEventElapsedTime(&am, kev[0], kev[1]);
                     R.stats.ms_async += am;
                 }
-                D3G_TRY(finish_points(defer.p, nd));
-                D3G_CUDA(cudaMemsetAsync(n_defer, 0, sizeof(int), s));
+                D3G_TRY(finish_points(A.defer, nd));
+                D3G_CUDA(cudaMemsetAsync(A.n_defer, 0, sizeof(int), s));
                 if (opt.validate) D3G_TRY(validate_tables("after", lev));
                 if (opt.timing) cudaEventRecord(kev[0], s);
             }

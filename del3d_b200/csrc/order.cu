@@ -181,9 +181,9 @@ __device__ __forceinline__ unsigned long long hilbert3(unsigned x, unsigned y, u
     return spread3(x) << 2 | spread3(y) << 1 | spread3(z);
 }
 
-/// The key of every point.  A point's level is how often its hash, as a
-/// fraction of 2^32, can be multiplied by `growth` before it reaches 1, counted
-/// from the finest level: a level is then growth times the points before it.
+/// The key of every point.  A point's level comes from its hash as a fraction of
+/// 2^32: the coarse levels share the part below kCoarsePoints / n, each `growth`
+/// times the points before it, the others the part above, likewise.
 __global__ void __launch_bounds__(256) k_order_keys(const double* __restrict__ xyz, const int64_t* __restrict__ off,
                                                     int nsets, int64_t n, const unsigned long long* __restrict__ box,
                                                     int growth, int bits, int level_bits,
@@ -207,14 +207,19 @@ __global__ void __launch_bounds__(256) k_order_keys(const double* __restrict__ x
             q[a] = f > 0.0 ? min(unsigned(f), (1u << bits) - 1) : 0u;
             h = mix64(h + 0x9E3779B97F4A7C15ull + coord_bits(x));
         }
-        const int nlev = order_levels(off[set + 1] - off[set], growth);
-        uint32_t r = uint32_t(h >> 32);
-        int down = 0;   // levels below the finest
-        while (down + 1 < nlev && uint64_t(r) * unsigned(growth) < (uint64_t(1) << 32)) {
-            r *= unsigned(growth);
-            ++down;
+        const int64_t ns = off[set + 1] - off[set];
+        const int nlev = order_levels(ns, growth), ncoarse = coarse_levels(ns, growth);
+        const uint64_t one = uint64_t(1) << 32, t0 = ns <= kCoarsePoints ? one : one * kCoarsePoints / uint64_t(ns);
+        uint64_t r = h >> 32;
+        int lev;
+        if (r < t0) {
+            lev = ncoarse - 1;
+            for (; lev > 0 && r * unsigned(growth) < t0; --lev) r *= unsigned(growth);
+        } else {
+            lev = ncoarse;
+            for (uint64_t t = t0 * unsigned(growth); lev < nlev - 1 && r >= t; t *= unsigned(growth)) ++lev;
         }
-        const unsigned long long code = (unsigned long long)set << level_bits | unsigned(nlev - 1 - down);
+        const unsigned long long code = (unsigned long long)set << level_bits | unsigned(lev);
         keys[p] = code << (3 * bits) | hilbert3(q[0], q[1], q[2], bits);
         idx[p] = int32_t(p);
     }

@@ -11,15 +11,27 @@ namespace d3g {
 /// Levels a build's own order uses at most (growth 2 of 2^27 points: 22).
 constexpr int kMaxOrderLevels = 32;
 
-/// Levels of a set of n points when each level is `growth` times the points
-/// before it: n, n / growth, ... while at least 64 points are left (as the
-/// reference's multiscale split, src/spatial_sort.cpp:130-137, at growth 8).
-__host__ __device__ inline int order_levels(int64_t n, int growth) {
+/// The coarsest levels of every set together have about this many points (fewer
+/// if the set has), so that one block can build them in shared memory
+/// (k_coarse), which has room for kCoarseCap: the number of points in a level
+/// comes from a hash and scatters by its square root.
+constexpr int kCoarsePoints = 790;
+constexpr int kCoarseCap = 880;
+
+/// The first levels of a set of n points: the ones up to kCoarsePoints points, a
+/// half (1 / growth) of what is left each while 64 points are, as the reference's
+/// multiscale split at growth 8 (src/spatial_sort.cpp:130-137).
+__host__ __device__ inline int coarse_levels(int64_t n, int growth) {
     int k = 1;
-    while (n >= 64 && k < kMaxOrderLevels) {
-        n /= growth;
-        ++k;
-    }
+    for (int64_t m = n < kCoarsePoints ? n : kCoarsePoints; m >= 64; m /= growth) ++k;
+    return k;
+}
+
+/// All levels of a set of n points: behind the coarse ones, levels that make the
+/// points in so far `growth` times as many.
+__host__ __device__ inline int order_levels(int64_t n, int growth) {
+    int k = coarse_levels(n, growth);
+    for (int64_t m = kCoarsePoints; m < n && k < kMaxOrderLevels; m *= growth) ++k;
     return k;
 }
 
