@@ -2049,7 +2049,7 @@ __global__ void k_cell_flags(const int4* __restrict__ rec, int ntet,
 }
 
 /// Writes the flagged tets, mapped to input point indices and canonicalised,
-/// plus (khi given) their sort keys (shifted by one so the infinite vertex, -1,
+/// plus their sort keys (shifted by one so the infinite vertex, -1,
 /// is 0).
 __global__ void k_cells_out(const int4* __restrict__ rec, const int32_t* __restrict__ flag,
                             const int32_t* __restrict__ pos, int ntet,
@@ -2069,11 +2069,9 @@ __global__ void k_cells_out(const int4* __restrict__ rec, const int32_t* __restr
         q = canonical(q);
         const int o = pos[t];
         cells[o] = q;
-        if (khi) {
-            khi[o] = ((unsigned long long)(uint32_t(q.x + 1)) << kbits) | uint32_t(q.y + 1);
-            klo[o] = ((unsigned long long)(uint32_t(q.z + 1)) << kbits) | uint32_t(q.w + 1);
-            idx[o] = o;
-        }
+        khi[o] = ((unsigned long long)(uint32_t(q.x + 1)) << kbits) | uint32_t(q.y + 1);
+        klo[o] = ((unsigned long long)(uint32_t(q.z + 1)) << kbits) | uint32_t(q.w + 1);
+        idx[o] = o;
     }
 }
 
@@ -2086,31 +2084,61 @@ __global__ void k_cells_out(const int4* __restrict__ rec, const int32_t* __restr
 // bucket - the few cells whose smallest vertex is that point - is sorted by its
 // other three vertices.
 
-/// One thread sorts a bucket of up to kBucketThread cells, one block one of up
+/// Buckets of up to kBucketThread cells are sorted many to a block, one block sorts one of up
 /// to kBucketBlock; a larger bucket leaves the whole output to the radix sort.
 constexpr int kBucketThread = 32;
 constexpr int kBucketBlock = 2048;
 
-__device__ __forceinline__ int cell_bucket(const int4& q, const int32_t* __restrict__ cset,
-                                           const int64_t* __restrict__ off, int64_t o) {
-    return int(cset ? off[cset[o]] : 0) + q.x;
+/// The finite cells, mapped to input indices and canonicalised, in any order, with
+/// their buckets, which it also counts.  Each block packs the cells of
+/// kEmitTets tet slots behind one another (one atomic for their place), so the
+/// slots are read once and no flags or scan over them are needed.  Bound by the
+/// gathers of the vertices' input indices and the bucket counts, one atomic a cell.
+constexpr int kEmitThreads = 256, kEmitItems = 8, kEmitTets = kEmitThreads * kEmitItems;
+__global__ void __launch_bounds__(kEmitThreads) k_cells_emit(const int4* __restrict__ rec, int ntet,
+                                                             const int32_t* __restrict__ vert_point,
+                                                             const int32_t* __restrict__ vset,
+                                                             const int64_t* __restrict__ off, bool sets,
+                                                             int4* __restrict__ cells, int* __restrict__ bucket,
+                                                             int* __restrict__ count, int* total) {
+    typedef cub::BlockScan<int, kEmitThreads> BlockScan;
+    __shared__ typename BlockScan::TempStorage tmp;
+    __shared__ int base;
+    int4 q[kEmitItems];
+    unsigned mask = 0;
+    const int first = int(blockIdx.x) * kEmitTets + int(threadIdx.x);
+#pragma unroll
+    for (int k = 0; k < kEmitItems; ++k) {
+        const int t = first + k * kEmitThreads;
+        q[k] = t < ntet ? rec[2 * int64_t(t)] : make_int4(0, 0, 0, 0);
+        if (q[k].x != q[k].y && inf_pos(q[k]) < 0) mask |= 1u << k;
+    }
+    int at_ = 0, sum = 0;
+    BlockScan(tmp).ExclusiveSum(__popc(mask), at_, sum);
+    if (threadIdx.x == 0) base = atomicAdd(total, sum);
+    __syncthreads();
+    int o = base + at_;
+#pragma unroll
+    for (int k = 0; k < kEmitItems; ++k) {
+        if (!(mask >> k & 1u)) continue;
+        const int4 c = q[k];
+        const int4 w = canonical(make_int4(vert_point[c.x], vert_point[c.y], vert_point[c.z], vert_point[c.w]));
+        const int b = (sets ? int(off[vset[c.x]]) : 0) + w.x;
+        cells[o] = w;
+        bucket[o] = b;
+        atomicAdd(count + b, 1);
+        ++o;
+    }
 }
 
-__global__ void k_bucket_count(const int4* __restrict__ cells, const int32_t* __restrict__ cset,
-                               const int64_t* __restrict__ off, int64_t n, int* __restrict__ count) {
-    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-         i += int64_t(gridDim.x) * blockDim.x)
-        atomicAdd(count + cell_bucket(cells[i], cset, off, i), 1);
-}
-
-__global__ void k_bucket_place(const int4* __restrict__ cells, const int32_t* __restrict__ cset,
-                               const int64_t* __restrict__ off, int64_t n, const int* __restrict__ start,
-                               int* __restrict__ fill, int4* __restrict__ out) {
-    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-         i += int64_t(gridDim.x) * blockDim.x) {
-        const int4 q = cells[i];
-        const int b = cell_bucket(q, cset, off, i);
-        out[start[b] + atomicAdd(fill + b, 1)] = q;
+/// Puts every cell in its bucket; `count` runs down to zero again.
+__global__ void k_bucket_place(const int4* __restrict__ cells, const int* __restrict__ bucket,
+                               const int* __restrict__ total, const int* __restrict__ start, int* __restrict__ count,
+                               int4* __restrict__ out) {
+    const int n = *total;
+    for (int i = int(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int b = bucket[i];
+        out[start[b] + atomicSub(count + b, 1) - 1] = cells[i];
     }
 }
 
@@ -2120,30 +2148,53 @@ __device__ __forceinline__ bool cell_tail_less(const int4& a, const int4& b) {
     return a.w < b.w;
 }
 
-/// One thread per bucket: insertion sort by the last three vertices.  A
-/// bucket of more than kBucketThread cells is listed in `mid` for
-/// k_bucket_sort_block, one of more than kBucketBlock only raises `big`.
-__global__ void k_bucket_sort(int4* __restrict__ cells, const int* __restrict__ start, int nb,
-                              int* __restrict__ mid, int* __restrict__ nmid, int* __restrict__ big) {
-    for (int b = int(blockIdx.x) * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x) {
-        const int lo = start[b], hi = start[b + 1];
-        if (hi - lo > kBucketBlock) {
-            *big = 1;
+/// Sorts the buckets of up to kBucketThread cells by the last three vertices, 128
+/// buckets a block: the block loads their cells in order into shared memory, and
+/// each cell, one thread each, counts the cells of its bucket that come before it
+/// and goes to that place.  All cells do about the same work, where a thread that
+/// sorts a bucket by itself keeps its warp waiting for the largest (664 us in
+/// place in device memory for 11.4 M cells, 1056 us in shared memory).  A bucket of
+/// more cells is listed in `mid` for k_bucket_sort_block, one of more than
+/// kBucketBlock only raises `big`.
+constexpr int kBucketStage = 1024;
+__global__ void __launch_bounds__(128) k_bucket_sort(int4* __restrict__ cells, const int* __restrict__ start, int nb,
+                                                     int* __restrict__ mid, int* __restrict__ nmid,
+                                                     int* __restrict__ big) {
+    __shared__ int4 stage[kBucketStage];
+    __shared__ int lo_of[129];
+    __shared__ uint8_t owner[kBucketStage];
+    const int b0 = int(blockIdx.x) * 128, nbuckets = min(128, nb - b0);
+    for (int k = int(threadIdx.x); k <= nbuckets; k += 128) lo_of[k] = start[b0 + k];
+    __syncthreads();
+    if (int(threadIdx.x) < nbuckets) {
+        const int n = lo_of[threadIdx.x + 1] - lo_of[threadIdx.x];
+        if (n > kBucketBlock) *big = 1;
+        else if (n > kBucketThread) mid[atomicAdd(nmid, 1)] = b0 + int(threadIdx.x);
+    }
+    // Whole buckets, as many as fit the stage, at a time.
+    for (int k0 = 0; k0 < nbuckets;) {
+        int k1 = k0;
+        while (k1 < nbuckets && lo_of[k1 + 1] - lo_of[k0] <= kBucketStage) ++k1;
+        if (k1 == k0) {          // one bucket beyond the stage: listed above
+            ++k0;
             continue;
         }
-        if (hi - lo > kBucketThread) {
-            mid[atomicAdd(nmid, 1)] = b;
-            continue;
+        const int first = lo_of[k0], n = lo_of[k1] - first;
+        for (int i = int(threadIdx.x); i < n; i += 128) stage[i] = cells[first + i];
+        if (int(threadIdx.x) >= k0 && int(threadIdx.x) < k1)
+            for (int i = lo_of[threadIdx.x] - first; i < lo_of[threadIdx.x + 1] - first; ++i)
+                owner[i] = uint8_t(threadIdx.x);
+        __syncthreads();
+        for (int i = int(threadIdx.x); i < n; i += 128) {
+            const int k = owner[i], lo = lo_of[k] - first, hi = lo_of[k + 1] - first;
+            if (hi - lo < 2 || hi - lo > kBucketThread) continue;
+            const int4 x = stage[i];
+            int rank = lo;
+            for (int j = lo; j < hi; ++j) rank += cell_tail_less(stage[j], x) ? 1 : 0;
+            cells[first + rank] = x;
         }
-        for (int i = lo + 1; i < hi; ++i) {
-            const int4 x = cells[i];
-            int j = i - 1;
-            while (j >= lo && cell_tail_less(x, cells[j])) {
-                cells[j + 1] = cells[j];
-                --j;
-            }
-            cells[j + 1] = x;
-        }
+        __syncthreads();
+        k0 = k1;
     }
 }
 
@@ -3285,9 +3336,9 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
     D3G_CUDA(cudaMemcpyAsync(&ntet, tet_count.p, sizeof ntet, cudaMemcpyDeviceToHost, s));
     D3G_CUDA(cudaStreamSynchronize(s));
     const int kbits = bits_for(uint64_t(max_n) + 1);
-    for (int pass = 0; pass < (single && opt.want_all_cells ? 2 : 1); ++pass) {
-        const bool with_inf = pass == 1;
-        DevBuf<int32_t> flag, pos, idx, cset;
+    // Every cell's flag and place among the flagged (for the radix sorts).
+    DevBuf<int32_t> flag, pos;
+    auto flag_cells = [&](bool with_inf, int64_t* n) -> int {
         D3G_TRY(flag.alloc(size_t(ntet), s));
         D3G_TRY(pos.alloc(size_t(ntet), s));
         k_cell_flags<<<grid_for(ntet, 256), 256, 0, s>>>(rec.p, ntet, with_inf, flag.p);
@@ -3296,66 +3347,60 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
         D3G_CUDA(cudaMemcpyAsync(&last_pos, pos.p + ntet - 1, sizeof(int), cudaMemcpyDeviceToHost, s));
         D3G_CUDA(cudaMemcpyAsync(&last_flag, flag.p + ntet - 1, sizeof(int), cudaMemcpyDeviceToHost, s));
         D3G_CUDA(cudaStreamSynchronize(s));
-        const int64_t nc = int64_t(last_pos) + last_flag;
+        *n = int64_t(last_pos) + last_flag;
+        return D3G_OK;
+    };
+    auto radix_cells = [&](bool with_inf, DevBuf<int4>& out, int64_t* n) -> int {
         DevBuf<int4> raw;
         DevBuf<unsigned long long> khi, klo;
-        D3G_TRY(raw.alloc(size_t(nc), s));
-        D3G_TRY(khi.alloc(size_t(nc), s));
-        D3G_TRY(klo.alloc(size_t(nc), s));
-        D3G_TRY(idx.alloc(size_t(nc), s));
-        if (!single) D3G_TRY(cset.alloc(size_t(nc), s));
-        if (!with_inf) {
-            // Buckets by first vertex; the radix sort of every cell only if a
-            // bucket is too large for one thread.
-            k_cells_out<<<grid_for(ntet, 256), 256, 0, s>>>(rec.p, flag.p, pos.p, ntet, vert_point.p, vset.p,
-                                                            kbits, raw.p, nullptr, nullptr, nullptr,
-                                                            single ? nullptr : cset.p);
-            DevBuf<int> bstart, bfill, big, mid;
-            D3G_TRY(bstart.alloc(size_t(N) + 1, s));
-            D3G_TRY(bfill.alloc(size_t(N) + 1, s));
-            D3G_TRY(big.alloc(2, s));
-            D3G_TRY(mid.alloc(size_t(nc / (kBucketThread + 1)) + 1, s));
-            D3G_TRY(R.cells.alloc(size_t(nc), s));
-            D3G_CUDA(cudaMemsetAsync(bfill.p, 0, sizeof(int) * (size_t(N) + 1), s));
-            D3G_CUDA(cudaMemsetAsync(big.p, 0, 2 * sizeof(int), s));
-            if (nc > 0) {
-                k_bucket_count<<<grid_for(nc, 256), 256, 0, s>>>(raw.p, single ? nullptr : cset.p, d_off.p, nc,
-                                                                 bfill.p);
-            }
-            D3G_TRY(exclusive_scan(bfill.p, bstart.p, int64_t(N) + 1, s));
-            D3G_CUDA(cudaMemsetAsync(bfill.p, 0, sizeof(int) * (size_t(N) + 1), s));
-            if (nc > 0) {
-                k_bucket_place<<<grid_for(nc, 256), 256, 0, s>>>(raw.p, single ? nullptr : cset.p, d_off.p, nc,
-                                                                 bstart.p, bfill.p, R.cells.p);
-                k_bucket_sort<<<grid_for(N, 128), 128, 0, s>>>(R.cells.p, bstart.p, N, mid.p, big.p + 1, big.p);
-            }
-            int hbig[2] = {0, 0};
-            D3G_CUDA(cudaMemcpyAsync(hbig, big.p, sizeof hbig, cudaMemcpyDeviceToHost, s));
-            if (!single) {
-                DevBuf<int64_t> coff;
-                D3G_TRY(coff.alloc(size_t(nsets) + 1, s));
-                k_cell_off<<<grid_for(nsets + 1, 128), 128, 0, s>>>(bstart.p, d_off.p, nsets, coff.p);
-                D3G_CUDA(cudaMemcpyAsync(R.cell_off.data(), coff.p, sizeof(int64_t) * (size_t(nsets) + 1),
-                                         cudaMemcpyDeviceToHost, s));
-            }
-            D3G_CUDA(cudaStreamSynchronize(s));
-            R.n_cells = nc;
-            if (single) R.cell_off[1] = nc;
-            if (!hbig[0] && hbig[1] > 0)
-                k_bucket_sort_block<<<unsigned(hbig[1]), 512, 0, s>>>(R.cells.p, bstart.p, mid.p);
-            if (hbig[0]) {
-                k_cells_out<<<grid_for(ntet, 256), 256, 0, s>>>(rec.p, flag.p, pos.p, ntet, vert_point.p, vset.p,
-                                                                kbits, raw.p, khi.p, klo.p, idx.p,
-                                                                single ? nullptr : cset.p);
-                D3G_TRY(sort_cells(raw, khi, klo, idx, single ? nullptr : cset.p, nsets, nc, kbits, R.cells, s));
-            }
-        } else {
-            k_cells_out<<<grid_for(ntet, 256), 256, 0, s>>>(rec.p, flag.p, pos.p, ntet, vert_point.p, vset.p,
-                                                            kbits, raw.p, khi.p, klo.p, idx.p, nullptr);
-            D3G_TRY(sort_cells(raw, khi, klo, idx, nullptr, 1, nc, kbits, R.all, s));
-            R.n_all = nc;
+        DevBuf<int32_t> idx, cset;
+        D3G_TRY(flag_cells(with_inf, n));
+        D3G_TRY(raw.alloc(size_t(*n), s));
+        D3G_TRY(khi.alloc(size_t(*n), s));
+        D3G_TRY(klo.alloc(size_t(*n), s));
+        D3G_TRY(idx.alloc(size_t(*n), s));
+        if (!single) D3G_TRY(cset.alloc(size_t(*n), s));
+        k_cells_out<<<grid_for(ntet, 256), 256, 0, s>>>(rec.p, flag.p, pos.p, ntet, vert_point.p, vset.p, kbits, raw.p,
+                                                        khi.p, klo.p, idx.p, single ? nullptr : cset.p);
+        D3G_TRY(sort_cells(raw, khi, klo, idx, single ? nullptr : cset.p, nsets, *n, kbits, out, s));
+        return D3G_OK;
+    };
+    {
+        // Buckets by first vertex; the radix sort of every cell only if a bucket is
+        // too large for one block.
+        DevBuf<int4> raw;
+        DevBuf<int> bucket, bstart, bcount, ctl, mid;
+        D3G_TRY(raw.alloc(size_t(ntet), s));
+        D3G_TRY(bucket.alloc(size_t(ntet), s));
+        D3G_TRY(bstart.alloc(size_t(N) + 1, s));
+        D3G_TRY(bcount.alloc(size_t(N) + 1, s));
+        D3G_TRY(ctl.alloc(3, s));
+        D3G_TRY(mid.alloc(size_t(ntet / (kBucketThread + 1)) + 1, s));
+        D3G_TRY(R.cells.alloc(size_t(ntet), s));
+        D3G_CUDA(cudaMemsetAsync(bcount.p, 0, sizeof(int) * (size_t(N) + 1), s));
+        D3G_CUDA(cudaMemsetAsync(ctl.p, 0, 3 * sizeof(int), s));
+        k_cells_emit<<<unsigned((ntet + kEmitTets - 1) / kEmitTets), kEmitThreads, 0, s>>>(
+            rec.p, ntet, vert_point.p, vset.p, d_off.p, !single, raw.p, bucket.p, bcount.p, ctl.p);
+        D3G_TRY(exclusive_scan(bcount.p, bstart.p, int64_t(N) + 1, s));
+        k_bucket_place<<<grid_for(ntet, 256), 256, 0, s>>>(raw.p, bucket.p, ctl.p, bstart.p, bcount.p, R.cells.p);
+        k_bucket_sort<<<unsigned((N + 127) / 128), 128, 0, s>>>(R.cells.p, bstart.p, N, mid.p, ctl.p + 2, ctl.p + 1);
+        int hctl[3] = {0, 0, 0};
+        D3G_CUDA(cudaMemcpyAsync(hctl, ctl.p, sizeof hctl, cudaMemcpyDeviceToHost, s));
+        if (!single) {
+            DevBuf<int64_t> coff;
+            D3G_TRY(coff.alloc(size_t(nsets) + 1, s));
+            k_cell_off<<<grid_for(nsets + 1, 128), 128, 0, s>>>(bstart.p, d_off.p, nsets, coff.p);
+            D3G_CUDA(cudaMemcpyAsync(R.cell_off.data(), coff.p, sizeof(int64_t) * (size_t(nsets) + 1),
+                                     cudaMemcpyDeviceToHost, s));
         }
+        D3G_CUDA(cudaStreamSynchronize(s));
+        R.n_cells = hctl[0];
+        if (single) R.cell_off[1] = R.n_cells;
+        if (hctl[1]) D3G_TRY(radix_cells(false, R.cells, &R.n_cells));
+        else if (hctl[2] > 0)
+            k_bucket_sort_block<<<unsigned(hctl[2]), 512, 0, s>>>(R.cells.p, bstart.p, mid.p);
     }
+    if (single && opt.want_all_cells) D3G_TRY(radix_cells(true, R.all, &R.n_all));
     if (single && opt.want_incident) {
         const int64_t m = 4 * R.n_cells;
         DevBuf<int32_t> pt, cell, pt2, cnt;

@@ -232,6 +232,14 @@ cudaError_t device_block_alloc(void** p, size_t bytes, cudaStream_t s, size_t* c
     }
     if (bytes < kBlockCacheMin || d < 0 || d >= kMaxDevices || is_capturing(s))
         return cudaMallocAsync(p, bytes, s);
+    // Sizes in steps of 1/16 to 1/32 of themselves: a build's tables have a few slots
+    // more or less each time, and a request a little above every idle block would go
+    // to the pool, which can hold the thread for hundreds of milliseconds.
+    {
+        size_t step = kBlockCacheMin >> 4;
+        while (step << 5 <= bytes) step <<= 1;
+        bytes = (bytes + step - 1) / step * step;
+    }
     DeviceBlockCache& c = block_cache(d);
     bool hit = false;
     size_t size = 0;

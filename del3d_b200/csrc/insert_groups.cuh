@@ -662,9 +662,7 @@ __global__ void __launch_bounds__(kThreads, kThreads == kGroupThreads ? kGroupBl
 // groups of 32 lanes insert into it (insert_step as everywhere), and the block
 // then writes the finished mesh to the tables, where the later levels go on.
 
-#ifndef CAL
-#define CAL 16
-#endif
+constexpr int kCoarseAlpha = 16;   // (12 and 24 were within 3 %)
 constexpr int kCoarseThreads = 512;
 constexpr int kCoarseVerts = kCoarseCap + 2;                 // and two of the first tet's from outside
 constexpr int kCoarseTets = 8 * kCoarseVerts + 32;
@@ -875,7 +873,7 @@ __global__ void __launch_bounds__(kCoarseThreads, 1)
             // About one group per kCoarseAlpha points in the mesh.
             if (L.sub == 0) {
                 S.nstash = 0;
-                S.open = cnt > 0 && group * CAL <= lb;
+                S.open = cnt > 0 && group * kCoarseAlpha <= lb;
                 S.pool = make_int4(0, 0, 0, 0);
                 S.vlo = 0;
                 S.vhi = n0 + 2;
