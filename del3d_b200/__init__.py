@@ -26,6 +26,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import threading
 from typing import List, Optional, Sequence
 
 import numpy as np
@@ -266,6 +267,51 @@ def _ptr(a: np.ndarray) -> int:
     return a.ctypes.data
 
 
+class _Lent:
+    """One array of an _Owned result, as numpy sees it; the array keeps it alive."""
+
+    def __init__(self, owner, address: int, typestr: str, n: int):
+        self.owner = owner
+        self.__array_interface__ = {"data": (address, False), "shape": (n,), "typestr": typestr, "version": 3}
+
+
+class _Owned:
+    """A result of the C library that lives as long as the arrays made over it.
+
+    The library hands results out in pinned blocks it keeps for reuse; an array
+    over such a block costs nothing, where a copy into fresh pages takes longer
+    than the copy from the device (475 MB of cells of a burst of requests: about
+    100 ms of 170).  Blocks lent this way are bounded by LIMIT bytes in all;
+    beyond it `array` copies."""
+
+    LIMIT = 4 << 30
+    _mu = threading.Lock()
+    _held = 0
+
+    def __init__(self, res, free, nbytes: int):
+        self._res, self._free, self._bytes = res, free, int(nbytes)
+        with _Owned._mu:
+            self.lent = _Owned._held + self._bytes <= _Owned.LIMIT
+            if self.lent:
+                _Owned._held += self._bytes
+
+    def array(self, pointer, dtype, n: int) -> np.ndarray:
+        n = int(n)
+        if n == 0 or not pointer:
+            return np.zeros(0, dtype=dtype)
+        a = np.asarray(_Lent(self, ctypes.addressof(pointer.contents), np.dtype(dtype).str, n))
+        return a if self.lent else a.copy()
+
+    def __del__(self):
+        try:
+            self._free(ctypes.byref(self._res))
+            if self.lent:
+                with _Owned._mu:
+                    _Owned._held -= self._bytes
+        except Exception:
+            pass                # the interpreter is going down
+
+
 def _points(points) -> np.ndarray:
     """(n, 3) float64 C-contiguous view/copy of `points` (array-like or Point3 list)."""
     if isinstance(points, np.ndarray):
@@ -445,26 +491,20 @@ class Delaunay:
         opts.want_incident = int(incident)
         res = _Result()
         _check(lib.d3g_build(_ptr(pts), pts.shape[0], ctypes.byref(opts), ctypes.byref(res)), "build")
-        try:
-            nc, na = res.n_cells, res.n_all
-            self._cells = (np.ctypeslib.as_array(res.cells, shape=(nc * 4,)).reshape(nc, 4).copy()
-                           if nc else np.zeros((0, 4), dtype=np.int32))
-            self._all = (np.ctypeslib.as_array(res.all_cells, shape=(na * 4,)).reshape(na, 4).copy()
-                         if na else np.zeros((0, 4), dtype=np.int32))
-            n = pts.shape[0]
-            if res.incident_offsets:
-                self._inc_off = np.ctypeslib.as_array(res.incident_offsets, shape=(n + 1,)).copy()
-            else:                                   # incident lists not asked for
-                self._inc_off = np.zeros(n + 1, dtype=np.int64)
-            ninc = int(self._inc_off[-1])
-            self._inc = (np.ctypeslib.as_array(res.incident, shape=(ninc,)).copy()
-                         if ninc else np.zeros(0, dtype=np.int32))
-            self._n_vertices = int(res.n_vertices)
-            self.stats = res.stats.as_dict()
-            self.rounds = int(res.stats.rounds)
-            self.device_ms = float(res.device_ms)
-        finally:
-            lib.d3g_result_free(ctypes.byref(res))
+        n, nc, na = pts.shape[0], res.n_cells, res.n_all
+        ninc = int(res.incident_offsets[n]) if res.incident_offsets else 0
+        own = _Owned(res, lib.d3g_result_free, 16 * (nc + na) + 8 * (n + 1) + 4 * ninc)
+        self._cells = own.array(res.cells, np.int32, nc * 4).reshape(nc, 4)
+        self._all = own.array(res.all_cells, np.int32, na * 4).reshape(na, 4)
+        if res.incident_offsets:
+            self._inc_off = own.array(res.incident_offsets, np.int64, n + 1)
+        else:                                       # incident lists not asked for
+            self._inc_off = np.zeros(n + 1, dtype=np.int64)
+        self._inc = own.array(res.incident, np.int32, ninc)
+        self._n_vertices = int(res.n_vertices)
+        self.stats = res.stats.as_dict()
+        self.rounds = int(res.stats.rounds)
+        self.device_ms = float(res.device_ms)
 
     def finite_cells(self) -> np.ndarray:
         """(n_cells, 4) int32 finite tets, canonical order."""
@@ -550,17 +590,14 @@ def build_batch(sets, chunk: int = 0, stats: Optional[dict] = None):
     res = _BatchResult()
     _check(lib.d3g_build_batch(_ptr(xyz), _ptr(offs), len(arrays), ctypes.byref(opts), ctypes.byref(res)),
            "build_batch")
-    try:
-        co = np.ctypeslib.as_array(res.cell_offsets, shape=(len(arrays) + 1,)).copy()
-        nv = np.ctypeslib.as_array(res.n_vertices, shape=(len(arrays),)).copy()
-        total = int(co[-1])
-        cells = (np.ctypeslib.as_array(res.cells, shape=(total * 4,)).reshape(total, 4).copy()
-                 if total else np.zeros((0, 4), dtype=np.int32))
-        if stats is not None:
-            stats.update(res.stats.as_dict())
-            stats["device_ms"] = res.device_ms
-    finally:
-        lib.d3g_batch_result_free(ctypes.byref(res))
+    total = int(res.cell_offsets[len(arrays)])
+    own = _Owned(res, lib.d3g_batch_result_free, 16 * total)
+    co = np.ctypeslib.as_array(res.cell_offsets, shape=(len(arrays) + 1,)).copy()
+    nv = np.ctypeslib.as_array(res.n_vertices, shape=(len(arrays),)).copy()
+    cells = own.array(res.cells, np.int32, total * 4).reshape(total, 4)
+    if stats is not None:
+        stats.update(res.stats.as_dict())
+        stats["device_ms"] = res.device_ms
     return [cells[co[i]:co[i + 1]] for i in range(len(arrays))], [int(v) for v in nv]
 
 
@@ -653,18 +690,15 @@ class Server:
         if st == NOT_READY:
             raise TimeoutError(f"request {ticket} not complete within {timeout} s")
         self._keep.pop(int(ticket), None)
-        try:
-            _check(st, "server_wait")
-            r = Request()
-            nc = res.n_cells
-            r.cells = (np.ctypeslib.as_array(res.cells, shape=(nc * 4,)).reshape(nc, 4).copy()
-                       if nc else np.zeros((0, 4), dtype=np.int32))
-            r.n_vertices = int(res.n_vertices)
-            r.t_submit, r.t_admit, r.t_done = res.t_submit, res.t_admit, res.t_done
-            r.batch_sets = int(res.batch_sets)
-            return r
-        finally:
-            lib.d3g_request_result_free(ctypes.byref(res))
+        own = _Owned(res, lib.d3g_request_result_free, 16 * res.n_cells)
+        _check(st, "server_wait")
+        r = Request()
+        nc = res.n_cells
+        r.cells = own.array(res.cells, np.int32, nc * 4).reshape(nc, 4)
+        r.n_vertices = int(res.n_vertices)
+        r.t_submit, r.t_admit, r.t_done = res.t_submit, res.t_admit, res.t_done
+        r.batch_sets = int(res.batch_sets)
+        return r
 
     def stats(self) -> dict:
         st = _ServerStats()
