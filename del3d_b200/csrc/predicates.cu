@@ -149,6 +149,69 @@ __global__ void __launch_bounds__(256) k_filter_in_sphere(const double* __restri
     }
 }
 
+/// The queued in_sphere calls whose five points lie on a common grid (the largest
+/// power of two all their coordinates are multiples of) and within kNearSteps of
+/// its steps of each other: decided in 64-bit integers (72 kNearSteps^5 < 2^63
+/// bounds the determinant), and a tie by the reference's tie-break, whose
+/// orientations are exact in double at that size.  The others go to `rest`, for
+/// k_exact_in_sphere, whose limbs need 255 registers.  Bound by the gather of the
+/// points and 64-bit multiplies (10^7 queries, a tenth of them degenerate: 83 us here and
+/// 190 for the rest, 730 before; the call 1.88 -> 1.08 ms).
+constexpr double kNearSteps = 2600.0;
+__global__ void __launch_bounds__(128) k_near_in_sphere(const double* __restrict__ pts,
+                                                        const int32_t* __restrict__ idx, int8_t* __restrict__ out,
+                                                        const int64_t* __restrict__ queue,
+                                                        const unsigned long long* qcount, int perturbed,
+                                                        int64_t* rest, unsigned long long* nrest, uint32_t* status) {
+    const int64_t n = int64_t(*qcount), stride = int64_t(gridDim.x) * blockDim.x;
+    const int64_t n_pad = (n + 31) & ~int64_t(31);
+    for (int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; k < n_pad; k += stride) {
+        bool push = false;
+        int64_t q = 0;
+        if (k < n) {
+            q = queue[k];
+            const int32_t* t = idx + 5 * q;
+            const Pt a = load_pt(pts, t[0]), b = load_pt(pts, t[1]), c = load_pt(pts, t[2]), d = load_pt(pts, t[3]),
+                     e = load_pt(pts, t[4]);
+            // The lowest set bit of any coordinate, and the differences in its steps.
+            int emin = 1 << 20;
+            auto low = [&](double x) {
+                if (x != 0.0) {
+                    const Decomp v = decompose(x);
+                    emin = min(emin, v.e + ctz64(v.m));
+                }
+            };
+            low(a.x); low(a.y); low(a.z); low(b.x); low(b.y); low(b.z); low(c.x); low(c.y); low(c.z);
+            low(d.x); low(d.y); low(d.z); low(e.x); low(e.y); low(e.z);
+            bool near = emin >= -200 && emin <= 190;
+            const double inv = near ? scalbn(1.0, -emin) : 0.0;
+            auto step = [&](double x, double y) {
+                const double s = fmul(fsub(x, y), inv);
+                near = near && fabs_(s) <= kNearSteps;
+                return (long long)s;
+            };
+            const long long ax = step(a.x, e.x), ay = step(a.y, e.y), az = step(a.z, e.z);
+            const long long bx = step(b.x, e.x), by = step(b.y, e.y), bz = step(b.z, e.z);
+            const long long cx = step(c.x, e.x), cy = step(c.y, e.y), cz = step(c.z, e.z);
+            const long long dx = step(d.x, e.x), dy = step(d.y, e.y), dz = step(d.z, e.z);
+            push = !near;
+            if (near) {
+                const long long ab = ax * by - bx * ay, bc = bx * cy - cx * by, cd = cx * dy - dx * cy,
+                                da = dx * ay - ax * dy, ac = ax * cy - cx * ay, bd = bx * dy - dx * by;
+                const long long abc = az * bc - bz * ac + cz * ab, bcd = bz * cd - cz * bd + dz * bc,
+                                cda = cz * da + dz * ac + az * cd, dab = dz * ab + az * bd + bz * da;
+                const long long det = ((dx * dx + dy * dy + dz * dz) * abc - (cx * cx + cy * cy + cz * cz) * dab) +
+                                      ((bx * bx + by * by + bz * bz) * cda - (ax * ax + ay * ay + az * az) * bcd);
+                int s = det > 0 ? -1 : (det < 0 ? 1 : 0);   // in_sphere = -sign(det)
+                if (s == 0 && perturbed)
+                    s = in_sphere_perturb<true>(a, b, c, d, e, t[0], t[1], t[2], t[3], t[4], status);
+                out[q] = int8_t(s);
+            }
+        }
+        warp_push(push, q, rest, nrest);
+    }
+}
+
 __global__ void __launch_bounds__(128) k_exact_in_sphere(const double* __restrict__ pts,
                                                          const int32_t* __restrict__ idx,
                                                          int8_t* __restrict__ out,
@@ -318,12 +381,13 @@ int predicates_device(const double* d_pts, int64_t n_pts, const int32_t* d_idx, 
     // Scratch: status word, queue counter, wide-queue counter, and the queues
     // of the exact stage and of its wide tier.
     DevBuf<unsigned long long> counters;
-    D3G_TRY(counters.alloc(3, stream));
-    D3G_CUDA(cudaMemsetAsync(counters.p, 0, 3 * sizeof(unsigned long long), stream));
+    D3G_TRY(counters.alloc(4, stream));
+    D3G_CUDA(cudaMemsetAsync(counters.p, 0, 4 * sizeof(unsigned long long), stream));
     uint32_t* status = reinterpret_cast<uint32_t*>(counters.p);
     unsigned long long* qcount = counters.p + 1;
     unsigned long long* wcount = counters.p + 2;
-    DevBuf<int64_t> queue, wqueue;
+    unsigned long long* ncount = counters.p + 3;   // calls k_near_in_sphere leaves
+    DevBuf<int64_t> queue, rest, wqueue;
     const int64_t wcap = std::min<int64_t>(nq, kWideQueueCap);
     const int blk = 256;
     const bool queued = kind == D3G_ORIENT3D || kind == D3G_IN_SPHERE || kind == D3G_IN_SPHERE_UNPERTURBED;
@@ -339,7 +403,10 @@ int predicates_device(const double* d_pts, int64_t n_pts, const int32_t* d_idx, 
         } else {
             k_filter_in_sphere<<<g, blk, 0, stream>>>(d_pts, n_pts, d_idx, nq, d_out, queue.p,
                                                       qcount, status);
-            k_exact_in_sphere<<<kNumSMs * 8, 128, 0, stream>>>(d_pts, d_idx, d_out, queue.p, qcount,
+            D3G_TRY(rest.alloc(size_t(nq), stream));
+            k_near_in_sphere<<<kNumSMs * 8, 128, 0, stream>>>(d_pts, d_idx, d_out, queue.p, qcount,
+                                                              kind == D3G_IN_SPHERE ? 1 : 0, rest.p, ncount, status);
+            k_exact_in_sphere<<<kNumSMs * 8, 128, 0, stream>>>(d_pts, d_idx, d_out, rest.p, ncount,
                                                                kind == D3G_IN_SPHERE ? 1 : 0, wqueue.p, wcount,
                                                                wcap, status);
         }
