@@ -1928,10 +1928,43 @@ __global__ void k_own_voff(const int32_t* __restrict__ level_start, int nsets, i
         voff[s] = level_start[int64_t(s) * levels];
 }
 
-/// Per set: the first vertex (in insertion order) not collinear with its first
-/// two, and then the first not coplanar with those three.
+/// Per set, one warp: the first vertex (in insertion order) not collinear with its
+/// first two, and then the first not coplanar with those three, looked for among
+/// its first kFirstLook vertices, where nearly every set has them; raises `more`
+/// for a set that has not (the next two kernels, one thread per vertex, then look
+/// through all; they took 574 us for 256 sets of 1.9 M points).
+constexpr int kFirstLook = 1024;
+__global__ void __launch_bounds__(128) k_first_four(const double* __restrict__ vx, const int32_t* __restrict__ voff,
+                                                    int nsets, int* found2, int* found3, int* more, uint32_t* st) {
+    const int set = int((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = int(threadIdx.x & 31u);
+    if (set >= nsets) return;
+    const int base = voff[set], end = voff[set + 1], last = min(end, base + kFirstLook);
+    int v2 = INT_MAX, v3 = INT_MAX;
+    for (int v0 = base + 2; v0 < last && v2 == INT_MAX; v0 += 32) {
+        const int v = v0 + lane;
+        const bool hit = v < last && !collinear(vpt(vx, base), vpt(vx, base + 1), vpt(vx, v), st);
+        const unsigned m = __ballot_sync(kFull, hit);
+        if (m) v2 = v0 + __ffs(int(m)) - 1;
+    }
+    for (int v0 = base + 2; v0 < last && v2 != INT_MAX && v3 == INT_MAX; v0 += 32) {
+        const int v = v0 + lane;
+        const bool hit = v < last && v != v2 &&
+                         orient3d(vpt(vx, base), vpt(vx, base + 1), vpt(vx, v2), vpt(vx, v), st) != 0;
+        const unsigned m = __ballot_sync(kFull, hit);
+        if (m) v3 = v0 + __ffs(int(m)) - 1;
+    }
+    if (lane == 0) {
+        if (v2 != INT_MAX) found2[set] = v2;
+        if (v3 != INT_MAX) found3[set] = v3;
+        if (v3 == INT_MAX && end > last) atomicOr(more, 1);
+    }
+}
+
+/// The same over all vertices, for the sets k_first_four has not settled.
 __global__ void k_find_noncollinear(const double* __restrict__ vx, int nv, const int32_t* __restrict__ vset,
-                                    const int32_t* __restrict__ voff, int* found, uint32_t* st) {
+                                    const int32_t* __restrict__ voff, int* found, const int* __restrict__ more,
+                                    uint32_t* st) {
+    if (*more == 0) return;
     for (int v = int(blockIdx.x) * blockDim.x + threadIdx.x; v < nv; v += gridDim.x * blockDim.x) {
         const int set = vset[v], base = voff[set];
         if (v - base < 2 || v > found[set]) continue;
@@ -1941,7 +1974,8 @@ __global__ void k_find_noncollinear(const double* __restrict__ vx, int nv, const
 
 __global__ void k_find_noncoplanar(const double* __restrict__ vx, int nv, const int32_t* __restrict__ vset,
                                    const int32_t* __restrict__ voff, const int* found2, int* found3,
-                                   uint32_t* st) {
+                                   const int* __restrict__ more, uint32_t* st) {
+    if (*more == 0) return;
     for (int v = int(blockIdx.x) * blockDim.x + threadIdx.x; v < nv; v += gridDim.x * blockDim.x) {
         const int set = vset[v], base = voff[set], v2 = found2[set];
         if (v2 >= voff[set + 1] || v - base < 2 || v == v2 || v > found3[set]) continue;
@@ -2531,11 +2565,15 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
     // ---- each set's first tet: its first four affinely independent vertices ----
     DevBuf<int> found;
     DevBuf<int4> skips;
-    D3G_TRY(found.alloc(2 * size_t(nsets), s));
+    D3G_TRY(found.alloc(2 * size_t(nsets) + 1, s));
     D3G_TRY(skips.alloc(size_t(nsets), s));
     D3G_CUDA(cudaMemsetAsync(found.p, 0x7F, 2 * sizeof(int) * size_t(nsets), s));
-    k_find_noncollinear<<<grid_for(nv, 256), 256, 0, s>>>(vx.p, nv, vset.p, voff.p, found.p, status.p);
-    k_find_noncoplanar<<<grid_for(nv, 256), 256, 0, s>>>(vx.p, nv, vset.p, voff.p, found.p, found.p + nsets,
+    int* more = found.p + 2 * size_t(nsets);
+    D3G_CUDA(cudaMemsetAsync(more, 0, sizeof(int), s));
+    k_first_four<<<unsigned((int64_t(nsets) * 32 + 127) / 128), 128, 0, s>>>(vx.p, voff.p, nsets, found.p,
+                                                                            found.p + nsets, more, status.p);
+    k_find_noncollinear<<<grid_for(nv, 256), 256, 0, s>>>(vx.p, nv, vset.p, voff.p, found.p, more, status.p);
+    k_find_noncoplanar<<<grid_for(nv, 256), 256, 0, s>>>(vx.p, nv, vset.p, voff.p, found.p, found.p + nsets, more,
                                                          status.p);
     k_set_skips<<<grid_for(nsets, 128), 128, 0, s>>>(voff.p, found.p, found.p + nsets, nsets, skips.p);
     std::vector<int4> hskips(static_cast<size_t>(nsets));

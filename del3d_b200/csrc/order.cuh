@@ -19,11 +19,12 @@ constexpr int kCoarsePoints = 790;
 constexpr int kCoarseCap = 880;
 
 /// The first levels of a set of n points: the ones up to kCoarsePoints points, a
-/// half (1 / growth) of what is left each while 64 points are, as the reference's
-/// multiscale split at growth 8 (src/spatial_sort.cpp:130-137).
+/// half (1 / growth) of what is left each while 16 points are (the reference's
+/// multiscale split, src/spatial_sort.cpp:130-137, stops at 64: its levels bound
+/// a walk's length, these also how many groups may insert at a time).
 __host__ __device__ inline int coarse_levels(int64_t n, int growth) {
     int k = 1;
-    for (int64_t m = n < kCoarsePoints ? n : kCoarsePoints; m >= 64; m /= growth) ++k;
+    for (int64_t m = n < kCoarsePoints ? n : kCoarsePoints; m >= 16; m /= growth) ++k;
     return k;
 }
 
