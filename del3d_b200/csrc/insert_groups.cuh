@@ -240,7 +240,7 @@ __device__ __forceinline__ int insert_step(const M& m, Scratch& S, const Lanes<G
         bool walking = live;
         while (__any_sync(kFull, walking)) {
             int4 pv = make_int4(0, 0, 0, 0), pn = pv;
-            if (walking && L.sub >= 4 && L.sub < 8) m.rec(at(tn, L.sub & 3) >> 2, pv, pn);
+            if (!M::kLocal && walking && L.sub >= 4 && L.sub < 8) m.rec(at(tn, L.sub & 3) >> 2, pv, pn);
             h = h * 1664525u + 1013904223u;
             const int s0 = int(h >> 30);
             bool neg = false;
@@ -252,11 +252,16 @@ __device__ __forceinline__ int insert_step(const M& m, Scratch& S, const Lanes<G
             const unsigned cross = L.own(__ballot_sync(kFull, neg)) & 0xFu;
             const unsigned rot = ((cross >> s0) | (cross << (4 - s0))) & 0xFu;
             const int i = (s0 + __ffs(int(rot)) - 1) & 3;
-            const int src = L.gbase + 4 + i;
-            const int4 nv = make_int4(__shfl_sync(kFull, pv.x, src), __shfl_sync(kFull, pv.y, src),
-                                      __shfl_sync(kFull, pv.z, src), __shfl_sync(kFull, pv.w, src));
-            const int4 nn = make_int4(__shfl_sync(kFull, pn.x, src), __shfl_sync(kFull, pn.y, src),
-                                      __shfl_sync(kFull, pn.z, src), __shfl_sync(kFull, pn.w, src));
+            int4 nv, nn;
+            if (M::kLocal) {                              // the chosen neighbour is as near as a shuffle
+                m.rec(cross ? at(tn, i) >> 2 : t, nv, nn);
+            } else {
+                const int src = L.gbase + 4 + i;
+                nv = make_int4(__shfl_sync(kFull, pv.x, src), __shfl_sync(kFull, pv.y, src),
+                               __shfl_sync(kFull, pv.z, src), __shfl_sync(kFull, pv.w, src));
+                nn = make_int4(__shfl_sync(kFull, pn.x, src), __shfl_sync(kFull, pn.y, src),
+                               __shfl_sync(kFull, pn.z, src), __shfl_sync(kFull, pn.w, src));
+            }
             if (!walking) continue;
             if (cross == 0) {
                 walking = false;
