@@ -371,12 +371,12 @@ def run_reference(args):
 
 
 # Measured DRAM traffic of the insertion kernel per point it inserts, from a
-# one-kernel ncu capture: dram__bytes_read.sum + dram__bytes_write.sum of the
-# fast variant's launch at the finest level of a 256-set case of this workload
-# (8.40 GB + 5.77 GB), over the 1,069,032 points that launch inserted.  Traffic
-# per inserted point stays the same at full size: every insertion does the same
-# kind of work on a tet table much larger than L2.
-INSERT_DRAM_BYTES_PER_POINT = 13249.0
+# ncu pass: dram__bytes_read.sum + dram__bytes_write.sum of all k_insert_groups and
+# k_locate launches of a 256-set case of this workload (9.02 GB + 2.94 GB), over its
+# 1,917,906 points.  The same kernel moves more per point on a larger table (13.5 KB
+# at the finest level of a 3 x 10^6-point build), so at full size this is a lower
+# figure.
+INSERT_DRAM_BYTES_PER_POINT = 6233.0
 # Algorithmic bytes of the build per point: the coordinates read (24 B) plus the
 # finite tets written (6.75 per point x 16 B).
 BUILD_BYTES_PER_POINT = 24.0 + 6.75 * 16.0
@@ -646,13 +646,13 @@ def run_ours(args):
         # neighbour record (16 B) of every region tet; the asynchronous pass
         # also writes the new tets (32 B each, one per boundary facet) and the
         # outside tets' back pointers (4 B each).
-        kern = {"k_insert_async": stats.get("ms_async", 0.0), "k_cavity": stats.get("ms_cavity", 0.0),
+        kern = {"k_insert_groups": stats.get("ms_async", 0.0), "k_cavity": stats.get("ms_cavity", 0.0),
                 "k_check": stats.get("ms_check", 0.0), "k_restar": stats.get("ms_restar", 0.0)}
         dom = max(kern, key=kern.get)
         C, F = stats.get("region_tets", 0), stats.get("boundary_facets", 0)
         inserted = max(1, n - len(sets))
         share = min(1.0, stats.get("async_inserted", 0) / inserted)
-        if dom == "k_insert_async":
+        if dom == "k_insert_groups":
             Ca, Fa = C * share, F * share
             model_bytes = 20 * (Ca + Fa) + 16 * Ca + 36 * Fa
             launches = max(1, stats.get("launches_async", 1))
@@ -668,7 +668,7 @@ def run_ours(args):
         alg_bytes = BUILD_BYTES_PER_POINT * units / launches
         achieved = alg_bytes / sec_per_launch / 1e9 if sec_per_launch else 0.0
         model_achieved = (model_bytes / launches) / sec_per_launch / 1e9 if sec_per_launch else 0.0
-        traffic = INSERT_DRAM_BYTES_PER_POINT * units / launches if dom == "k_insert_async" else None
+        traffic = INSERT_DRAM_BYTES_PER_POINT * units / launches if dom == "k_insert_groups" else None
         line = {
             "metric": METRIC, "value": value, "unit": "points/s", "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms_max,

@@ -1,16 +1,22 @@
 // The Delaunay build on the device: del3d::Delaunay::build
-// (src/triangulation.cpp:65-120, 702-769, 932-968) as parallel insertion rounds.
+// (src/triangulation.cpp:65-120, 702-769, 932-968) as parallel insertion.
 //
 // Why a parallel build can return the reference's tets: in_sphere never
 // returns ZERO (symbolic perturbation, src/predicates.cpp:206-232) and the hull
 // conflict rule is fixed (src/triangulation.cpp:588-602), so the set of finite
 // cells is a function of the point set alone, whatever the insertion order.
-// The device therefore inserts many points at once, in rounds:
+// The device therefore inserts many points at once.  By default the build's own
+// order (order.cu) puts the points into levels that double what is in, the
+// first levels of up to 148 sets are built in shared memory (k_coarse), and
+// k_insert_groups inserts the others asynchronously under per-tet locks (see
+// "asynchronous insertion" below and insert_groups.cuh).  What it cannot do goes
+// through k_insert_full, and what that leaves through lockstep rounds, which
+// schedule = 1 uses for every point:
 //
-//   * Points are ordered by the spatial sort (sort.cu) and grouped into BRIO
-//     levels; each level is cut into chunks, one per worker.  A worker inserts
-//     its chunk's points one per round, so the points in flight in a round are
-//     spread along the Hilbert curve, i.e. far apart.
+//   * Points are grouped into levels, along a Hilbert curve in each; each level
+//     is cut into chunks, one per worker.  A worker inserts its chunk's points
+//     one per round, so the points in flight in a round are spread along the
+//     curve, i.e. far apart.
 //   * k_cavity   each worker walks from the last vertex it inserted to the tet
 //                its point conflicts with (visibility walk, exact orient3d),
 //                then grows the conflict region breadth-first with the
@@ -253,8 +259,8 @@ __device__ __noinline__ int hull_in_circle(double ax, double ay, double az, doub
 /// Outcome bits of a conflict test: in conflict; the floating-point filter
 /// could not certify the sign (the set's exact filter value, the exact stage or
 /// a tie-break decided it); the exact value was zero (decided by the symbolic
-/// perturbation, or the hull in-circle test); and, for the fast variant only,
-/// undecided (left to the full variant).
+/// perturbation, or the hull in-circle test); and, from in_conflict_fast only,
+/// undecided (left to k_insert_full, whose test has the exact stage).
 enum : int { CT_IN = 1, CT_UNCERTAIN = 2, CT_TIE = 4, CT_UNDECIDED = 8 };
 
 /// What a set's coordinates make exact (k_set_exact).
@@ -732,29 +738,31 @@ __global__ void __launch_bounds__(128, 8) k_restar(Tables T, Workers W, Round R,
 // ---- asynchronous insertion --------------------------------------------------
 //
 // The rounds above insert in lockstep: every round waits for its slowest
-// worker.  k_insert_async lets every warp run at its own pace instead.  A
-// persistent grid of warps takes the level's chunks from a queue and inserts
-// their points one after another.  An insertion try-locks every tet it reads
+// worker.  k_insert_groups (insert_groups.cuh) and k_insert_full below let every
+// group of lanes, or warp, run at its own pace instead.  A persistent grid takes
+// the level's points from a queue.  An insertion try-locks every tet it reads
 // to decide its conflict region - the region tets and the tets across the
 // region boundary - and holds the locks until its new tets are written, so
 // insertions whose locks succeed touch disjoint tets and commute: the result
 // is that of some sequential order, hence (the tet set does not depend on the
-// insertion order) the canonical set.  A lock held by another warp makes the
-// insertion give back its locks and try again after a back-off; after a few
-// failures, and for a conflict region too large for the warp's scratch, the
-// point is left for the rounds, which finish it.  No warp ever waits while it
-// holds a lock, and every loop is bounded.
+// insertion order) the canonical set.  A lock held by another insertion makes
+// this one give back its locks and try again after a back-off; after some
+// failures, and for a conflict region too large for its scratch, the point is
+// left for a later pass, which finishes it.  The only wait for a lock while
+// others are held is that of the widest groups, which poll a lock of a lower
+// priority kWaitPolls times and then give way; every loop is bounded.
 //
-// Lock word of a tet: 0 free, else (owner << 1) | ring, owner = warp slot + 1;
-// ring = 1 for a tet across the region boundary, 0 for a region tet.  Locks are
+// Lock word of a tet: 0 free, -1 a slot no tet has been written to yet, else
+// (owner << 1) | ring, owner = group or warp slot + 1; ring = 1 for a tet
+// across the region boundary, 0 for a region tet.  Locks are
 // taken with acquire and released with release ordering, and every read of
 // tet data that other warps write goes to L2 (__ldcg), not the SM's L1.
 
 constexpr int kAsyncRetries = 6;
-// Passes of the full variant over a level's left points before the rounds.
+// Passes of k_insert_full over the points left to it before the rounds.
 constexpr int kLeftPasses = 8;
-// BRIO level growth of the build's own order when a set's filters are exact,
-// or when the whole build has fewer than kSmallBuildPoints points.
+// Level growth of a build by lockstep rounds alone, when a set's filters are
+// exact or the whole build has fewer than kSmallBuildPoints points (else 8).
 constexpr int kExactSetGrowth = 4;
 constexpr int64_t kSmallBuildPoints = 65536;
 constexpr int kAsyncWalkLimit = 1 << 14;
@@ -782,7 +790,7 @@ struct AsyncCtx {
     unsigned long long* ekey;       // per warp slot: 3 edge keys per boundary facet (re-star)
     unsigned long long* stats;      // [0] lock conflicts, [1] walk restarts, [2] invalid seeds,
                                     // [3] regions too big, [4] points left, [5] first points left,
-                                    // [6] points deferred by the fast variant
+                                    // [6] points with a test the filters could not decide
 };
 
 using LockRef = cuda::atomic_ref<int, cuda::thread_scope_device>;
@@ -1113,7 +1121,7 @@ __device__ __forceinline__ int hull_in_circle_ex(const M& m, int tet, int ip, in
     return in_circle_tiebreak_ex(m, va, vb, vd, pid);
 }
 
-/// The conflict test of the fast variant (reference src/triangulation.cpp:588-602,
+/// The conflict test of k_insert_groups (reference src/triangulation.cpp:588-602,
 /// as conflict_test) of tet `tet` = t, with its outcome bits; CT_UNDECIDED when
 /// the filter cannot decide and the exact stage is needed.  Call-free: where the
 /// set's coordinates make the filters exact (`ex`: EX_*), or (kNear) the points
@@ -2451,10 +2459,11 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
     // ---- insertion order and duplicate groups ----
     // BRIO levels of the build's own insertion order: each level `growth` times
     // the points before it.  Any order gives the same cells, so the build may
-    // take more and shorter levels than the reference's 8, as it does by default
-    // when a set's coordinates make the filters exact (lattices and coarse grids,
-    // whose long levels collide most) and for a build too small to fill the GPU
-    // (whose levels are inserted chunk by chunk, so shorter ones finish sooner).
+    // take more and shorter levels than the reference's 8: kGroupGrowth in an
+    // asynchronous build; in one by rounds alone, 4 when a set's coordinates make
+    // the filters exact (lattices and coarse grids, whose long levels collide
+    // most) and for a build too small to fill the GPU (whose levels are inserted
+    // chunk by chunk, so shorter ones finish sooner).
     int growth = opt.level_growth;
     SetScan scan;
     D3G_TRY(scan_sets(d_xyz, d_off.p, nsets, n, scan, status.p + 1, s));

@@ -41,8 +41,8 @@ namespace d3g {
 namespace {
 
 /// Device bytes one batch needs, from its point count: tet tables (8 tets per
-/// point at 57 B), per-worker scratch, spatial-sort and output-sort buffers,
-/// plus the big-round scratch and small fixed buffers per batch.  Calibrated
+/// point at 36 B, 60 B when rounds are needed), the order's and the output's
+/// buffers, plus per-worker scratch and small fixed buffers per batch.  Calibrated
 /// against the pool's high-water mark (tests/test_server_gpu.py checks it).
 constexpr int64_t kBytesPerPoint = 1600;
 constexpr int64_t kBytesPerBatch = int64_t(160) << 20;

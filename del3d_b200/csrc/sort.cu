@@ -322,7 +322,8 @@ struct SelTask {
 /// than kSelShared the passes run in device memory; then its keys and a 16-bit
 /// permutation move to shared memory, the remaining passes move only those, and
 /// the elements are permuted once at the end.  k_select for 3 x 10^6
-/// uniform points: 12 launches, 8.3 ms; the whole sort 26.5 -> 22.1 ms.
+/// uniform points: 12 launches, 8.3 ms; the whole sort 26.5 -> 22.1 ms (19 ms
+/// with k_tile_jump).
 __global__ void __launch_bounds__(kSelThreads) k_select(const SelTask* __restrict__ tasks, Elems E,
                                                          Elems B, int32_t* __restrict__ rk) {
     typedef cub::BlockScan<int, kSelThreads> BlockScan;

@@ -156,11 +156,12 @@ typedef struct d3g_options {
     int32_t want_all_cells;  /* also produce all_cells                           */
     int32_t want_incident;   /* also produce incident_cells                      */
     int32_t chunk;           /* > 0: points per worker chunk; < 0: -alpha, one   */
-                             /* worker per alpha earlier points; 0 = default    */
+                             /* worker (asynchronous insertion: one group of    */
+                             /* lanes) per alpha earlier points; 0 = default    */
     int32_t max_rounds;      /* 0 = default                                      */
     int32_t timing;          /* time each insertion kernel with CUDA events      */
     int32_t alpha_small;     /* > 0: densest worker pool (one per alpha_small    */
-                             /* earlier points) while a round's pool stays below */
+                             /* earlier points) while a level's pool stays below */
                              /* one latency wave of the GPU; 0 = never denser;   */
                              /* default 24                                       */
     int32_t split;           /* grow the worker pool within a level as points go */
@@ -192,12 +193,10 @@ typedef struct d3g_options {
                              /* description in d3g_last_error()                  */
     int32_t level_growth;    /* points of a BRIO level over the points before it */
     /* in the build's own insertion order: 8 (the reference's multiscale ratio  */
-    /* 1/8) or 2-7 (more, shorter levels); 0 = default: 4 when a set's          */
-    /* coordinates make the filters exact (lattices, coarse grids) or the build */
-    /* has fewer than 65536 points, else 8.                                     */
-    /* Input with repeated points is always ordered with 8, since the           */
-    /* reference's order decides which copy keeps its index.  The cells do not */
-    /* depend on it.                                                            */
+    /* 1/8) or 2-7 (more, shorter levels); 0 = default: 2 with asynchronous     */
+    /* insertion; with lockstep rounds only, 4 when a set's coordinates make    */
+    /* the filters exact (lattices, coarse grids) or the build has fewer than   */
+    /* 65536 points, else 8.  The cells do not depend on it.                    */
 } d3g_options;
 
 /* What a build did (filled by d3g_build and d3g_build_device). */
@@ -215,9 +214,10 @@ typedef struct d3g_build_stats {
     int64_t walk_steps;      /* with timing: point-location steps over all attempts  */
     int64_t bfs_steps;       /* with timing: conflict-region growth steps (8 tets each) */
     double ms_async;         /* with timing: device time of the asynchronous passes  */
-    int64_t launches_async;  /* asynchronous passes: per level the fast variant,    */
-                             /* then the full one over what it deferred or left,    */
-                             /* repeated while it inserts                           */
+    int64_t launches_async;  /* asynchronous passes: the first levels in shared     */
+                             /* memory, per level k_insert_groups and a pass over   */
+                             /* what is left so far, the last passes, then the full */
+                             /* variant while it inserts                            */
     int64_t async_inserted;  /* points the asynchronous passes inserted              */
     /* Conflict tests (in_sphere, or orient3d against a hull facet) the insertion
      * kernels evaluated, attempts that gave way included; of these, the ones the
@@ -228,8 +228,8 @@ typedef struct d3g_build_stats {
     int64_t uncertain_tests;
     int64_t tie_breaks;
     int64_t max_region_tets;  /* the largest conflict region inserted (tets)         */
-    int64_t deferred_points;  /* points the fast asynchronous variant left to the    */
-                              /* full one (a test its filters could not decide)     */
+    int64_t deferred_points;  /* attempts k_insert_groups gave up at a test its      */
+                              /* filters could not decide                           */
 } d3g_build_stats;
 
 typedef struct d3g_result {
