@@ -24,6 +24,7 @@
 #include "order.cuh"
 
 #include <algorithm>
+#include <vector>
 
 namespace d3g {
 
@@ -229,13 +230,14 @@ __device__ __forceinline__ bool equal_points(const double* __restrict__ xyz, int
     return xyz[3 * i] == xyz[3 * j] && xyz[3 * i + 1] == xyz[3 * j + 1] && xyz[3 * i + 2] == xyz[3 * j + 2];
 }
 
-/// Over the sorted keys: flags the first copy of every point and counts the
-/// others (flags[0]); flags[1] is raised by a run of equal keys too long to be
-/// looked through.
+/// Over the sorted keys (the set above bit `set_shift`): flags the first copy of
+/// every point and counts the others (flags[0], and per set from flags[2] on);
+/// flags[1] is raised by a run of equal keys too long to be looked through.
 __global__ void __launch_bounds__(256) k_first_copies(const double* __restrict__ xyz,
                                                       const unsigned long long* __restrict__ keys,
-                                                      const int32_t* __restrict__ idx, int64_t n,
-                                                      int32_t* __restrict__ first, int* __restrict__ flags) {
+                                                      const int32_t* __restrict__ idx, int64_t n, int nsets,
+                                                      int set_shift, int32_t* __restrict__ first,
+                                                      int* __restrict__ flags) {
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
         const unsigned long long k = keys[i];
         bool copy = false;
@@ -243,14 +245,33 @@ __global__ void __launch_bounds__(256) k_first_copies(const double* __restrict__
         for (; j >= 0 && i - j <= kKeyRun && keys[j] == k; --j) copy = copy || equal_points(xyz, idx[i], idx[j]);
         if (i - j > kKeyRun && j >= 0 && keys[j] == k) atomicOr(flags + 1, 1);
         first[i] = copy ? 0 : 1;
-        if (copy) atomicAdd(flags, 1);
+        if (copy) {
+            atomicAdd(flags, 1);
+            atomicAdd(flags + 2 + (nsets > 1 ? int(k >> set_shift) : 0), 1);
+        }
     }
 }
 
-__global__ void k_ranks(const int32_t* __restrict__ order, const int64_t* __restrict__ off, int nsets, int64_t n,
+/// The coordinates of some sets side by side: set list[k] at off_of[k].
+__global__ void __launch_bounds__(256) k_gather_sets(const double* __restrict__ xyz, const int64_t* __restrict__ off,
+                                                     const int* __restrict__ list, const int64_t* __restrict__ off_of,
+                                                     int m, int64_t n, double* __restrict__ out) {
+    for (int64_t p = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; p < n; p += int64_t(gridDim.x) * blockDim.x) {
+        const int k = set_of(off_of, m, p);
+        const int64_t from = off[list[k]] + (p - off_of[k]);
+        for (int a = 0; a < 3; ++a) out[3 * p + a] = xyz[3 * from + a];
+    }
+}
+
+/// Ranks in the reference's order, from that order of the sets of `list` (see
+/// k_gather_sets; null: all sets).
+__global__ void k_ranks(const int32_t* __restrict__ order, const int64_t* __restrict__ off,
+                        const int* __restrict__ list, const int64_t* __restrict__ off_of, int m, int64_t n,
                         int32_t* __restrict__ rank) {
-    for (int64_t r = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; r < n; r += int64_t(gridDim.x) * blockDim.x)
-        rank[off[set_of(off, nsets, r)] + order[r]] = int32_t(r);
+    for (int64_t r = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; r < n; r += int64_t(gridDim.x) * blockDim.x) {
+        const int k = set_of(off_of, m, r);
+        rank[off[list ? list[k] : k] + order[r]] = int32_t(r - off_of[k]);
+    }
 }
 
 /// With repeated points: the vertices are the first copies, each reported under
@@ -270,7 +291,7 @@ __global__ void __launch_bounds__(256) k_compact_copies(const double* __restrict
         const int32_t g = idx[i];
         int32_t best = g;
         for (int64_t j = i + 1; j < n && keys[j] == k; ++j)
-            if (rank[idx[j]] > rank[best] && equal_points(xyz, g, idx[j])) best = idx[j];
+            if (equal_points(xyz, g, idx[j]) && rank[idx[j]] > rank[best]) best = idx[j];
         const int32_t v = pos[i];
         vert[v] = g;
         rep[v] = int32_t(best - off[set_of(off, nsets, g)]);
@@ -327,27 +348,56 @@ int own_order_sets(const double* d_xyz, const int64_t* h_off, const int64_t* d_o
     D3G_TRY(idx.alloc(size_t(n), s));
     D3G_TRY(idx2.alloc(size_t(n), s));
     D3G_TRY(first.alloc(size_t(n), s));
-    D3G_TRY(flags.alloc(2, s));
-    D3G_CUDA(cudaMemsetAsync(flags.p, 0, 2 * sizeof(int), s));
+    D3G_TRY(flags.alloc(2 + size_t(nsets), s));
+    D3G_CUDA(cudaMemsetAsync(flags.p, 0, sizeof(int) * (2 + size_t(nsets)), s));
     k_order_keys<<<grid_for(n, 256), 256, 0, s>>>(d_xyz, d_off, nsets, n, S.box.p, growth, bits, level_bits, keys2.p,
                                                   idx2.p);
     D3G_TRY(sort_pairs(keys2.p, keys.p, idx2.p, idx.p, n, 0, shift + level_bits + set_bits, s));
-    k_first_copies<<<grid_for(n, 256), 256, 0, s>>>(d_xyz, keys.p, idx.p, n, first.p, flags.p);
+    k_first_copies<<<grid_for(n, 256), 256, 0, s>>>(d_xyz, keys.p, idx.p, n, nsets, shift + level_bits, first.p,
+                                                     flags.p);
     const int64_t total = int64_t(nsets) * O.levels;
     D3G_TRY(O.level_start.alloc(size_t(total) + 1, s));
     k_level_starts<<<grid_for(n + 1, 256), 256, 0, s>>>(keys.p, n, shift, level_bits, O.levels, total,
                                                         O.level_start.p);
-    int hflags[2] = {0, 0};
-    D3G_CUDA(cudaMemcpyAsync(hflags, flags.p, sizeof hflags, cudaMemcpyDeviceToHost, s));
+    std::vector<int> hflags(flags.n);
+    D3G_CUDA(cudaMemcpyAsync(hflags.data(), flags.p, sizeof(int) * flags.n, cudaMemcpyDeviceToHost, s));
     D3G_CUDA(cudaStreamSynchronize(s));
     if (hflags[1]) return D3G_OK;
     O.nv = n - hflags[0];
     if (hflags[0] > 0) {
+        // Which copy keeps its index is the reference's order's to say, so the sets with
+        // copies are put in that order (4096 mixed sets, a fourth of them with one
+        // point in 97 twice: order 61 -> 23 ms, the build 437 -> 399).
+        std::vector<int> list;
+        std::vector<int64_t> hoff_of(1, 0);
+        for (int i = 0; i < nsets; ++i) {
+            if (!hflags[size_t(i) + 2]) continue;
+            list.push_back(i);
+            hoff_of.push_back(hoff_of.back() + (h_off[i + 1] - h_off[i]));
+        }
+        const int m = int(list.size());
+        const int64_t nm = hoff_of.back();
+        DevBuf<int> dlist;
+        DevBuf<int64_t> doff_of;
+        DevBuf<double> some;
         DevBuf<int32_t> order, rank;
-        D3G_TRY(order.alloc(size_t(n), s));
+        D3G_TRY(order.alloc(size_t(nm), s));
         D3G_TRY(rank.alloc(size_t(n), s));
-        D3G_TRY(spatial_order_sets_device(d_xyz, h_off, d_off, nsets, order.p, s));
-        k_ranks<<<grid_for(n, 256), 256, 0, s>>>(order.p, d_off, nsets, n, rank.p);
+        const double* pts = d_xyz;
+        const int64_t* off_of = d_off;
+        if (m < nsets) {
+            D3G_TRY(dlist.alloc(size_t(m), s));
+            D3G_TRY(doff_of.alloc(size_t(m) + 1, s));
+            D3G_TRY(some.alloc(size_t(3) * size_t(nm), s));
+            D3G_CUDA(cudaMemcpyAsync(dlist.p, list.data(), sizeof(int) * size_t(m), cudaMemcpyHostToDevice, s));
+            D3G_CUDA(cudaMemcpyAsync(doff_of.p, hoff_of.data(), sizeof(int64_t) * (size_t(m) + 1),
+                                     cudaMemcpyHostToDevice, s));
+            k_gather_sets<<<grid_for(nm, 256), 256, 0, s>>>(d_xyz, d_off, dlist.p, doff_of.p, m, nm, some.p);
+            pts = some.p;
+            off_of = doff_of.p;
+        }
+        D3G_TRY(spatial_order_sets_device(pts, hoff_of.data(), off_of, m, order.p, s));
+        k_ranks<<<grid_for(nm, 256), 256, 0, s>>>(order.p, d_off, dlist.p, off_of, m, nm, rank.p);
         D3G_TRY(exclusive_scan(first.p, idx2.p, n, s));
         D3G_TRY(O.vert.alloc(size_t(O.nv), s));
         D3G_TRY(O.rep.alloc(size_t(O.nv), s));

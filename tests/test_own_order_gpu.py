@@ -70,3 +70,18 @@ def test_batch_of_every_case(cuda):
         for k, pts in enumerate(batch):
             want = oracle.orc_build(pts) if len(pts) else {"cells": np.zeros((0, 4), np.int32), "n_vertices": 0}
             assert nv[k] == want["n_vertices"] and np.array_equal(cells[k], want["cells"]), k
+
+
+@pytest.mark.parametrize("doubled", [[], [0], [6], [1, 2, 5], list(range(7))])
+def test_batch_with_copies_in_some_sets(cuda, doubled):
+    """The sets with repeated points alone go through the reference's order: every set of a
+    batch must come out as the oracle builds it, whichever sets hold copies."""
+    sizes = [700, 5, 1200, 4, 1, 2500, 333]
+    sets = [d3.gen_uniform(n, 20 + k) for k, n in enumerate(sizes)]
+    for k in doubled:
+        sets[k] = np.concatenate([sets[k], sets[k][::2]])
+    cells, n_vertices = d3.build_batch(sets)
+    for k, pts in enumerate(sets):
+        want = oracle.orc_build(np.ascontiguousarray(pts))
+        assert n_vertices[k] == want["n_vertices"]
+        assert np.array_equal(cells[k], want["cells"])
