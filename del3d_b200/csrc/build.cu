@@ -3156,7 +3156,7 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
         D3G_TRY(defer.alloc(size_t(nv), s));
         for (auto& l : left) D3G_TRY(l.alloc(size_t(nv), s));
         D3G_TRY(pool.alloc(size_t(kMaxGroups), s));
-        D3G_TRY(cnt.alloc(size_t(4) * size_t(nlev + kLastPasses + 1) + 4, s));
+        D3G_TRY(cnt.alloc(size_t(4) * size_t(nlev + kLastPasses + 1) + 6, s));
         D3G_CUDA(cudaMemcpyAsync(dctl.p, ctl.data(), sizeof(int) * ctl.size(), cudaMemcpyHostToDevice, s));
         D3G_CUDA(cudaMemsetAsync(pool.p, 0, sizeof(int4) * size_t(kMaxGroups), s));
         D3G_CUDA(cudaMemsetAsync(cnt.p, 0, sizeof(int) * cnt.n, s));
@@ -3300,20 +3300,25 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
             }
             if (lev == nlev - 1) {
                 // Regions beyond that pass's scratch (and the odd undecided point) get one of
-                // kBigCapacity; what it leaves in turn is for the full variant.
+                // kBigCapacity: 16 groups, then - such regions of one set overlap, and take
+                // longer than a group waits for another - one by itself.  What that leaves is
+                // for the full variant.
                 auto* kernel = k_insert_groups<32, true, kBigCapacity, 32>;
                 D3G_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                               int(sizeof(GroupScratch<32, kBigCapacity>))));
-                A.items = defer.p;
-                A.n_items = n_defer;
-                A.next = n_defer - 2;
-                A.left = A.defer = left_of(0);
-                A.n_left = A.n_defer = n_defer - 3;
                 A.cavity = opt.cavity_capacity > 0 ? cav_normal : kBigCapacity;
-                A.ngroups = std::min(16, std::max(1, nv / kPoolSlots));
-                kernel<<<unsigned(A.ngroups), 32, sizeof(GroupScratch<32, kBigCapacity>), s>>>(T, A, Rd, vx.p);
-                D3G_CUDA(cudaGetLastError());
-                R.stats.launches_async += 1;
+                int* count[3] = {n_defer, n_defer - 3, n_defer - 5};
+                for (int k = 0; k < 2; ++k) {
+                    A.items = k == 0 ? defer.p : left_of(0);
+                    A.n_items = count[k];
+                    A.next = k == 0 ? n_defer - 2 : n_defer - 4;
+                    A.left = A.defer = k == 0 ? left_of(0) : defer.p;
+                    A.n_left = A.n_defer = count[k + 1];
+                    A.ngroups = k == 0 ? std::min(16, std::max(1, nv / kPoolSlots)) : 1;
+                    kernel<<<unsigned(A.ngroups), 32, sizeof(GroupScratch<32, kBigCapacity>), s>>>(T, A, Rd, vx.p);
+                    D3G_CUDA(cudaGetLastError());
+                    R.stats.launches_async += 1;
+                }
             }
             if (opt.validate || lev == nlev - 1) {
                 int nd = 0;

@@ -27,7 +27,10 @@ constexpr int kGroupBlocks = 5;
 constexpr int kGroupStash = 6;        // points a group keeps to try again later
 constexpr int kGroupTries = 24;       // attempts before a point is left
 constexpr int kWaitPolls = 150;       // polls of a lock before its holder's point is given way to
-constexpr int kBigCapacity = 2048;    // region tets and boundary facets of the widest groups' last pass
+/// Region tets and boundary facets of the widest groups' last pass (139 KB of scratch;
+/// 4096 mixed sets, whose largest region is 2592 tets, with 2048 386 ms, since the
+/// region beyond it needed the rounds and their tables; with this 377, with 6144 the same).
+constexpr int kBigCapacity = 4096;
 constexpr int kPoolSlots = 16;        // tet slots a group takes from the table at a time
 
 /// kCap: region tets, and boundary facets, a group has room for.

@@ -51,6 +51,23 @@ def test_regions_beyond_the_scratch(cuda, around):
     assert np.array_equal(d.finite_cells(), want["cells"]) and np.array_equal(d.all_cells(), want["all"])
 
 
+@pytest.mark.parametrize("around", [900, 1800, 4000])
+def test_big_regions_that_overlap(cuda, around):
+    """Sets whose inner points' regions hold thousands of tets of a shell (4096 is the
+    widest group's room) and get in each other's way; on a grid, so that ties abound."""
+    rng = np.random.default_rng(around)
+    sets = []
+    for k in range(6):
+        v = rng.standard_normal((around, 3))
+        shell = np.round(1024.0 * v / np.linalg.norm(v, axis=1, keepdims=True))
+        inner = rng.integers(-20, 21, (15, 3))
+        sets.append(np.unique(np.concatenate([shell, inner]), axis=0)[rng.permutation(around)[:around - 50]])
+    cells, n_vertices = d3.build_batch(sets)
+    for k, pts in enumerate(sets):
+        want = oracle.orc_build(pts)
+        assert n_vertices[k] == want["n_vertices"] and np.array_equal(cells[k], want["cells"]), k
+
+
 def test_offset_lattice_and_caller_chunks(cuda):
     """A lattice away from the origin, and the worker densities a caller may ask for."""
     pts = d3.gen_lattice(9000) + [700.0, -300.0, 55.0]
