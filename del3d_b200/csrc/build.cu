@@ -754,9 +754,11 @@ __global__ void __launch_bounds__(128, 8) k_restar(Tables T, Workers W, Round R,
 //
 // Lock word of a tet: 0 free, -1 a slot no tet has been written to yet, else
 // (owner << 1) | ring, owner = group or warp slot + 1; ring = 1 for a tet
-// across the region boundary, 0 for a region tet.  Locks are
-// taken with acquire and released with release ordering, and every read of
-// tet data that other warps write goes to L2 (__ldcg), not the SM's L1.
+// across the region boundary, 0 for a region tet.  Locks are taken with acquire
+// ordering; after the tets are written they are released by a warp barrier, then
+// a fence in every lane, then plain stores (k_insert_groups), or by a barrier and
+// compare-and-swaps with release ordering (k_insert_full).  Every read of tet
+// data that other warps write goes to L2 (__ldcg), not the SM's L1.
 
 constexpr int kAsyncRetries = 6;
 // Passes of k_insert_full over the points left to it before the rounds.

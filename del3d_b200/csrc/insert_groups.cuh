@@ -516,8 +516,12 @@ __device__ __forceinline__ int insert_step(const M& m, Scratch& S, const Lanes<G
         if (bad) report(status, ST_INTERNAL);
     }
     // ---- publish, then give the locks back ----
-    m.fence();
+    // A lane gives back locks of tets that other lanes wrote, so its fence has to
+    // stand behind the barrier: the barrier orders their writes before the fence,
+    // and the fence with the plain store to the lock word behind it is the release
+    // that the next owner's acquire meets.
     __syncwarp();
+    m.fence();
     if (win) {
         for (int k = L.sub; k < F; k += G) {
             const int w = S.fac[k].w;
