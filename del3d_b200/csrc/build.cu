@@ -246,14 +246,45 @@ __device__ __forceinline__ int orient_replaced(const Pt* q, int i, const Pt& p, 
     return orient3d_x(A, B, C, D, ex, st);
 }
 
+/// Whether the normal that in_circle_filter computes for facet (a, b, d) points to
+/// the right side of its plane.  The filter's value is that of in_sphere with the
+/// facet's vertices and the point p + normal, so its sign hangs on that side, but its
+/// bound is relative to the normal's rounded length: on a facet whose vertices are
+/// collinear but for rounding it can certify the wrong sign.  Each component is off by
+/// at most 4 eps of the sum of its two products' sizes (8 here).
+__device__ __forceinline__ bool normal_certain(const Pt& a, const Pt& b, const Pt& d) {
+    const double px = fsub(b.x, a.x), py = fsub(b.y, a.y), pz = fsub(b.z, a.z);
+    const double qx = fsub(d.x, a.x), qy = fsub(d.y, a.y), qz = fsub(d.z, a.z);
+    const double x0 = fmul(py, qz), x1 = fmul(pz, qy), y0 = fmul(pz, qx), y1 = fmul(px, qz), z0 = fmul(px, qy),
+                 z1 = fmul(py, qx);
+    const double longest = fmax(fmax(fabs_(fsub(x0, x1)), fabs_(fsub(y0, y1))), fabs_(fsub(z0, z1)));
+    const double sizes = fadd(fadd(fadd(fabs_(x0), fabs_(x1)), fadd(fabs_(y0), fabs_(y1))), fadd(fabs_(z0), fabs_(z1)));
+    return longest > fmul(8.0 * kEps, sizes);
+}
+
 /// coplanar_in_circle for the hull case of the conflict test (rare: the point
 /// lies in the plane of a hull facet), out of line so that its code stays out
-/// of the hot path's instruction stream.
+/// of the hot path's instruction stream.  It is coplanar_in_circle except on facets
+/// without a certain normal, which go to the exact stage where that reaches: the
+/// reference takes the filter's sign there (src/predicates2.cpp:182-231), and in an
+/// unlucky order of insertions a wrong one gives a region that is no ball, or other
+/// cells.
 __device__ __noinline__ int hull_in_circle(double ax, double ay, double az, double bx, double by, double bz,
                                            double dx, double dy, double dz, double px, double py, double pz,
                                            int ia, int ib, int id_, int ip, uint32_t* st) {
-    const int64_t id[4] = {ia, ib, id_, ip};
-    return coplanar_in_circle(Pt{ax, ay, az}, Pt{bx, by, bz}, Pt{dx, dy, dz}, Pt{px, py, pz}, id, st);
+    const Pt a{ax, ay, az}, b{bx, by, bz}, d{dx, dy, dz}, p{px, py, pz};
+    const InCircleFilter f = in_circle_filter(a, b, d, p);
+    if (f.certain) {
+        bool use = normal_certain(a, b, d);
+        if (!use) {
+            Span s;
+            s.add(ax); s.add(ay); s.add(az); s.add(bx); s.add(by); s.add(bz);
+            s.add(dx); s.add(dy); s.add(dz); s.add(px); s.add(py); s.add(pz);
+            use = limbs_for(7 * (s.bits() + 1) + 9) > kMaxLimbs;
+        }
+        if (use) return sign_of(f.det);
+    }
+    return in_circle_degenerate(ax, ay, az, bx, by, bz, dx, dy, dz, px, py, pz, ia, ib, id_, ip, f.det, 1, st);
 }
 
 /// Outcome bits of a conflict test: in conflict; the floating-point filter
