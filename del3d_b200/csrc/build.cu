@@ -42,12 +42,14 @@
 #include "order.cuh"
 
 #include <algorithm>
-#include <mutex>
-#include <numeric>
-#include <optional>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
+#include <mutex>
+#include <numeric>
+#include <optional>
+#include <utility>
 #include <vector>
 
 namespace d3g {
@@ -291,7 +293,7 @@ __device__ __noinline__ int hull_in_circle(double ax, double ay, double az, doub
 /// could not certify the sign (the set's exact filter value, the exact stage or
 /// a tie-break decided it); the exact value was zero (decided by the symbolic
 /// perturbation, or the hull in-circle test); and, from in_conflict_fast only,
-/// undecided (left to k_insert_full, whose test has the exact stage).
+/// undecided (the exact stage is needed).
 enum : int { CT_IN = 1, CT_UNCERTAIN = 2, CT_TIE = 4, CT_UNDECIDED = 8 };
 
 /// What a set's coordinates make exact (k_set_exact).
@@ -345,9 +347,10 @@ __device__ int conflict_test(const int4 t, const Pt& p, int pid, const double* _
     return ((tie ? r - 4 : r) > 0 ? CT_IN : 0) | CT_UNCERTAIN | (tie ? CT_TIE : 0);
 }
 
-/// conflict_test out of line, for the once-per-insertion seed check (one inline
-/// copy, in the breadth-first growth, is enough).
-__device__ __noinline__ int conflict_test_seed(int4 t, double px, double py, double pz, int pid,
+/// conflict_test out of line: for the once-per-insertion seed check of k_insert_full
+/// (one inline copy, in the breadth-first growth, is enough) and for the tests that
+/// the filters of k_insert_groups leave undecided.
+__device__ __noinline__ int conflict_test_exact(int4 t, double px, double py, double pz, int pid,
                                                const double* __restrict__ vx, bool ex, uint32_t* st) {
     return conflict_test(t, Pt{px, py, pz}, pid, vx, ex, st);
 }
@@ -805,6 +808,19 @@ constexpr int kAsyncWalkLimit = 1 << 14;
 constexpr int kGroupGrowth = 2;
 // Passes of k_insert_groups over what the last level left.
 constexpr int kLastPasses = 3;
+// Passes with the exact stage over the points with undecided tests that are left
+// after the last level.
+constexpr int kExactPasses = 3;
+// Each level is followed by a look at how many points with undecided tests wait; from
+// the first that finds more than one in kUndecidedShare of the points so far, every
+// level is followed by a pass with the exact stage.  (Fewer wait for the end.)  A point
+// that is not in makes the regions of those after it larger, and a test that one point
+// cannot decide is met by the next ones near it: with passes from the level of 4096
+// points on, a set with half of its 300000 points in one corner of 2^-30 of its
+// extent took 990 ms, without any 11 s.
+constexpr int kUndecidedShare = 128;
+// Points the last pass of a single group takes at most.
+constexpr int kLonePoints = 256;
 // Vertices of the level before, to either side along the curve, among which a
 // vertex's guide is the nearest.
 constexpr int kGuideReach = 4;
@@ -1245,7 +1261,7 @@ __device__ int insert_full(int v, int t0, const Tables& T, const Workers& W, con
             const int4 stv = ld4(&T.tv(seed));
             htn[0] = ld4(&T.tn(seed));
             if (stv.x != stv.y && T.vset[stv.x != kInf ? stv.x : stv.y] == T.vset[v]) {
-                r = conflict_test_seed(stv, p.x, p.y, p.z, v, vx, ex, st);
+                r = conflict_test_exact(stv, p.x, p.y, p.z, v, vx, ex, st);
                 ctr.count(r);
             }
             if (r & CT_IN) {
@@ -3072,10 +3088,10 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
         }
         return D3G_OK;
     };
-    // The points k_insert_groups left (tests its filters cannot decide, regions
-    // beyond its scratch, persistent conflicts) through the full variant, one
-    // worker per point, all of them at once, again while a pass inserts at least a
-    // quarter of its points; what that leaves through the rounds.
+    // The points k_insert_groups left (regions beyond its scratch, persistent
+    // conflicts) through the full variant, one worker per point, all of them at once,
+    // again while a pass inserts at least a quarter of its points; what that leaves
+    // through the rounds.
     DevBuf<int> aleft, aleft2, actl;
     auto finish_points = [&](int* list, int count) -> int {
         if (count <= 0) return D3G_OK;
@@ -3179,17 +3195,24 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
             }
             m_of[lev] = total - first_of[lev];
         }
-        DevBuf<int> dctl, items, guide, hint, lstart, defer, left[2], cnt;
+        constexpr int kPassHeads = 256;    // queue heads of passes with the exact stage
+        DevBuf<int> heads;
+        int head = 0;
+        DevBuf<int> dctl, items, guide, hint, lstart, defer[2], big, left[2], cnt;
         DevBuf<int4> pool;
         D3G_TRY(dctl.alloc(ctl.size(), s));
         D3G_TRY(items.alloc(size_t(std::max(total, 1)), s));
         D3G_TRY(guide.alloc(size_t(nv), s));
         D3G_TRY(hint.alloc(size_t(nv), s));
         D3G_CUDA(cudaMemsetAsync(hint.p, 0xFF, sizeof(int) * size_t(nv), s));
-        D3G_TRY(defer.alloc(size_t(nv), s));
+        for (auto& l : defer) D3G_TRY(l.alloc(size_t(nv), s));
+        D3G_TRY(big.alloc(size_t(nv), s));
         for (auto& l : left) D3G_TRY(l.alloc(size_t(nv), s));
         D3G_TRY(pool.alloc(size_t(kMaxGroups), s));
-        D3G_TRY(cnt.alloc(size_t(4) * size_t(nlev + kLastPasses + 1) + 6, s));
+        // Counters: four per list of points left, one per list of deferred ones (at most
+        // one after each level and kExactPasses each time they are drained), six more.
+        const size_t nleft_lists = size_t(nlev) + kLastPasses + 1, ndefer_lists = size_t(nlev) * (kExactPasses + 1) + 2;
+        D3G_TRY(cnt.alloc(4 * nleft_lists + ndefer_lists + 6, s));
         D3G_CUDA(cudaMemcpyAsync(dctl.p, ctl.data(), sizeof(int) * ctl.size(), cudaMemcpyHostToDevice, s));
         D3G_CUDA(cudaMemsetAsync(pool.p, 0, sizeof(int4) * size_t(kMaxGroups), s));
         D3G_CUDA(cudaMemsetAsync(cnt.p, 0, sizeof(int) * cnt.n, s));
@@ -3219,14 +3242,20 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
         auto head_of = [&](int k) { return cnt.p + 4 * k; };
         auto n_left_of = [&](int k) { return cnt.p + 4 * k + 1; };
         auto left_of = [&](int k) { return left[k & 1].p; };
-        int* n_defer = cnt.p + (cnt.n - 1);
-        int list = 0;
+        // Likewise the lists of points with undecided tests.
+        auto defer_of = [&](int k) { return defer[k & 1].p; };
+        auto n_defer_of = [&](int k) { return cnt.p + 4 * nleft_lists + k; };
+        int* const coarse_queue = cnt.p + (cnt.n - 6);
+        int* const big_ctl = coarse_queue + 1;   // [0] points too big, [1] and [3] queue heads, [2] and [4] left
+        int list = 0, deferred = 0;
         GroupArgs A{};
         A.lock = alock.p;
         A.guide = guide.p;
         A.hint = hint.p;
-        A.defer = defer.p;
-        A.n_defer = n_defer;
+        A.defer = defer_of(0);
+        A.n_defer = n_defer_of(0);
+        A.big = big.p;
+        A.n_big = big_ctl;
         A.pool = pool.p;
         A.skips = skips.p;
         A.set_exact = set_exact.p;
@@ -3234,14 +3263,18 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
         A.voff = voff.p;
         A.stats = astats.p;
         A.cavity = cav_normal;
-        auto launch = [&](int G, int ngroups, bool near) {
+        A.first = 0;
+        A.most = INT_MAX;
+        auto launch = [&](int G, int ngroups, int mode) {
             // At most one group per kPoolSlots vertices, so that the slots groups hold
             // without using them stay within the table's room for them.
-            A.ngroups = std::max(1, std::min({ngroups, kNumSMs * kGroupBlocks * (kGroupThreads / G), nv / kPoolSlots}));
+            const int blocks = mode == kExact ? kExactBlocks : kGroupBlocks;
+            A.ngroups = std::max(1, std::min({ngroups, kNumSMs * blocks * (kGroupThreads / G), nv / kPoolSlots}));
             const unsigned grid = unsigned((A.ngroups + kGroupThreads / G - 1) / (kGroupThreads / G));
-            auto* kernel = G == 8 ? (near ? k_insert_groups<8, true, 64, kGroupThreads> : k_insert_groups<8, false, 64, kGroupThreads>)
-                         : (G == 16 ? (near ? k_insert_groups<16, true, 128, kGroupThreads> : k_insert_groups<16, false, 128, kGroupThreads>)
-                                    : (near ? k_insert_groups<32, true, 256, kGroupThreads> : k_insert_groups<32, false, 256, kGroupThreads>));
+            auto* kernel = mode == kExact ? k_insert_groups<32, kExact, 256, kGroupThreads>
+                         : G == 8  ? (mode == kNear ? k_insert_groups<8, kNear, 64, kGroupThreads> : k_insert_groups<8, kFilter, 64, kGroupThreads>)
+                         : G == 16 ? (mode == kNear ? k_insert_groups<16, kNear, 128, kGroupThreads> : k_insert_groups<16, kFilter, 128, kGroupThreads>)
+                                   : (mode == kNear ? k_insert_groups<32, kNear, 256, kGroupThreads> : k_insert_groups<32, kFilter, 256, kGroupThreads>);
             const size_t scratch = G == 8 ? sizeof(GroupScratch<8, 64>) * 16
                                           : (G == 16 ? sizeof(GroupScratch<16, 128>) * 8 : sizeof(GroupScratch<32, 256>) * 4);
             kernel<<<grid, kGroupThreads, scratch, s>>>(T, A, Rd, vx.p);
@@ -3255,24 +3288,146 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
         int64_t on_grid = 0;
         for (int st = 0; st < nsets; ++st)
             if (hexact[size_t(st)] & EX_GRID) on_grid += R.set_nv[size_t(st)];
-        const bool near_main = 2 * on_grid > nv;
+        const int main_mode = 2 * on_grid > nv ? kNear : kFilter;
         // A pass of the widest groups over the current list; what it leaves is the next.
         auto left_pass = [&](int ngroups, bool last = false) {
             A.items = left_of(list);
             A.n_items = n_left_of(list);
             A.next = head_of(list) + 2;
             ++list;
-            A.left = last ? defer.p : left_of(list);
-            A.n_left = last ? n_defer : n_left_of(list);
-            launch(32, ngroups, true);
+            A.left = last ? A.big : left_of(list);
+            A.n_left = last ? A.n_big : n_left_of(list);
+            launch(32, ngroups, kNear);
+        };
+        // The same with the exact stage, over the points with undecided tests: about `n` of
+        // them, where `in` points are in.  Where that is more than are in, a part after
+        // the other, each about as many points as are in, as levels do.
+        auto exact_pass = [&](int64_t n, int64_t in, int ngroups) -> int {
+            if (!heads.p) D3G_TRY(heads.alloc(kPassHeads, s));
+            A.items = defer_of(deferred);
+            A.n_items = n_defer_of(deferred);
+            ++deferred;
+            A.left = A.defer = defer_of(deferred);
+            A.n_left = A.n_defer = n_defer_of(deferred);
+            in = std::max<int64_t>(in, 16);
+            for (int64_t k = 0; k >= 0;) {
+                if (head == 0) D3G_CUDA(cudaMemsetAsync(heads.p, 0, sizeof(int) * kPassHeads, s));
+                A.next = heads.p + head;
+                head = (head + 1) % kPassHeads;
+                const int64_t part = std::max<int64_t>(in, 64);
+                A.first = int(k);
+                A.most = k + part < n ? int(part) : INT_MAX;
+                launch(32, int(std::min<int64_t>(std::max<int64_t>(in / alpha, 1), ngroups)), kExact);
+                k = k + part < n ? k + part : -1;
+                in += part;
+            }
+            A.first = 0;
+            A.most = INT_MAX;
+            return D3G_OK;
+        };
+        // What the levels' passes could not do, while the host looks on: points with
+        // undecided tests, with fewer and fewer groups in the way of one another; regions
+        // beyond the widest groups' scratch (and points worn out by conflicts) with one of
+        // kBigCapacity, by 16 groups, then - such regions of one set overlap, and take
+        // longer than a group waits for another - by one alone; the rest by k_insert_full.
+        auto drain = [&]() -> int {
+            int nd = 0, nb[5] = {0, 0, 0, 0, 0};
+            auto look = [&]() -> int {
+                uint32_t hs = 0;
+                D3G_CUDA(cudaGetLastError());
+                if (opt.timing) cudaEventRecord(kev[1], s);
+                D3G_CUDA(cudaMemcpyAsync(&nd, n_defer_of(deferred), sizeof nd, cudaMemcpyDeviceToHost, s));
+                D3G_CUDA(cudaMemcpyAsync(nb, big_ctl, sizeof nb, cudaMemcpyDeviceToHost, s));
+                D3G_CUDA(cudaMemcpyAsync(&hs, status.p, sizeof hs, cudaMemcpyDeviceToHost, s));
+                D3G_CUDA(cudaStreamSynchronize(s));
+                if (opt.timing) {
+                    float am = 0.f;
+                    cudaEventElapsedTime(&am, kev[0], kev[1]);
+                    R.stats.ms_async += am;
+                    cudaEventRecord(kev[0], s);
+                }
+                if (trace) fprintf(stderr, "d3g drain: %d undecided, too big %d %d %d\n", nd, nb[0], nb[2], nb[4]);
+                const int st = status_from_bits(hs);
+                if (st == D3G_ERR_OOM) set_error("d3g_build: tet table full");
+                return st;
+            };
+            D3G_TRY(look());
+            for (int k = 0; nd > 0 && k < kExactPasses; ++k) {
+                D3G_TRY(exact_pass(nd, int64_t(nv) - nd, std::max(kNumSMs * kExactBlocks * (kGroupThreads / 32) >> (3 * k), 16)));
+                D3G_TRY(look());
+            }
+            if (nb[0] > 0) {
+                // (the list behind the deferred one is free here)
+                int* const lists[3] = {big.p, defer_of(deferred + 1), big.p};
+                // (the exact stage's stack only where some point has needed it)
+                auto* kernel = deferred > 0 ? k_insert_groups<32, kExact, kBigCapacity, 32>
+                                            : k_insert_groups<32, kNear, kBigCapacity, 32>;
+                D3G_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              int(sizeof(GroupScratch<32, kBigCapacity>))));
+                GroupArgs B = A;
+                B.cavity = opt.cavity_capacity > 0 ? cav_normal : kBigCapacity;
+                for (int k = 0; k < 2; ++k) {
+                    B.items = lists[k];
+                    B.n_items = big_ctl + 2 * k;
+                    B.most = k == 0 ? INT_MAX : kLonePoints;
+                    B.next = big_ctl + 1 + 2 * k;
+                    B.left = B.big = lists[k + 1];
+                    B.n_left = B.n_big = big_ctl + 2 + 2 * k;
+                    B.ngroups = k == 0 ? std::min(16, std::max(1, nv / kPoolSlots)) : 1;
+                    kernel<<<unsigned(B.ngroups), 32, sizeof(GroupScratch<32, kBigCapacity>), s>>>(T, B, Rd, vx.p);
+                    R.stats.launches_async += 1;
+                    D3G_TRY(look());
+                    if (nb[2] == 0) break;
+                }
+                D3G_TRY(finish_points(lists[1] + kLonePoints, nb[2] - kLonePoints));
+                D3G_TRY(finish_points(lists[2], nb[4]));
+            }
+            D3G_TRY(finish_points(defer_of(deferred), nd));
+            D3G_CUDA(cudaMemsetAsync(big_ctl, 0, 5 * sizeof(int), s));
+            D3G_CUDA(cudaMemsetAsync(n_defer_of(deferred), 0, sizeof(int), s));
+            return D3G_OK;
+        };
+        // The look behind a level is at the counts of the level before, which the device
+        // has passed by then, so that it never waits for the host.
+        const bool may_defer = std::any_of(hexact.begin(), hexact.end(), [](uint8_t e) { return (e & EX_BOTH) != EX_BOTH; });
+        struct Look {
+            int* n = nullptr;            // pinned
+            cudaEvent_t ev = nullptr;
+            int64_t points = 0;          // inserted or waiting when it was taken
+            ~Look() {
+                if (ev) cudaEventSynchronize(ev), cudaEventDestroy(ev);
+                host_result_free(n);
+            }
+        } look;
+        bool exact_levels = false;
+        int64_t waiting = 0;
+        auto look_behind = [&](int lev) -> int {
+            if (!exact_levels && look.points > 0) {
+                D3G_CUDA(cudaEventSynchronize(look.ev));
+                exact_levels = int64_t(*look.n) * kUndecidedShare > look.points;
+                waiting = int64_t(*look.n) + m_of[lev];        // the level just launched may leave all of its points
+            }
+            if (exact_levels) {
+                const int64_t points = first_of[lev] + m_of[lev];
+                const int64_t n = std::exchange(waiting, 0);   // later levels' are decided as they come
+                return exact_pass(n, points - n, 1 << 24);
+            }
+            if (!look.ev) {
+                look.n = static_cast<int*>(host_result_alloc(sizeof(int)));
+                D3G_CUDA(cudaEventCreateWithFlags(&look.ev, cudaEventDisableTiming));
+            }
+            look.points = first_of[lev] + m_of[lev];
+            D3G_CUDA(cudaMemcpyAsync(look.n, n_defer_of(deferred), sizeof(int), cudaMemcpyDeviceToHost, s));
+            D3G_CUDA(cudaEventRecord(look.ev, s));
+            return D3G_OK;
         };
         if (opt.timing) cudaEventRecord(kev[0], s);
         if (use_coarse) {
             NvtxRange nvtx_level("d3g.coarse");
             A.left = left_of(list);
             A.n_left = n_left_of(list);
-            const CoarseArgs K{starts, start_stride, dctl.p + (coarse - ctl.data()), nsets, n_defer - 1};
-            auto* kernel = near_main ? k_coarse<true> : k_coarse<false>;
+            const CoarseArgs K{starts, start_stride, dctl.p + (coarse - ctl.data()), nsets, coarse_queue};
+            auto* kernel = main_mode == kNear ? k_coarse<kNear> : k_coarse<kFilter>;
             D3G_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(CoarseShared))));
             kernel<<<unsigned(std::min(nsets, kNumSMs)), kCoarseThreads, sizeof(CoarseShared), s>>>(T, A, K, Rd, vx.p);
             D3G_CUDA(cudaGetLastError());
@@ -3302,8 +3457,9 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
                 // caller's walk limit holds for an insertion's whole walk.)
                 if ((lev > 0 || use_coarse) && opt.walk_limit <= 0)
                     k_locate<<<grid_for(m_of[lev], 128), 128, 0, s>>>(T, A, vx.p);
-                launch(G, int(std::min<int64_t>(groups_of[size_t(lev)], 1 << 24)), near_main);
+                launch(G, int(std::min<int64_t>(groups_of[size_t(lev)], 1 << 24)), main_mode);
                 left_pass(kNumSMs * (kGroupThreads / 32));
+                if (may_defer) D3G_TRY(look_behind(lev));
             }
             D3G_CUDA(cudaGetLastError());
             if (trace) {
@@ -3314,7 +3470,7 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
                 int c[4] = {0, 0, 0, 0}, nd = 0;
                 unsigned long long as[7], ht[2];
                 cudaMemcpy(c, cnt.p + 4 * std::max(list - 1, 0), sizeof c, cudaMemcpyDeviceToHost);
-                cudaMemcpy(&nd, n_defer, sizeof nd, cudaMemcpyDeviceToHost);
+                cudaMemcpy(&nd, A.n_defer, sizeof nd, cudaMemcpyDeviceToHost);
                 cudaMemcpy(as, astats.p, sizeof as, cudaMemcpyDeviceToHost);
                 cudaMemcpy(ht, totals.p, sizeof ht, cudaMemcpyDeviceToHost);
                 fprintf(stderr, "d3g level %d sets %d points %d groups %d of %d lanes: left to wider groups %d, "
@@ -3326,52 +3482,12 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
                 cudaEventDestroy(ev1);
             }
             if (lev == nlev - 1) {
-                // The points still left, with fewer and fewer groups in the way of one another;
-                // the last pass hands what remains to the full variant.
+                // The points still left, with fewer and fewer groups in the way of one another.
                 for (int k = 0; k < kLastPasses; ++k)
                     left_pass(std::max(kNumSMs * (kGroupThreads / 32) >> (3 * k), 16), k == kLastPasses - 1);
             }
-            if (lev == nlev - 1) {
-                // Regions beyond that pass's scratch (and the odd undecided point) get one of
-                // kBigCapacity: 16 groups, then - such regions of one set overlap, and take
-                // longer than a group waits for another - one by itself.  What that leaves is
-                // for the full variant.
-                auto* kernel = k_insert_groups<32, true, kBigCapacity, 32>;
-                D3G_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              int(sizeof(GroupScratch<32, kBigCapacity>))));
-                A.cavity = opt.cavity_capacity > 0 ? cav_normal : kBigCapacity;
-                int* count[3] = {n_defer, n_defer - 3, n_defer - 5};
-                for (int k = 0; k < 2; ++k) {
-                    A.items = k == 0 ? defer.p : left_of(0);
-                    A.n_items = count[k];
-                    A.next = k == 0 ? n_defer - 2 : n_defer - 4;
-                    A.left = A.defer = k == 0 ? left_of(0) : defer.p;
-                    A.n_left = A.n_defer = count[k + 1];
-                    A.ngroups = k == 0 ? std::min(16, std::max(1, nv / kPoolSlots)) : 1;
-                    kernel<<<unsigned(A.ngroups), 32, sizeof(GroupScratch<32, kBigCapacity>), s>>>(T, A, Rd, vx.p);
-                    D3G_CUDA(cudaGetLastError());
-                    R.stats.launches_async += 1;
-                }
-            }
             if (opt.validate || lev == nlev - 1) {
-                int nd = 0;
-                uint32_t hs = 0;
-                if (opt.timing) cudaEventRecord(kev[1], s);
-                D3G_CUDA(cudaMemcpyAsync(&nd, A.n_defer, sizeof nd, cudaMemcpyDeviceToHost, s));
-                D3G_CUDA(cudaMemcpyAsync(&hs, status.p, sizeof hs, cudaMemcpyDeviceToHost, s));
-                D3G_CUDA(cudaStreamSynchronize(s));
-                if (hs != 0) {
-                    const int st = status_from_bits(hs);
-                    if (st == D3G_ERR_OOM) set_error("d3g_build: tet table full");
-                    return st;
-                }
-                if (opt.timing) {
-                    float am = 0.f;
-                    cudaEventElapsedTime(&am, kev[0], kev[1]);
-                    R.stats.ms_async += am;
-                }
-                D3G_TRY(finish_points(A.defer, nd));
-                D3G_CUDA(cudaMemsetAsync(A.n_defer, 0, sizeof(int), s));
+                D3G_TRY(drain());
                 if (opt.validate) D3G_TRY(validate_tables("after", lev));
                 if (opt.timing) cudaEventRecord(kev[0], s);
             }

@@ -24,9 +24,13 @@ constexpr int kGroupThreads = 128;
 /// bytes of spills, 228 KB of the SM's 256 taken by scratch, so spills miss L1)
 /// 4096 mixed sets took 440 ms against 409, with 4 457 against 429.
 constexpr int kGroupBlocks = 5;
+constexpr int kExactBlocks = 2;       // the same with kExact (255 registers)
 constexpr int kGroupStash = 6;        // points a group keeps to try again later
 constexpr int kGroupTries = 24;       // attempts before a point is left
 constexpr int kWaitPolls = 150;       // polls of a lock before its holder's point is given way to
+/// The same with kExact: an insertion with a dozen steps in the exact stage holds its locks
+/// for some 300 us, ten times as long as others.
+constexpr int kExactTries = 100, kExactPolls = 2000;
 /// Region tets and boundary facets of the widest groups' last pass (139 KB of scratch;
 /// 4096 mixed sets, whose largest region is 2592 tets, with 2048 386 ms, since the
 /// region beyond it needed the rounds and their tables; with this 377, with 6144 the same).
@@ -64,13 +68,16 @@ struct GroupArgs {
     const int* items;        // points to insert (-1: nothing to do)
     const int* guide;        // per vertex: a vertex near it that should be in already
     const int* n_items;      // how many
+    int first, most;         // of them, the launch takes those from `first` on, at most `most`
     int* hint;               // per vertex: a tet near it (k_locate), -1: none
     int* next;               // queue head
     int* left;               // points to try again by wider groups or with kNear (regions too big, too many
-                             // conflicts, undecided tests) ...
+                             // conflicts, undecided tests), ...
     int* n_left;
-    int* defer;              // ... and points for the full variant (a test the filters cannot decide)
+    int* defer;              // ... points with a test that kNear cannot decide either (for kExact), ...
     int* n_defer;
+    int* big;                // ... and points whose region has no room with the widest groups
+    int* n_big;
     int4* pool;              // per group: tet slots it holds (GroupScratch::pool)
     const int4* skips;       // per set: its first tet's vertices
     const uint8_t* set_exact;    // per set: EX_*
@@ -152,6 +159,20 @@ struct GlobalMesh {
     __device__ __forceinline__ void fence() const { __threadfence(); }
 };
 
+/// How a kernel treats a test its filter cannot decide: it gives the point up, settles
+/// the test for near points on a grid (in_sphere_near), or settles every test (the
+/// exact stage, out of line).
+enum : int { kFilter = 0, kNear = 1, kExact = 2 };
+
+/// orient_facet_filter's sign from the exact stage; 0 as well where the stage's limbs
+/// do not reach (the walk then does not cross the facet).
+__device__ __noinline__ int orient_facet_exact(const double* __restrict__ vx, int4 t, int i, int v) {
+    const int x = i == 0 ? t.z : (i == 2 ? t.y : t.x);
+    const int y = i == 0 ? t.y : (i == 1 ? t.z : (i == 2 ? t.x : t.y));
+    const int z = i == 3 ? t.z : t.w;
+    return orient3d(vpt(vx, x), vpt(vx, y), vpt(vx, z), vpt(vx, v), nullptr);
+}
+
 /// Locates a level's points, one thread each, in the mesh as it is before the
 /// level: the walk of an insertion, which has a group's lanes wait for one chain
 /// of reads, then starts a step or two from its end.  Reads may use L1, since
@@ -202,10 +223,10 @@ __global__ void __launch_bounds__(128) k_locate(Tables T, GroupArgs A, const dou
 /// (-1 for a group without a point); `t` becomes the seed, -1 after a walk that hit
 /// its limit.  M is where the mesh lies: in device memory (GlobalMesh) or in a
 /// block's shared memory (SharedMesh).
-template <int G, bool kNear, class M, class Scratch>
+template <int G, int kMode, class M, class Scratch>
 __device__ __forceinline__ int insert_step(const M& m, Scratch& S, const Lanes<G>& L, int group, bool live, int v, int ex,
                                            int& t, int cavity, uint32_t* status, unsigned long long* stats,
-                                           const SharedCounters& ctr, unsigned& tests) {
+                                           const SharedCounters& ctr, unsigned& tests, uint32_t* lacking = nullptr) {
     constexpr int kPool = M::kPool;
     const unsigned lt = (1u << L.lane) - 1u;
     const int region = (group + 1) << 1, ring = region | 1;
@@ -220,8 +241,9 @@ __device__ __forceinline__ int insert_step(const M& m, Scratch& S, const Lanes<G
 
     // ---- walk (see walk_async; lanes 0-3 test the facets, lanes 4-7 fetch the
     //      neighbours' records) ----
-    // A facet the filter cannot decide is not crossed: the seed is tested in any
-    // case, and if it fails the test the point is left to the full variant.
+    // A facet the filter cannot decide is not crossed (kExact: the exact stage
+    // decides it): the seed is tested in any case, and if it fails the test the
+    // point is deferred.
     int outcome = live ? AI_DONE : -1;
     bool fuzzy = false;
     {
@@ -248,7 +270,9 @@ __device__ __forceinline__ int insert_step(const M& m, Scratch& S, const Lanes<G
             const int s0 = int(h >> 30);
             bool neg = false;
             if (walking && L.sub < 4 && (at(tn, L.sub) >> 2) != prev && min(min(tv.x, tv.y), min(tv.z, tv.w)) >= 0) {
-                const int o = orient_facet_filter(m, tv, L.sub, p, ex & EX_ORIENT);
+                int o = orient_facet_filter(m, tv, L.sub, p, ex & EX_ORIENT);
+                if constexpr (kMode == kExact)
+                    if (o == 2) o = orient_facet_exact(m.vx, tv, L.sub, v);
                 fuzzy = fuzzy || o == 2;
                 neg = o < 0;
             }
@@ -311,7 +335,7 @@ __device__ __forceinline__ int insert_step(const M& m, Scratch& S, const Lanes<G
                 // one with a higher number, which gives way itself when it meets this one's
                 // locks (so no two wait for each other), and gives way to one with a lower
                 // number.  Not for narrower groups, where the other may be in the same warp.
-                for (int k = 0; k < kWaitPolls && seen > ring; ++k) {
+                for (int k = 0; k < (kMode == kExact ? kExactPolls : kWaitPolls) && seen > ring; ++k) {
                     __nanosleep(200);
                     seen = m.cas(nb, ring);
                 }
@@ -324,16 +348,25 @@ __device__ __forceinline__ int insert_step(const M& m, Scratch& S, const Lanes<G
             if (got) {
                 int r = 0;
                 for (;;) {
-                    r = in_conflict_fast<kNear>(m, nb, guess, p, v, ex);
+                    r = in_conflict_fast<kMode != kFilter>(m, nb, guess, p, v, ex);
                     if (guess.x == tv.x && guess.y == tv.y && guess.z == tv.z && guess.w == tv.w) break;
                     guess = tv;
                 }
                 if (nreg == 0) {
                     // The seed may come from a half-written record: only a live
-                    // tet of the point's own set will do (see insert_full).
+                    // tet of the point's own set will do.
                     const int u = tv.x != kInf ? tv.x : tv.y;
                     bad_seed = tv.x == tv.y || u < S.vlo || u >= S.vhi;
                     if (bad_seed) r = 0;
+                }
+                if constexpr (kMode == kExact) {
+                    // Where the exact stage's limbs do not reach either, the point waits: with
+                    // others in, the test may no longer come up.
+                    if (r & CT_UNDECIDED) {
+                        *lacking = 0;
+                        r = conflict_test_exact(tv, p.x, p.y, p.z, v, m.vx, (ex & EX_BOTH) == EX_BOTH, lacking);
+                        if (*static_cast<volatile uint32_t*>(lacking)) r = CT_UNCERTAIN | CT_UNDECIDED;
+                    }
                 }
                 ++tests;
                 if (r & (CT_UNCERTAIN | CT_TIE)) ctr.count(r);
@@ -545,8 +578,8 @@ __device__ __forceinline__ int insert_step(const M& m, Scratch& S, const Lanes<G
     return outcome;
 }
 
-template <int G, bool kNear, int kCapacity, int kThreads>
-__global__ void __launch_bounds__(kThreads, kThreads == kGroupThreads ? kGroupBlocks : 1)
+template <int G, int kMode, int kCapacity, int kThreads>
+__global__ void __launch_bounds__(kThreads, kThreads != kGroupThreads ? 1 : (kMode == kExact ? kExactBlocks : kGroupBlocks))
     k_insert_groups(Tables T, GroupArgs A, Round R, const double* __restrict__ vx) {
     typedef GroupScratch<G, kCapacity> Scratch;
     const GlobalMesh m{T, A, vx};
@@ -557,10 +590,11 @@ __global__ void __launch_bounds__(kThreads, kThreads == kGroupThreads ? kGroupBl
     const Lanes<G> L;
     Scratch& S = scratch[threadIdx.x / G];
     const int group = int(blockIdx.x) * kPerBlock + int(threadIdx.x) / G;
+    __shared__ uint32_t lacking[kMode == kExact ? kThreads : 1];   // status words of the lanes' exact tests
     __shared__ int nitems;
     __shared__ long long stride;
     if (threadIdx.x == 0) {
-        nitems = *A.n_items;
+        nitems = min(max(*A.n_items - A.first, 0), A.most);
         // Points go out in a scattered order (a stride near the golden ratio of their
         // number and coprime with it), so that those in flight lie far apart along the
         // curve.
@@ -592,7 +626,7 @@ __global__ void __launch_bounds__(kThreads, kThreads == kGroupThreads ? kGroupBl
             S.attempt = 0;
             while (item < 0 && S.nstash < kGroupStash && S.open) {
                 const int q = atomicAdd(A.next, 1);
-                if (q < nitems) item = A.items[int((q * stride) % nitems)];
+                if (q < nitems) item = A.items[A.first + int((q * stride) % nitems)];
                 else S.open = 0;
             }
             if (item < 0 && S.nstash > 0) {
@@ -622,23 +656,24 @@ __global__ void __launch_bounds__(kThreads, kThreads == kGroupThreads ? kGroupBl
         const int ex = A.set_exact[T.vset[v]];
         t = max(__shfl_sync(kFull, t, L.gbase), 0);
 
-        const int outcome = insert_step<G, kNear>(m, S, L, group, live, v, ex, t, A.cavity, R.status, A.stats, ctr, tests);
+        const int outcome = insert_step<G, kMode>(m, S, L, group, live, v, ex, t, A.cavity, R.status, A.stats, ctr, tests,
+                                                  lacking + (kMode == kExact ? threadIdx.x : 0));
         const bool win = live && outcome == AI_DONE;
         // ---- what was not inserted: again later, or left ----
         bool idle = true;
         unsigned wait = 0;
         if (L.sub == 0 && live && !win) {
             const int attempt = S.attempt + 1;
-            if (outcome == AI_RETRY && attempt < kGroupTries) {
+            if (outcome == AI_RETRY && attempt < (kMode == kExact ? kExactTries : kGroupTries)) {
                 S.stash[S.nstash] = v;
                 S.stash_tries[S.nstash++] = attempt;
                 if (t >= 0) A.hint[v] = t;
                 idle = !S.open;
                 wait = min(attempt, 3);
             } else {
-                // Too big for the widest group, or undecided even so: the full variant.
-                const bool def = (outcome == AI_DEFER && kNear) || (outcome == AI_LEAVE && G == 32);
-                (def ? A.defer : A.left)[atomicAdd(def ? A.n_defer : A.n_left, 1)] = v;
+                const bool def = outcome == AI_DEFER && kMode != kFilter, big = outcome == AI_LEAVE && G == 32;
+                int* const list = def ? A.defer : (big ? A.big : A.left);
+                list[atomicAdd(def ? A.n_defer : (big ? A.n_big : A.n_left), 1)] = v;
                 atomicAdd(A.stats + 4, 1ull);
             }
         } else if (win) {
@@ -791,7 +826,7 @@ struct CoarseArgs {
     int* next;
 };
 
-template <bool kNear>
+template <int kMode>
 __global__ void __launch_bounds__(kCoarseThreads, 1)
     k_coarse(Tables T, GroupArgs A, CoarseArgs K, Round R, const double* __restrict__ vx) {
     extern __shared__ __align__(16) unsigned char coarse_smem[];
@@ -819,7 +854,7 @@ __global__ void __launch_bounds__(kCoarseThreads, 1)
         const int* ls = K.starts + int64_t(set) * K.stride;
         const int nlev = K.levels[set];
         const int v0 = ls[0], n0 = ls[nlev] - v0;
-        const SharedMesh m{C, kNear ? A.inv_grid[set] : 0.0};
+        const SharedMesh m{C, kMode != kFilter ? A.inv_grid[set] : 0.0};
         // ---- vertices, the first tet and its four caps, from the tables ----
         if (threadIdx.x == 0) {
             C.count = 5;
@@ -921,7 +956,7 @@ __global__ void __launch_bounds__(kCoarseThreads, 1)
                 const int v = S.item;
                 if (v < 0) break;
                 int t = m.near_start(v, n0, L.lane);
-                const int outcome = insert_step<32, kNear>(m, S, L, group, true, v, ex, t, 96, R.status, A.stats, ctr, tests);
+                const int outcome = insert_step<32, kMode>(m, S, L, group, true, v, ex, t, 96, R.status, A.stats, ctr, tests);
                 bool again = false;
                 if (outcome != AI_DONE) {
                     again = outcome == AI_RETRY && S.attempt + 1 < kGroupTries;
