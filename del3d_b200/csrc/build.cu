@@ -1714,6 +1714,23 @@ __global__ void __launch_bounds__(256) k_level_items(const int32_t* __restrict__
                 if ((keys[m] & mask) < k) x = m + 1;
                 else y = m;
             }
+            // Where many vertices there share the key (a cell with far more points than
+            // others, see order.cu), the place at the same fraction of them.
+            const int far = 2 * kGuideReach;
+            if (x + far < hi && (keys[x + far] & mask) == k) {
+                auto bound = [&](int from, int to, bool upper) {   // of k among the keys [from, to)
+                    while (from < to) {
+                        const int m = (from + to) >> 1;
+                        const unsigned long long q = keys[m] & mask;
+                        if (q < k || (upper && q == k)) from = m + 1;
+                        else to = m;
+                    }
+                    return from;
+                };
+                const int own0 = bound(hi, v, false), own1 = bound(v, b[lev + 1], true);   // (the last level's end
+                                                                                             // is the next set's start)
+                x += int(double(v - own0) / double(own1 - own0) * double(bound(x, hi, true) - x));
+            }
             // The nearest of the kGuideReach vertices before and after it there.
             const Pt p = vpt(vx, v);
             double best = 1e300;
@@ -2538,7 +2555,7 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
     // The own order, or - where its keys cannot tell the points apart - the
     // spatial sort with the sorts that find repeated points.
     OwnOrder own;
-    D3G_TRY(own_order_sets(d_xyz, h_off, d_off.p, nsets, growth, scan, own, s));
+    D3G_TRY(own_order_sets(d_xyz, h_off, d_off.p, nsets, growth, scan, status.p + 1, own, s));
     std::vector<int32_t> hlevel;   // own order: first vertex of each (set, level)
     if (own.ok) {
         nv = int(own.nv);

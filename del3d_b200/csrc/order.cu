@@ -36,8 +36,12 @@ namespace {
 constexpr unsigned kFullMask = 0xffffffffu;
 /// Points with equal keys looked through for equal points; a longer run (many
 /// copies of one point, or a set far denser than its bounding cube's grid in
-/// one place) sends the call to the spatial sort.
+/// one place) is sorted again by the grid of its own bounding cube.
 constexpr int kKeyRun = 32;
+/// How often: each time makes the cells at least 2^13 times smaller (2^21 times with
+/// few runs).  Where runs are left even then, or a set's extent overflows, the call goes
+/// to the spatial sort.
+constexpr int kRefine = 12;
 
 __device__ __forceinline__ int set_of(const int64_t* __restrict__ off, int nsets, int64_t g) {
     int lo = 0, hi = nsets - 1;
@@ -182,6 +186,13 @@ __device__ __forceinline__ unsigned long long hilbert3(unsigned x, unsigned y, u
     return spread3(x) << 2 | spread3(y) << 1 | spread3(z);
 }
 
+/// The cell of x, on a grid of 2^bits cells from lo on; scale 0 for one point or an
+/// overflow.
+__device__ __forceinline__ unsigned cell_of(double x, double lo, double scale, int bits) {
+    const double f = (x - lo) * scale;
+    return f > 0.0 ? min(unsigned(f), (1u << bits) - 1) : 0u;
+}
+
 /// The key of every point.  A point's level comes from its hash as a fraction of
 /// 2^32: the coarse levels share the part below kCoarsePoints / n, each `growth`
 /// times the points before it, the others the part above, likewise.
@@ -198,14 +209,13 @@ __global__ void __launch_bounds__(256) k_order_keys(const double* __restrict__ x
             lo[a] = dbl_from_order_key(b[a]);
             ext = fmax(ext, dbl_from_order_key(b[3 + a]) - lo[a]);
         }
-        // 2^bits cells along the longest side; 0 for one point or an overflow.
+        // 2^bits cells along the longest side.
         const double scale = ext > 0.0 ? double((1u << bits) - 1) / ext : 0.0;
         unsigned q[3];
         unsigned long long h = 0;
         for (int a = 0; a < 3; ++a) {
             const double x = xyz[3 * p + a];
-            const double f = (x - lo[a]) * scale;
-            q[a] = f > 0.0 ? min(unsigned(f), (1u << bits) - 1) : 0u;
+            q[a] = cell_of(x, lo[a], scale, bits);
             h = mix64(h + 0x9E3779B97F4A7C15ull + coord_bits(x));
         }
         const int64_t ns = off[set + 1] - off[set];
@@ -230,24 +240,179 @@ __device__ __forceinline__ bool equal_points(const double* __restrict__ xyz, int
     return xyz[3 * i] == xyz[3 * j] && xyz[3 * i + 1] == xyz[3 * j + 1] && xyz[3 * i + 2] == xyz[3 * j + 2];
 }
 
-/// Over the sorted keys (the set above bit `set_shift`): flags the first copy of
-/// every point and counts the others (flags[0], and per set from flags[2] on);
-/// flags[1] is raised by a run of equal keys too long to be looked through.
+/// Over the sorted keys (the set above bit `set_shift`): the first copy of every
+/// point (head[i] == i for one), and how many others there are (flags[0], and per
+/// set from flags[2] on); flags[1] is raised by a run of equal keys too long to be
+/// looked through.
 __global__ void __launch_bounds__(256) k_first_copies(const double* __restrict__ xyz,
                                                       const unsigned long long* __restrict__ keys,
                                                       const int32_t* __restrict__ idx, int64_t n, int nsets,
-                                                      int set_shift, int32_t* __restrict__ first,
+                                                      int set_shift, int32_t* __restrict__ head,
                                                       int* __restrict__ flags) {
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
         const unsigned long long k = keys[i];
-        bool copy = false;
-        int64_t j = i - 1;
-        for (; j >= 0 && i - j <= kKeyRun && keys[j] == k; --j) copy = copy || equal_points(xyz, idx[i], idx[j]);
+        int64_t first = i, j = i - 1;
+        for (; j >= 0 && i - j <= kKeyRun && keys[j] == k; --j)
+            if (equal_points(xyz, idx[i], idx[j])) first = j;
         if (i - j > kKeyRun && j >= 0 && keys[j] == k) atomicOr(flags + 1, 1);
-        first[i] = copy ? 0 : 1;
-        if (copy) {
+        head[i] = int32_t(first);
+        if (first != i) {
             atomicAdd(flags, 1);
             atomicAdd(flags + 2 + (nsets > 1 ? int(k >> set_shift) : 0), 1);
+        }
+    }
+}
+
+// ---- long runs of equal keys --------------------------------------------------------
+//
+// A run's points share set, level and cell.  The runs longer than kKeyRun are sorted
+// again by the Hilbert index in their own bounding cubes, together (run | index), and
+// what is left of them once more, until no run is long but those of one point's
+// copies, whose cube has no extent.  tie[i]: 0 where i's key differs from that of the
+// one before, 1 where it is equal, 2 where the points are.
+
+enum : uint8_t { TIE_NONE = 0, TIE_KEY = 1, TIE_COPY = 2 };
+
+__global__ void k_tie_init(const unsigned long long* __restrict__ keys, int64_t n, uint8_t* __restrict__ tie) {
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
+        tie[i] = i > 0 && keys[i] == keys[i - 1] ? TIE_KEY : TIE_NONE;
+}
+
+/// Heads of runs, to be summed up into every point's run number (plus one).
+__global__ void k_run_heads(const uint8_t* __restrict__ tie, int64_t n, int32_t* __restrict__ head) {
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i <= n; i += int64_t(gridDim.x) * blockDim.x)
+        head[i] = i < n && tie[i] == TIE_NONE ? 1 : 0;
+}
+
+/// start[r]: run r's first point, over the exclusive sums of the heads (n + 1 of them).
+__global__ void k_run_starts(const uint8_t* __restrict__ tie, const int32_t* __restrict__ before, int64_t n,
+                             int32_t* __restrict__ start) {
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i <= n; i += int64_t(gridDim.x) * blockDim.x)
+        if (i == n || tie[i] == TIE_NONE) start[before[i]] = int32_t(i);
+}
+
+__device__ __forceinline__ int run_of(const uint8_t* __restrict__ tie, const int32_t* __restrict__ before, int64_t i) {
+    return before[i] - (tie[i] == TIE_NONE ? 0 : 1);
+}
+
+/// Flags the points of the long runs (not those of copies), and of these the first.
+__global__ void k_long_flags(const uint8_t* __restrict__ tie, const int32_t* __restrict__ before,
+                             const int32_t* __restrict__ start, int64_t n, int32_t* __restrict__ in,
+                             int32_t* __restrict__ first) {
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i <= n; i += int64_t(gridDim.x) * blockDim.x) {
+        int yes = 0, head = 0;
+        if (i < n) {
+            const int r = run_of(tie, before, i), a = start[r], e = start[r + 1];
+            yes = e - a > kKeyRun && tie[a + 1] == TIE_KEY ? 1 : 0;
+            head = yes && a == i ? 1 : 0;
+        }
+        in[i] = yes;
+        first[i] = head;
+    }
+}
+
+/// The flagged points side by side: where they stand (at) and their run among the
+/// long ones (seg); the sums are exclusive, of n + 1 flags.
+__global__ void k_long_gather(const int32_t* __restrict__ in, const int32_t* __restrict__ first, int64_t n,
+                              int32_t* __restrict__ at, int32_t* __restrict__ seg) {
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
+        if (in[i + 1] == in[i]) continue;
+        at[in[i]] = int32_t(i);
+        seg[in[i]] = first[i + 1] - 1;
+    }
+}
+
+__global__ void k_box_init(unsigned long long* box, int nseg) {
+    for (int i = int(blockIdx.x) * blockDim.x + threadIdx.x; i < 6 * nseg; i += gridDim.x * blockDim.x)
+        box[i] = i % 6 < 3 ? ~0ull : 0ull;
+}
+
+/// The bounding boxes of the long runs; a warp whose points are all of one run adds
+/// them up first.
+__global__ void __launch_bounds__(256) k_long_boxes(const double* __restrict__ xyz, const int32_t* __restrict__ idx,
+                                                    const int32_t* __restrict__ at, const int32_t* __restrict__ seg,
+                                                    int m, unsigned long long* __restrict__ box) {
+    const int lane = threadIdx.x & 31;
+    const int padded = (m + 31) & ~31;
+    for (int j = int(blockIdx.x) * blockDim.x + threadIdx.x; j < padded; j += gridDim.x * blockDim.x) {
+        const bool have = j < m;
+        const int s = have ? seg[j] : -1;
+        const int64_t p = have ? idx[at[j]] : 0;
+        const int s0 = __shfl_sync(kFullMask, s, 0);
+        const bool one = __all_sync(kFullMask, s >= 0 && s == s0);
+        for (int a = 0; a < 3; ++a) {
+            unsigned long long lo = have ? dbl_order_key(xyz[3 * p + a]) : 0ull, hi = lo;
+            if (one)
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) {
+                    lo = min(lo, __shfl_xor_sync(kFullMask, lo, o));
+                    hi = max(hi, __shfl_xor_sync(kFullMask, hi, o));
+                }
+            if (have && (!one || lane == 0)) {
+                atomicMin(box + 6 * int64_t(s) + a, lo);
+                atomicMax(box + 6 * int64_t(s) + 3 + a, hi);
+            }
+        }
+    }
+}
+
+__global__ void __launch_bounds__(256) k_long_keys(const double* __restrict__ xyz, const int32_t* __restrict__ idx,
+                                                   const int32_t* __restrict__ at, const int32_t* __restrict__ seg,
+                                                   int m, const unsigned long long* __restrict__ box, int bits,
+                                                   unsigned long long* __restrict__ keys,
+                                                   int32_t* __restrict__ val) {
+    for (int j = int(blockIdx.x) * blockDim.x + threadIdx.x; j < m; j += gridDim.x * blockDim.x) {
+        const unsigned long long* b = box + 6 * int64_t(seg[j]);
+        const int32_t p = idx[at[j]];
+        double ext = 0.0, lo[3];
+        for (int a = 0; a < 3; ++a) {
+            lo[a] = dbl_from_order_key(b[a]);
+            ext = fmax(ext, dbl_from_order_key(b[3 + a]) - lo[a]);
+        }
+        const double scale = ext > 0.0 ? double((1u << bits) - 1) / ext : 0.0;
+        unsigned q[3];
+        for (int a = 0; a < 3; ++a) q[a] = cell_of(xyz[3 * int64_t(p) + a], lo[a], scale, bits);
+        keys[j] = (unsigned long long)seg[j] << (3 * bits) | hilbert3(q[0], q[1], q[2], bits);
+        val[j] = p;
+    }
+}
+
+/// The sorted points back in their places.
+__global__ void k_long_scatter(const unsigned long long* __restrict__ keys, const int32_t* __restrict__ val,
+                               const int32_t* __restrict__ at, int m, const unsigned long long* __restrict__ box,
+                               int seg_shift, int32_t* __restrict__ idx, uint8_t* __restrict__ tie) {
+    for (int j = int(blockIdx.x) * blockDim.x + threadIdx.x; j < m; j += gridDim.x * blockDim.x) {
+        const unsigned long long k = keys[j];
+        const unsigned long long* b = box + 6 * (k >> seg_shift);
+        uint8_t t = TIE_NONE;
+        if (j > 0 && (keys[j - 1] >> seg_shift) == (k >> seg_shift)) {
+            double ext = 0.0;
+            for (int a = 0; a < 3; ++a) ext = fmax(ext, dbl_from_order_key(b[3 + a]) - dbl_from_order_key(b[a]));
+            t = ext == 0.0 ? TIE_COPY : (keys[j - 1] == k ? TIE_KEY : TIE_NONE);
+        }
+        idx[at[j]] = val[j];
+        tie[at[j]] = t;
+    }
+}
+
+/// k_first_copies by the ties.
+__global__ void __launch_bounds__(256) k_first_tied(const double* __restrict__ xyz,
+                                                    const unsigned long long* __restrict__ keys,
+                                                    const int32_t* __restrict__ idx, const uint8_t* __restrict__ tie,
+                                                    const int32_t* __restrict__ before,
+                                                    const int32_t* __restrict__ start, int64_t n, int nsets,
+                                                    int set_shift, int32_t* __restrict__ head,
+                                                    int* __restrict__ flags) {
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
+        int64_t first = i;
+        if (tie[i] == TIE_COPY) first = start[run_of(tie, before, i)];
+        else
+            for (int64_t j = i; tie[j] == TIE_KEY; --j)
+                if (equal_points(xyz, idx[i], idx[j - 1])) first = j - 1;
+        head[i] = int32_t(first);
+        if (first != i) {
+            atomicAdd(flags, 1);
+            atomicAdd(flags + 2 + (nsets > 1 ? int(keys[i] >> set_shift) : 0), 1);
         }
     }
 }
@@ -274,29 +439,45 @@ __global__ void k_ranks(const int32_t* __restrict__ order, const int64_t* __rest
     }
 }
 
-/// With repeated points: the vertices are the first copies, each reported under
-/// the copy whose rank in the reference's order is the last.
-__global__ void __launch_bounds__(256) k_compact_copies(const double* __restrict__ xyz,
-                                                        const unsigned long long* __restrict__ keys,
+/// With repeated points, each is reported under the copy whose rank in the
+/// reference's order is the last: best[first copy] = (rank + 1) << 32 | local index
+/// (0: no other copy).
+__global__ void __launch_bounds__(256) k_best_copies(const int32_t* __restrict__ idx,
+                                                     const int32_t* __restrict__ head,
+                                                     const int32_t* __restrict__ rank,
+                                                     const int64_t* __restrict__ off, int nsets, int64_t n,
+                                                     unsigned long long* __restrict__ best) {
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
+        const int32_t h = head[i];
+        if (h == i) continue;
+        const int32_t g = idx[i], f = idx[h];
+        const int64_t set = off[set_of(off, nsets, g)];
+        atomicMax(best + h, max((unsigned long long)(rank[g] + 1) << 32 | unsigned(g - set),
+                                (unsigned long long)(rank[f] + 1) << 32 | unsigned(f - set)));
+    }
+}
+
+/// The vertices are the first copies.
+__global__ void __launch_bounds__(256) k_compact_copies(const unsigned long long* __restrict__ keys,
                                                         const int32_t* __restrict__ idx,
-                                                        const int32_t* __restrict__ first,
+                                                        const int32_t* __restrict__ head,
                                                         const int32_t* __restrict__ pos,
-                                                        const int32_t* __restrict__ rank,
+                                                        const unsigned long long* __restrict__ best,
                                                         const int64_t* __restrict__ off, int nsets, int64_t n,
                                                         int32_t* __restrict__ vert, int32_t* __restrict__ rep,
                                                         unsigned long long* __restrict__ vkeys) {
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
-        if (!first[i]) continue;
-        const unsigned long long k = keys[i];
-        const int32_t g = idx[i];
-        int32_t best = g;
-        for (int64_t j = i + 1; j < n && keys[j] == k; ++j)
-            if (equal_points(xyz, g, idx[j]) && rank[idx[j]] > rank[best]) best = idx[j];
-        const int32_t v = pos[i];
+        if (head[i] != i) continue;
+        const int32_t g = idx[i], v = pos[i];
         vert[v] = g;
-        rep[v] = int32_t(best - off[set_of(off, nsets, g)]);
-        vkeys[v] = k;
+        rep[v] = best[i] ? int32_t(best[i]) : int32_t(g - off[set_of(off, nsets, g)]);
+        vkeys[v] = keys[i];
     }
+}
+
+__global__ void k_head_flags(const int32_t* __restrict__ head, int64_t n, int32_t* __restrict__ flag) {
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
+        flag[i] = head[i] == i ? 1 : 0;
 }
 
 /// start[c] = the first vertex of (set, level) c, over the vertices' sorted
@@ -328,8 +509,59 @@ int scan_sets(const double* d_xyz, const int64_t* d_off, int nsets, int64_t n, S
     return D3G_OK;
 }
 
+namespace {
+
+/// Sorts the long runs of equal keys (see above) and finds the first copies (head and
+/// flags as k_first_copies; flags[1] stays raised if runs are left).
+int refine_runs(const double* d_xyz, int64_t n, int nsets, int set_shift, const unsigned long long* keys, int32_t* idx,
+                int32_t* head, int* flags, size_t nflags, cudaStream_t s) {
+    DevBuf<uint8_t> tie;
+    DevBuf<int32_t> before, start, in, first, at, seg, val, val2;
+    DevBuf<unsigned long long> box, sub, sub2;
+    D3G_TRY(tie.alloc(size_t(n), s));
+    for (DevBuf<int32_t>* d : {&before, &start, &in, &first}) D3G_TRY(d->alloc(size_t(n) + 2, s));
+    k_tie_init<<<grid_for(n, 256), 256, 0, s>>>(keys, n, tie.p);
+    int left = 0;
+    for (int pass = 0;; ++pass) {
+        k_run_heads<<<grid_for(n + 1, 256), 256, 0, s>>>(tie.p, n, before.p);
+        D3G_TRY(exclusive_scan(before.p, before.p, n + 1, s));
+        k_run_starts<<<grid_for(n + 1, 256), 256, 0, s>>>(tie.p, before.p, n, start.p);
+        k_long_flags<<<grid_for(n + 1, 256), 256, 0, s>>>(tie.p, before.p, start.p, n, in.p, first.p);
+        D3G_TRY(exclusive_scan(in.p, in.p, n + 1, s));
+        D3G_TRY(exclusive_scan(first.p, first.p, n + 1, s));
+        int m = 0, nseg = 0;
+        D3G_CUDA(cudaMemcpyAsync(&m, in.p + n, sizeof m, cudaMemcpyDeviceToHost, s));
+        D3G_CUDA(cudaMemcpyAsync(&nseg, first.p + n, sizeof nseg, cudaMemcpyDeviceToHost, s));
+        D3G_CUDA(cudaStreamSynchronize(s));
+        left = m;
+        if (m == 0 || pass == kRefine) break;
+        const int seg_bits = bits_for(uint64_t(nseg)), bits = std::min(21, (64 - seg_bits) / 3);
+        for (DevBuf<int32_t>* d : {&at, &seg, &val, &val2}) D3G_TRY(d->alloc(size_t(m), s));
+        for (DevBuf<unsigned long long>* d : {&sub, &sub2}) D3G_TRY(d->alloc(size_t(m), s));
+        D3G_TRY(box.alloc(size_t(6) * size_t(nseg), s));
+        k_long_gather<<<grid_for(n, 256), 256, 0, s>>>(in.p, first.p, n, at.p, seg.p);
+        k_box_init<<<grid_for(6 * int64_t(nseg), 256), 256, 0, s>>>(box.p, nseg);
+        k_long_boxes<<<grid_for(m, 256), 256, 0, s>>>(d_xyz, idx, at.p, seg.p, m, box.p);
+        k_long_keys<<<grid_for(m, 256), 256, 0, s>>>(d_xyz, idx, at.p, seg.p, m, box.p, bits, sub.p, val.p);
+        D3G_TRY(sort_pairs(sub.p, sub2.p, val.p, val2.p, m, 0, 3 * bits + seg_bits, s));
+        k_long_scatter<<<grid_for(m, 256), 256, 0, s>>>(sub2.p, val2.p, at.p, m, box.p, 3 * bits, idx, tie.p);
+        D3G_CUDA(cudaGetLastError());
+    }
+    D3G_CUDA(cudaMemsetAsync(flags, 0, sizeof(int) * nflags, s));
+    if (left > 0) {
+        D3G_CUDA(cudaMemsetAsync(flags + 1, 1, sizeof(int), s));
+        return D3G_OK;
+    }
+    k_first_tied<<<grid_for(n, 256), 256, 0, s>>>(d_xyz, keys, idx, tie.p, before.p, start.p, n, nsets, set_shift, head,
+                                                  flags);
+    D3G_CUDA(cudaGetLastError());
+    return D3G_OK;
+}
+
+}  // namespace
+
 int own_order_sets(const double* d_xyz, const int64_t* h_off, const int64_t* d_off, int nsets, int growth,
-                   const SetScan& S, OwnOrder& O, cudaStream_t s) {
+                   const SetScan& S, const uint32_t* d_nonfinite, OwnOrder& O, cudaStream_t s) {
     const int64_t n = h_off[nsets];
     O.ok = false;
     O.nv = 0;
@@ -341,28 +573,42 @@ int own_order_sets(const double* d_xyz, const int64_t* h_off, const int64_t* d_o
     const int bits = std::min(21, (64 - level_bits - set_bits) / 3);
     const int shift = 3 * bits;
     DevBuf<unsigned long long> keys, keys2;
-    DevBuf<int32_t> idx, idx2, first;
+    DevBuf<int32_t> idx, idx2, head;
     DevBuf<int> flags;
     D3G_TRY(keys.alloc(size_t(n), s));
     D3G_TRY(keys2.alloc(size_t(n), s));
     D3G_TRY(idx.alloc(size_t(n), s));
     D3G_TRY(idx2.alloc(size_t(n), s));
-    D3G_TRY(first.alloc(size_t(n), s));
+    D3G_TRY(head.alloc(size_t(n), s));
     D3G_TRY(flags.alloc(2 + size_t(nsets), s));
     D3G_CUDA(cudaMemsetAsync(flags.p, 0, sizeof(int) * (2 + size_t(nsets)), s));
     k_order_keys<<<grid_for(n, 256), 256, 0, s>>>(d_xyz, d_off, nsets, n, S.box.p, growth, bits, level_bits, keys2.p,
                                                   idx2.p);
     D3G_TRY(sort_pairs(keys2.p, keys.p, idx2.p, idx.p, n, 0, shift + level_bits + set_bits, s));
-    k_first_copies<<<grid_for(n, 256), 256, 0, s>>>(d_xyz, keys.p, idx.p, n, nsets, shift + level_bits, first.p,
+    k_first_copies<<<grid_for(n, 256), 256, 0, s>>>(d_xyz, keys.p, idx.p, n, nsets, shift + level_bits, head.p,
                                                      flags.p);
     const int64_t total = int64_t(nsets) * O.levels;
     D3G_TRY(O.level_start.alloc(size_t(total) + 1, s));
     k_level_starts<<<grid_for(n + 1, 256), 256, 0, s>>>(keys.p, n, shift, level_bits, O.levels, total,
                                                         O.level_start.p);
     std::vector<int> hflags(flags.n);
-    D3G_CUDA(cudaMemcpyAsync(hflags.data(), flags.p, sizeof(int) * flags.n, cudaMemcpyDeviceToHost, s));
-    D3G_CUDA(cudaStreamSynchronize(s));
-    if (hflags[1]) return D3G_OK;
+    uint32_t nonfinite = 0;
+    auto read_flags = [&]() -> int {
+        D3G_CUDA(cudaMemcpyAsync(hflags.data(), flags.p, sizeof(int) * flags.n, cudaMemcpyDeviceToHost, s));
+        D3G_CUDA(cudaMemcpyAsync(&nonfinite, d_nonfinite, sizeof nonfinite, cudaMemcpyDeviceToHost, s));
+        D3G_CUDA(cudaStreamSynchronize(s));
+        return D3G_OK;
+    };
+    D3G_TRY(read_flags());
+    if (nonfinite) {      // (its points cannot be ordered)
+        set_error("d3g_build: non-finite coordinate");
+        return D3G_ERR_INVALID_INPUT;
+    }
+    if (hflags[1]) {
+        D3G_TRY(refine_runs(d_xyz, n, nsets, shift + level_bits, keys.p, idx.p, head.p, flags.p, flags.n, s));
+        D3G_TRY(read_flags());
+        if (hflags[1]) return D3G_OK;
+    }
     O.nv = n - hflags[0];
     if (hflags[0] > 0) {
         // Which copy keeps its index is the reference's order's to say, so the sets with
@@ -398,11 +644,16 @@ int own_order_sets(const double* d_xyz, const int64_t* h_off, const int64_t* d_o
         }
         D3G_TRY(spatial_order_sets_device(pts, hoff_of.data(), off_of, m, order.p, s));
         k_ranks<<<grid_for(nm, 256), 256, 0, s>>>(order.p, d_off, dlist.p, off_of, m, nm, rank.p);
-        D3G_TRY(exclusive_scan(first.p, idx2.p, n, s));
+        DevBuf<unsigned long long> best;
+        D3G_TRY(best.alloc(size_t(n), s));
+        D3G_CUDA(cudaMemsetAsync(best.p, 0, sizeof(unsigned long long) * size_t(n), s));
+        k_best_copies<<<grid_for(n, 256), 256, 0, s>>>(idx.p, head.p, rank.p, d_off, nsets, n, best.p);
+        k_head_flags<<<grid_for(n, 256), 256, 0, s>>>(head.p, n, idx2.p);
+        D3G_TRY(exclusive_scan(idx2.p, idx2.p, n, s));
         D3G_TRY(O.vert.alloc(size_t(O.nv), s));
         D3G_TRY(O.rep.alloc(size_t(O.nv), s));
-        k_compact_copies<<<grid_for(n, 256), 256, 0, s>>>(d_xyz, keys.p, idx.p, first.p, idx2.p, rank.p, d_off,
-                                                          nsets, n, O.vert.p, O.rep.p, keys2.p);
+        k_compact_copies<<<grid_for(n, 256), 256, 0, s>>>(keys.p, idx.p, head.p, idx2.p, best.p, d_off, nsets, n,
+                                                          O.vert.p, O.rep.p, keys2.p);
         k_level_starts<<<grid_for(O.nv + 1, 256), 256, 0, s>>>(keys2.p, O.nv, shift, level_bits, O.levels, total,
                                                                O.level_start.p);
     } else {

@@ -58,8 +58,9 @@ struct OwnOrder {
     bool ok = false;             // false: the keys cannot tell the points apart (use the spatial sort)
 };
 /// Orders every set coarse to fine, each level along a Hilbert curve, and finds
-/// the repeated points.  `S` from scan_sets.  Synchronises `s`.
+/// the repeated points.  `S` and `d_nonfinite` from scan_sets (an error status where it
+/// is raised).  Synchronises `s`.
 int own_order_sets(const double* d_xyz, const int64_t* h_off, const int64_t* d_off, int nsets, int growth,
-                   const SetScan& S, OwnOrder& O, cudaStream_t s);
+                   const SetScan& S, const uint32_t* d_nonfinite, OwnOrder& O, cudaStream_t s);
 
 }  // namespace d3g
