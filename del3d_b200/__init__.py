@@ -285,7 +285,8 @@ class _Owned:
     beyond it `array` copies."""
 
     LIMIT = 4 << 30
-    _mu = threading.Lock()
+    # Re-entrant: the collector may end a result kept in a cycle while this thread holds it.
+    _mu = threading.RLock()
     _held = 0
 
     def __init__(self, res, free, nbytes: int):
