@@ -17,6 +17,9 @@ It mirrors the reference's public interface (``include/del3d/delaunay.h``,
 Everything but the input readers runs on the GPU; there is no CPU fallback.  Importing works without a
 GPU (the library loads), but every call then fails with :class:`Del3dError`.
 
+Results of host calls are arrays over pinned (page-locked) memory of the library
+as a rule; a slice of one keeps the whole result's block, ``slice.copy()`` does not.
+
 One documented difference: ``finite_cells()`` comes back in a canonical order
 (each tet rotated by an even permutation so its smallest index leads, tets
 sorted lexicographically) instead of the reference's cell-allocation order; the
@@ -281,20 +284,29 @@ class _Owned:
     The library hands results out in pinned blocks it keeps for reuse; an array
     over such a block costs nothing, where a copy into fresh pages takes longer
     than the copy from the device (475 MB of cells of a burst of requests: about
-    100 ms of 170).  Blocks lent this way are bounded by LIMIT bytes in all;
-    beyond it `array` copies."""
+    100 ms of 170).  But a block that does not come back has to be replaced, and
+    pinning takes twice as long as copying out (16 MB: 6.2 ms, the copy 3.7).  So a
+    program is lent FIRST bytes (and FIRST_RESULTS results) to begin with and beyond
+    that as much as it has given back, LIMIT bytes and MOST_RESULTS at most; what is
+    not lent is copied, and its block is free again at once.  (Blocks may be up to
+    twice as large as the results in them.)"""
 
     LIMIT = 4 << 30
+    FIRST, FIRST_RESULTS, MOST_RESULTS = 256 << 20, 256, 4096
     # Re-entrant: the collector may end a result kept in a cycle while this thread holds it.
     _mu = threading.RLock()
-    _held = 0
+    _held = _results = 0            # lent now
+    _back = _back_results = 0       # given back so far
 
     def __init__(self, res, free, nbytes: int):
         self._res, self._free, self._bytes = res, free, int(nbytes)
-        with _Owned._mu:
-            self.lent = _Owned._held + self._bytes <= _Owned.LIMIT
+        cls = _Owned
+        with cls._mu:
+            self.lent = (cls._held + self._bytes <= min(cls.LIMIT, cls.FIRST + cls._back) and
+                         cls._results < min(cls.MOST_RESULTS, cls.FIRST_RESULTS + cls._back_results))
             if self.lent:
-                _Owned._held += self._bytes
+                cls._held += self._bytes
+                cls._results += 1
 
     def array(self, pointer, dtype, n: int) -> np.ndarray:
         n = int(n)
@@ -309,6 +321,9 @@ class _Owned:
             if self.lent:
                 with _Owned._mu:
                     _Owned._held -= self._bytes
+                    _Owned._results -= 1
+                    _Owned._back += self._bytes
+                    _Owned._back_results += 1
         except Exception:
             pass                # the interpreter is going down
 
