@@ -166,36 +166,38 @@ struct Round {
 };
 
 /// A thread's conflict-test counters, added to Round::pstats once at the end
-/// of a launch (flush_counters).  `flags` holds the uncertain count in its low
-/// 20 bits and the tie count above: a thread makes far fewer than 2^20 tests in
-/// one launch (a warp inserts a few hundred points per launch, a few tests per
-/// lane each).  The insertion kernels keep them in shared memory, one slot per
-/// thread, so that they take no registers from the loops they count in.
+/// of a launch (flush_counters).  `flags` holds the uncertain count in its low half
+/// and the tie count above.  The insertion kernels keep them in shared memory, one
+/// slot per thread, so that they take no registers from the loops they count in.
 constexpr int kCounterThreads = 128;   // the insertion kernels' block size
 
 struct SharedCounters {
     unsigned* tests;
-    unsigned* flags;
+    unsigned long long* flags;
     int* max_region;
     __device__ void count(int r) const {
         tests[threadIdx.x] += 1;
-        flags[threadIdx.x] += ((r >> 1) & 1) + (((r >> 2) & 1) << 20);
+        flags[threadIdx.x] += (unsigned long long)(unsigned((r >> 2) & 1)) << 32 | unsigned((r >> 1) & 1);
     }
     __device__ void region(int c) const { max_region[threadIdx.x] = max(max_region[threadIdx.x], c); }
+    __device__ void clear() const {
+        tests[threadIdx.x] = 0;
+        flags[threadIdx.x] = 0;
+        max_region[threadIdx.x] = 0;
+    }
 };
 
-#define D3G_SHARED_COUNTERS(name)                                                   \
-    __shared__ unsigned name##_t[kCounterThreads], name##_f[kCounterThreads];     \
-    __shared__ int name##_m[kCounterThreads];                                       \
-    name##_t[threadIdx.x] = 0;                                                      \
-    name##_f[threadIdx.x] = 0;                                                      \
-    name##_m[threadIdx.x] = 0;                                                      \
-    const SharedCounters name{name##_t, name##_f, name##_m}
+#define D3G_SHARED_COUNTERS(name)                                \
+    __shared__ unsigned name##_t[kCounterThreads];               \
+    __shared__ unsigned long long name##_f[kCounterThreads];     \
+    __shared__ int name##_m[kCounterThreads];                    \
+    const SharedCounters name{name##_t, name##_f, name##_m};     \
+    name.clear()
 
 /// Sums the warp's counters into R.pstats (one atomic per counter per warp).
 __device__ void flush_counters(const SharedCounters& c, const Round& R) {
-    unsigned long long t = c.tests[threadIdx.x], u = c.flags[threadIdx.x] & 0xFFFFFu,
-                       z = c.flags[threadIdx.x] >> 20;
+    unsigned long long t = c.tests[threadIdx.x], u = c.flags[threadIdx.x] & 0xFFFFFFFFu,
+                       z = c.flags[threadIdx.x] >> 32;
     int m = c.max_region[threadIdx.x];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {

@@ -721,7 +721,8 @@ struct CoarseShared {
     int lock[kCoarseTets];
     uint16_t vert_tet[kCoarseVerts], guide[kCoarseVerts];    // 0xFFFF: none
     CoarseScratch scratch[kCoarseThreads / 32];
-    unsigned tests[kCoarseThreads], flags[kCoarseThreads];
+    unsigned long long flags[kCoarseThreads];
+    unsigned tests[kCoarseThreads];
     int max_region[kCoarseThreads];
     int count, next, set, base, extra[2], first[4];
     int stride;
@@ -835,8 +836,7 @@ __global__ void __launch_bounds__(kCoarseThreads, 1)
     const int group = int(threadIdx.x >> 5);
     CoarseScratch& S = C.scratch[group];
     const SharedCounters ctr{C.tests, C.flags, C.max_region};
-    ctr.tests[threadIdx.x] = ctr.flags[threadIdx.x] = 0;
-    ctr.max_region[threadIdx.x] = 0;
+    ctr.clear();
     unsigned tests = 0;
     if (L.sub == 0) S.won = S.tries = S.nC = S.nF = 0;
     for (;;) {
