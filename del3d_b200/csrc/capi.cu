@@ -235,6 +235,7 @@ cudaError_t device_block_alloc(void** p, size_t bytes, cudaStream_t s, size_t* c
     // Sizes in steps of 1/16 to 1/32 of themselves: a build's tables have a few slots
     // more or less each time, and a request a little above every idle block would go
     // to the pool, which can hold the thread for hundreds of milliseconds.
+    const size_t asked = bytes;
     {
         size_t step = kBlockCacheMin >> 4;
         while (step << 5 <= bytes) step <<= 1;
@@ -286,6 +287,11 @@ cudaError_t device_block_alloc(void** p, size_t bytes, cudaStream_t s, size_t* c
         }
         if (!all.empty()) {
             free_idle_on(c, all, s);
+            e = cudaMallocAsync(p, bytes, s);
+        }
+        if (e == cudaErrorMemoryAllocation && asked < bytes) {   // the last of the memory
+            cudaGetLastError();
+            bytes = asked;
             e = cudaMallocAsync(p, bytes, s);
         }
     }
