@@ -403,10 +403,15 @@ int predicates_device(const double* d_pts, int64_t n_pts, const int32_t* d_idx, 
         } else {
             k_filter_in_sphere<<<g, blk, 0, stream>>>(d_pts, n_pts, d_idx, nq, d_out, queue.p,
                                                       qcount, status);
-            D3G_TRY(rest.alloc(size_t(nq), stream));
-            k_near_in_sphere<<<kNumSMs * 8, 128, 0, stream>>>(d_pts, d_idx, d_out, queue.p, qcount,
-                                                              kind == D3G_IN_SPHERE ? 1 : 0, rest.p, ncount, status);
-            k_exact_in_sphere<<<kNumSMs * 8, 128, 0, stream>>>(d_pts, d_idx, d_out, rest.p, ncount,
+            // (without room for a second queue, every queued call goes to the exact stage)
+            const int room = rest.alloc(size_t(nq), stream);
+            if (room == D3G_OK)
+                k_near_in_sphere<<<kNumSMs * 8, 128, 0, stream>>>(d_pts, d_idx, d_out, queue.p, qcount,
+                                                                  kind == D3G_IN_SPHERE ? 1 : 0, rest.p, ncount, status);
+            else if (room == D3G_ERR_OOM) cudaGetLastError();
+            else return room;
+            k_exact_in_sphere<<<kNumSMs * 8, 128, 0, stream>>>(d_pts, d_idx, d_out, room == D3G_OK ? rest.p : queue.p,
+                                                               room == D3G_OK ? ncount : qcount,
                                                                kind == D3G_IN_SPHERE ? 1 : 0, wqueue.p, wcount,
                                                                wcap, status);
         }
@@ -419,6 +424,7 @@ int predicates_device(const double* d_pts, int64_t n_pts, const int32_t* d_idx, 
     D3G_CUDA(cudaMemcpyAsync(host_counters, counters.p, sizeof host_counters, cudaMemcpyDeviceToHost,
                              stream));
     queue.release();
+    rest.release();
     D3G_CUDA(cudaStreamSynchronize(stream));
     // The wide tier, for the calls queued: kWideSlots at a time, each thread
     // with its own piece of the arena.

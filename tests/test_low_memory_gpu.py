@@ -62,3 +62,10 @@ def test_a_block_of_its_own_size(cuda):
     that.  4104 MiB of queue, 4352 with the step, and 4240 free."""
     nq = 4104 * MB // 8
     _with_only(8 * nq + 136 * MB, nq, 4, d3.ORIENT3D)
+
+
+def test_in_sphere_without_a_second_queue(cuda):
+    """The queue of calls for the exact stage has room for one entry a query (0.8 GB here); the
+    64-bit stage's second one is done without where there is no room for it."""
+    nq = 100_000_000
+    _with_only(8 * nq + 300 * MB, nq, 5, d3.IN_SPHERE)
