@@ -168,18 +168,21 @@ struct Round {
 /// A thread's conflict-test counters, added to Round::pstats once at the end
 /// of a launch (flush_counters).  `flags` holds the uncertain count in its low half
 /// and the tie count above.  The insertion kernels keep them in shared memory, one
-/// slot per thread, so that they take no registers from the loops they count in.
+/// slot per thread, so that they take no registers from the loops they count in -
+/// and no more than 15 bytes a thread: with 16, five blocks of k_insert_groups<8, ...>
+/// take more than 196 KB, and L1 shrinks from 60 to 28 KB (10^7 uniform points 102 ->
+/// 108 ms).
 constexpr int kCounterThreads = 128;   // the insertion kernels' block size
 
 struct SharedCounters {
     unsigned* tests;
     unsigned long long* flags;
-    int* max_region;
+    uint16_t* max_region;   // (regions hold kBigCapacity tets at most here)
     __device__ void count(int r) const {
         tests[threadIdx.x] += 1;
         flags[threadIdx.x] += (unsigned long long)(unsigned((r >> 2) & 1)) << 32 | unsigned((r >> 1) & 1);
     }
-    __device__ void region(int c) const { max_region[threadIdx.x] = max(max_region[threadIdx.x], c); }
+    __device__ void region(int c) const { max_region[threadIdx.x] = uint16_t(max(int(max_region[threadIdx.x]), c)); }
     __device__ void clear() const {
         tests[threadIdx.x] = 0;
         flags[threadIdx.x] = 0;
@@ -190,7 +193,7 @@ struct SharedCounters {
 #define D3G_SHARED_COUNTERS(name)                                \
     __shared__ unsigned name##_t[kCounterThreads];               \
     __shared__ unsigned long long name##_f[kCounterThreads];     \
-    __shared__ int name##_m[kCounterThreads];                    \
+    __shared__ uint16_t name##_m[kCounterThreads];               \
     const SharedCounters name{name##_t, name##_f, name##_m};     \
     name.clear()
 

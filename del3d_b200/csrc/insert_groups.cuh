@@ -109,6 +109,11 @@ __device__ __forceinline__ void st_rec(const Tables& T, int t, const int4& tv, c
                  : "memory");
 }
 
+/// Five blocks with their static shared memory (counters, queue) and the 1 KB that the
+/// system takes of each leave L1 60 KB.
+static_assert(kGroupBlocks * (sizeof(GroupScratch<8, 64>) * 16 + 15 * kCounterThreads + 64 + 1024) <= 196 * 1024,
+              "k_insert_groups' shared memory");
+
 /// The most groups a launch has.
 constexpr int kMaxGroups = kNumSMs * kGroupBlocks * (kGroupThreads / 8);
 
@@ -723,7 +728,7 @@ struct CoarseShared {
     CoarseScratch scratch[kCoarseThreads / 32];
     unsigned long long flags[kCoarseThreads];
     unsigned tests[kCoarseThreads];
-    int max_region[kCoarseThreads];
+    uint16_t max_region[kCoarseThreads];
     int count, next, set, base, extra[2], first[4];
     int stride;
 };
