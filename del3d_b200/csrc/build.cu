@@ -843,8 +843,8 @@ struct AsyncCtx {
     int nw;
     unsigned long long* ekey;       // per warp slot: 3 edge keys per boundary facet (re-star)
     unsigned long long* stats;      // [0] lock conflicts, [1] walk restarts, [2] invalid seeds,
-                                    // [3] regions too big, [4] points left, [5] first points left,
-                                    // [6] points with a test the filters could not decide
+                                    // [3] regions too big, [4] points left,
+                                    // [5] points with a test the filters could not decide
 };
 
 using LockRef = cuda::atomic_ref<int, cuda::thread_scope_device>;
@@ -1486,42 +1486,21 @@ __global__ void __launch_bounds__(128, 8) k_insert_full(Tables T, Workers W, Asy
         if (q >= A.nw) break;
         const int w = int((int64_t(q) * A.stride) % A.nw);
         const bool ex = (W.set_exact[W.wset[w]] & EX_BOTH) == EX_BOTH;
-        const int b = W.beg[w], len = W.end[w] - b;
-        const int4 sk = W.skips[W.wset[w]];
-        int pos = W.pos[w], left = W.left[w];
-        int v = W.cur[w];
-        int last = -1;
-        const int guide = W.guide[w];
-        while (v >= 0) {
-            int outcome = AI_RETRY;
-            for (int attempt = 0; attempt < kAsyncRetries && outcome == AI_RETRY; ++attempt) {
-                if (attempt > 0) __nanosleep(200u << min(attempt, 6));
-                const int t0 = __ldcg(T.vert_tet + (last >= 0 ? last : guide));
-                outcome = insert_full(v, t0, T, W, A, vx, ex, R.status, slot, lane, &nC, &nF, ctr,
-                                              handed_tn[threadIdx.x >> 5]);
-                ++tries;
-                if (__ldcg(R.status) != 0) outcome = AI_LEAVE;
-            }
-            if (outcome == AI_DONE) {
-                ++won;
-                last = v;
-            } else if (lane == 0) {
-                A.leftover[atomicAdd(A.n_leftover, 1)] = v;
-                atomicAdd(A.stats + 4, 1ull);
-                if (last < 0) atomicAdd(A.stats + 5, 1ull);
-            }
-            if (__ldcg(R.status) != 0) break;
-            // next point of the chunk (as next_point)
-            v = -1;
-            while (left > 0) {
-                const int c = b + pos;
-                pos = pos + 1 == len ? 0 : pos + 1;
-                --left;
-                if (c != sk.x && c != sk.y && c != sk.z && c != sk.w) {
-                    v = c;
-                    break;
-                }
-            }
+        const int v = W.cur[w];
+        if (v < 0) continue;
+        int outcome = AI_RETRY;
+        for (int attempt = 0; attempt < kAsyncRetries && outcome == AI_RETRY; ++attempt) {
+            if (attempt > 0) __nanosleep(200u << min(attempt, 6));
+            outcome = insert_full(v, __ldcg(T.vert_tet + W.guide[w]), T, W, A, vx, ex, R.status, slot, lane, &nC, &nF,
+                                  ctr, handed_tn[threadIdx.x >> 5]);
+            ++tries;
+            if (__ldcg(R.status) != 0) outcome = AI_LEAVE;
+        }
+        if (outcome == AI_DONE) {
+            ++won;
+        } else if (lane == 0) {
+            A.leftover[atomicAdd(A.n_leftover, 1)] = v;
+            atomicAdd(A.stats + 4, 1ull);
         }
         if (__ldcg(R.status) != 0) break;
     }
@@ -2788,13 +2767,13 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
     D3G_TRY(steps.alloc(2, s));
     D3G_TRY(totals.alloc(6, s));
     D3G_TRY(pstats.alloc(4, s));
-    D3G_TRY(astats.alloc(7, s));
+    D3G_TRY(astats.alloc(6, s));
     D3G_TRY(dround.alloc(1, s));
     D3G_CUDA(cudaMemsetAsync(steps.p, 0, 2 * sizeof(unsigned long long), s));
     D3G_CUDA(cudaMemsetAsync(sums.p, 0, 2 * sizeof(unsigned long long), s));
     D3G_CUDA(cudaMemsetAsync(totals.p, 0, 6 * sizeof(unsigned long long), s));
     D3G_CUDA(cudaMemsetAsync(pstats.p, 0, 4 * sizeof(unsigned long long), s));
-    D3G_CUDA(cudaMemsetAsync(astats.p, 0, 7 * sizeof(unsigned long long), s));
+    D3G_CUDA(cudaMemsetAsync(astats.p, 0, 6 * sizeof(unsigned long long), s));
     D3G_CUDA(cudaMemsetAsync(dround.p, 0, sizeof(unsigned), s));
     Rd.counters = counters.p;
     Rd.sums = sums.p;
@@ -3303,7 +3282,7 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
             R.stats.launches_async += 1;
         };
         // The variant that settles undecided tests of near points in 64 bits needs more
-        // registers (36 bytes of spills at 96): 10^7 uniform points 107 -> 114 ms, 4096
+        // registers (52 bytes of spills stored and 60 loaded at 96): 10^7 uniform points 107 -> 114 ms, 4096
         // mixed sets 410 -> 437, but the 10^6 sphere on a 2^-10 grid 79 -> 27.  So it takes
         // the levels of a build most of whose points lie on such grids, and elsewhere
         // only what the plain one leaves.
@@ -3490,7 +3469,7 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
                 float ms = 0.f;
                 cudaEventElapsedTime(&ms, ev0, ev1);
                 int c[4] = {0, 0, 0, 0}, nd = 0;
-                unsigned long long as[7], ht[2];
+                unsigned long long as[6], ht[2];
                 cudaMemcpy(c, cnt.p + 4 * std::max(list - 1, 0), sizeof c, cudaMemcpyDeviceToHost);
                 cudaMemcpy(&nd, A.n_defer, sizeof nd, cudaMemcpyDeviceToHost);
                 cudaMemcpy(as, astats.p, sizeof as, cudaMemcpyDeviceToHost);
@@ -3499,7 +3478,7 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
                         "deferred so far %d, %.3f ms | inserted %llu attempts %llu lock-conflicts %llu walk-restarts %llu "
                         "bad-seeds %llu too-big %llu left %llu undecided %llu\n",
                         lev, sets_of[size_t(lev)], m_of[lev], int(std::min<int64_t>(groups_of[size_t(lev)], kMaxGroups)),
-                        G, c[1], nd, ms, ht[0], ht[1], as[0], as[1], as[2], as[3], as[4], as[6]);
+                        G, c[1], nd, ms, ht[0], ht[1], as[0], as[1], as[2], as[3], as[4], as[5]);
                 cudaEventDestroy(ev0);
                 cudaEventDestroy(ev1);
             }
@@ -3522,7 +3501,7 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
         D3G_TRY(run_lockstep());
     }
     {
-        unsigned long long hs2[2] = {0, 0}, ht[6], hst[2] = {0, 0}, hp[4] = {0, 0, 0, 0}, ha[7] = {};
+        unsigned long long hs2[2] = {0, 0}, ht[6], hst[2] = {0, 0}, hp[4] = {0, 0, 0, 0}, ha[6] = {};
         D3G_CUDA(cudaMemcpyAsync(hp, pstats.p, sizeof hp, cudaMemcpyDeviceToHost, s));
         D3G_CUDA(cudaMemcpyAsync(ha, astats.p, sizeof ha, cudaMemcpyDeviceToHost, s));
         D3G_CUDA(cudaMemcpyAsync(hs2, sums.p, sizeof hs2, cudaMemcpyDeviceToHost, s));
@@ -3539,7 +3518,7 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
         R.stats.uncertain_tests = int64_t(hp[1]);
         R.stats.tie_breaks = int64_t(hp[2]);
         R.stats.max_region_tets = int64_t(hp[3]);
-        R.stats.deferred_points = int64_t(ha[6]);
+        R.stats.deferred_points = int64_t(ha[5]);
         if (use_async) R.stats.async_inserted = int64_t(ht[0]) - to_rounds;
     }
     // Release round scratch before the output stage.

@@ -16,11 +16,12 @@
 // Everything an insertion needs between reading the mesh and writing it - the
 // facets still to test, the region's tets, the boundary facets with their
 // vertices - stays in shared memory, so each tet and each lock word goes over
-// L2 once.
+// L2 once per insertion, but for a record read along with its lock attempt and
+// again under the lock.
 
 constexpr int kGroupThreads = 128;
 /// Blocks per SM the insertion kernel is compiled for: 20 warps at 96 registers
-/// (92 used, no spills) and 38 KB of scratch a block.  With 6 (80 registers, 80
+/// (94 used with 8 or 16 lanes, 96 with 32; no spills) and 38 KB of scratch a block.  With 6 (80 registers, 80
 /// bytes of spills, 228 KB of the SM's 256 taken by scratch, so spills miss L1)
 /// 4096 mixed sets took 440 ms against 409, with 4 457 against 429.
 constexpr int kGroupBlocks = 5;
@@ -417,7 +418,7 @@ __device__ __forceinline__ int insert_step(const M& m, Scratch& S, const Lanes<G
                 }
                 for (int k = L.sub; k < nreg; k += G) m.set(S.reg[k], 0);
                 const bool bad = trouble && !und && !ab;   // the seed
-                if (L.sub == 0) atomicAdd(stats + (ab ? 0 : (und ? 6 : (bad ? 2 : 3))), 1ull);
+                if (L.sub == 0) atomicAdd(stats + (ab ? 0 : (und ? 5 : (bad ? 2 : 3))), 1ull);
                 outcome = und || (bad && fuzzy) ? AI_DEFER : (ab || bad ? AI_RETRY : AI_LEAVE);
                 growing = false;
             }

@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(256) k_scan_sets(const double* __restrict__ xy
 }
 
 /// A 64-bit finaliser (shift, multiply, shift): every input bit reaches every
-/// output bit.
+/// output bit.  Constant and shifts are those published as "degski64".
 __device__ __forceinline__ unsigned long long mix64(unsigned long long x) {
     x ^= x >> 32;
     x *= 0xD6E8FEB86659FD93ull;

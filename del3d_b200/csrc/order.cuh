@@ -8,7 +8,7 @@
 
 namespace d3g {
 
-/// Levels a build's own order uses at most (growth 2 of 2^27 points: 22).
+/// Levels a build's own order uses at most (growth 2 of 2^27 points: 25).
 constexpr int kMaxOrderLevels = 32;
 
 /// The coarsest levels of every set together have about this many points (fewer

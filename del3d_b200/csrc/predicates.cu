@@ -156,7 +156,8 @@ __global__ void __launch_bounds__(256) k_filter_in_sphere(const double* __restri
 /// orientations are exact in double at that size.  The others go to `rest`, for
 /// k_exact_in_sphere, whose limbs need 255 registers.  Bound by the gather of the
 /// points and 64-bit multiplies (10^7 queries, a tenth of them degenerate: 83 us here and
-/// 190 for the rest, 730 before; the call 1.88 -> 1.08 ms).
+/// 190 for the rest, 730 before; the call 1.88 -> 1.08 ms.  The rest is about seven queries
+/// that name one point twice: 190 us is the latency of one exact evaluation).
 constexpr double kNearSteps = 2600.0;
 __global__ void __launch_bounds__(128) k_near_in_sphere(const double* __restrict__ pts,
                                                         const int32_t* __restrict__ idx, int8_t* __restrict__ out,
