@@ -3333,14 +3333,16 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
         // longer than a group waits for another - by one alone; the rest by k_insert_full.
         auto drain = [&]() -> int {
             int nd = 0, nb[5] = {0, 0, 0, 0, 0};
+            std::vector<int> seen(ndefer_lists + 6);
             auto look = [&]() -> int {
                 uint32_t hs = 0;
                 D3G_CUDA(cudaGetLastError());
                 if (opt.timing) cudaEventRecord(kev[1], s);
-                D3G_CUDA(cudaMemcpyAsync(&nd, n_defer_of(deferred), sizeof nd, cudaMemcpyDeviceToHost, s));
-                D3G_CUDA(cudaMemcpyAsync(nb, big_ctl, sizeof nb, cudaMemcpyDeviceToHost, s));
+                D3G_CUDA(cudaMemcpyAsync(seen.data(), n_defer_of(0), sizeof(int) * seen.size(), cudaMemcpyDeviceToHost, s));
                 D3G_CUDA(cudaMemcpyAsync(&hs, status.p, sizeof hs, cudaMemcpyDeviceToHost, s));
                 D3G_CUDA(cudaStreamSynchronize(s));
+                nd = seen[size_t(deferred)];
+                std::copy(seen.end() - 5, seen.end(), nb);
                 if (opt.timing) {
                     float am = 0.f;
                     cudaEventElapsedTime(&am, kev[0], kev[1]);
@@ -3460,7 +3462,7 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
                     k_locate<<<grid_for(m_of[lev], 128), 128, 0, s>>>(T, A, vx.p);
                 launch(G, int(std::min<int64_t>(groups_of[size_t(lev)], 1 << 24)), main_mode);
                 left_pass(kNumSMs * (kGroupThreads / 32));
-                if (may_defer) D3G_TRY(look_behind(lev));
+                if (may_defer && lev < nlev - 1) D3G_TRY(look_behind(lev));   // (the last level is drained)
             }
             D3G_CUDA(cudaGetLastError());
             if (trace) {

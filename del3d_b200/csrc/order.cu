@@ -243,12 +243,14 @@ __device__ __forceinline__ bool equal_points(const double* __restrict__ xyz, int
 /// Over the sorted keys (the set above bit `set_shift`): the first copy of every
 /// point (head[i] == i for one), and how many others there are (flags[0], and per
 /// set from flags[2] on); flags[1] is raised by a run of equal keys too long to be
-/// looked through.
+/// looked through.  The finite check's result goes behind the flags, to be read back
+/// with them.
 __global__ void __launch_bounds__(256) k_first_copies(const double* __restrict__ xyz,
                                                       const unsigned long long* __restrict__ keys,
                                                       const int32_t* __restrict__ idx, int64_t n, int nsets,
-                                                      int set_shift, int32_t* __restrict__ head,
-                                                      int* __restrict__ flags) {
+                                                      int set_shift, const uint32_t* __restrict__ nonfinite,
+                                                      int32_t* __restrict__ head, int* __restrict__ flags) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) flags[2 + nsets] = int(*nonfinite);
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
         const unsigned long long k = keys[i];
         int64_t first = i, j = i - 1;
@@ -580,27 +582,25 @@ int own_order_sets(const double* d_xyz, const int64_t* h_off, const int64_t* d_o
     D3G_TRY(idx.alloc(size_t(n), s));
     D3G_TRY(idx2.alloc(size_t(n), s));
     D3G_TRY(head.alloc(size_t(n), s));
-    D3G_TRY(flags.alloc(2 + size_t(nsets), s));
-    D3G_CUDA(cudaMemsetAsync(flags.p, 0, sizeof(int) * (2 + size_t(nsets)), s));
+    D3G_TRY(flags.alloc(3 + size_t(nsets), s));
+    D3G_CUDA(cudaMemsetAsync(flags.p, 0, sizeof(int) * flags.n, s));
     k_order_keys<<<grid_for(n, 256), 256, 0, s>>>(d_xyz, d_off, nsets, n, S.box.p, growth, bits, level_bits, keys2.p,
                                                   idx2.p);
     D3G_TRY(sort_pairs(keys2.p, keys.p, idx2.p, idx.p, n, 0, shift + level_bits + set_bits, s));
-    k_first_copies<<<grid_for(n, 256), 256, 0, s>>>(d_xyz, keys.p, idx.p, n, nsets, shift + level_bits, head.p,
-                                                     flags.p);
+    k_first_copies<<<grid_for(n, 256), 256, 0, s>>>(d_xyz, keys.p, idx.p, n, nsets, shift + level_bits, d_nonfinite,
+                                                     head.p, flags.p);
     const int64_t total = int64_t(nsets) * O.levels;
     D3G_TRY(O.level_start.alloc(size_t(total) + 1, s));
     k_level_starts<<<grid_for(n + 1, 256), 256, 0, s>>>(keys.p, n, shift, level_bits, O.levels, total,
                                                         O.level_start.p);
     std::vector<int> hflags(flags.n);
-    uint32_t nonfinite = 0;
     auto read_flags = [&]() -> int {
         D3G_CUDA(cudaMemcpyAsync(hflags.data(), flags.p, sizeof(int) * flags.n, cudaMemcpyDeviceToHost, s));
-        D3G_CUDA(cudaMemcpyAsync(&nonfinite, d_nonfinite, sizeof nonfinite, cudaMemcpyDeviceToHost, s));
         D3G_CUDA(cudaStreamSynchronize(s));
         return D3G_OK;
     };
     D3G_TRY(read_flags());
-    if (nonfinite) {      // (its points cannot be ordered)
+    if (hflags.back()) {      // (its points cannot be ordered)
         set_error("d3g_build: non-finite coordinate");
         return D3G_ERR_INVALID_INPUT;
     }
