@@ -266,8 +266,11 @@ __device__ __forceinline__ int insert_step(const M& m, Scratch& S, const Lanes<G
             m.rec(t, tv, tn);
         }
         int prev = -1, step = 0;
-        uint32_t h = uint32_t(v) * 2654435761u + 12345u;
-        const int limit = min(kAsyncWalkLimit, m.walk_limit());
+        // Another way and more steps at each attempt, so that a point whose way is very long
+        // (along the hull of points nearly in a line, say) does not go it time and again.
+        const int attempt = S.attempt;
+        uint32_t h = (uint32_t(v) + uint32_t(attempt) * 0x9E3779B9u) * 2654435761u + 12345u;
+        const int limit = min(min(kAsyncWalkLimit, 1024 << min(attempt, 4)), m.walk_limit());
         bool walking = live;
         while (__any_sync(kFull, walking)) {
             int4 pv = make_int4(0, 0, 0, 0), pn = pv;
@@ -309,7 +312,7 @@ __device__ __forceinline__ int insert_step(const M& m, Scratch& S, const Lanes<G
                 } else if (++step >= limit) {
                     outcome = AI_RETRY;
                     walking = false;
-                    t = -1;
+                    if (attempt & 1) t = -1;        // from the guide again, else on from here
                     if (L.sub == 0) atomicAdd(stats + 1, 1ull);
                 }
             }
