@@ -824,7 +824,9 @@ constexpr int kExactPasses = 3;
 // points on, a set with half of its 300000 points in one corner of 2^-30 of its
 // extent took 990 ms, without any 11 s.
 constexpr int kUndecidedShare = 128;
-// Points the last pass of a single group takes at most.
+// Groups with room for kBigCapacity, and points the last pass of a single one takes at
+// most.
+constexpr int kBigGroups = 16;
 constexpr int kLonePoints = 256;
 // Vertices of the level before, to either side along the curve, among which a
 // vertex's guide is the nearest.
@@ -3213,9 +3215,9 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
         for (auto& l : left) D3G_TRY(l.alloc(size_t(nv), s));
         D3G_TRY(pool.alloc(size_t(kMaxGroups), s));
         // Counters: four per list of points left, one per list of deferred ones (at most
-        // one after each level and kExactPasses each time they are drained), six more.
+        // one after each level and kExactPasses each time they are drained), seven more.
         const size_t nleft_lists = size_t(nlev) + kLastPasses + 1, ndefer_lists = size_t(nlev) * (kExactPasses + 1) + 2;
-        D3G_TRY(cnt.alloc(4 * nleft_lists + ndefer_lists + 6, s));
+        D3G_TRY(cnt.alloc(4 * nleft_lists + ndefer_lists + 7, s));
         D3G_CUDA(cudaMemcpyAsync(dctl.p, ctl.data(), sizeof(int) * ctl.size(), cudaMemcpyHostToDevice, s));
         D3G_CUDA(cudaMemsetAsync(pool.p, 0, sizeof(int4) * size_t(kMaxGroups), s));
         D3G_CUDA(cudaMemsetAsync(cnt.p, 0, sizeof(int) * cnt.n, s));
@@ -3248,8 +3250,8 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
         // Likewise the lists of points with undecided tests.
         auto defer_of = [&](int k) { return defer[k & 1].p; };
         auto n_defer_of = [&](int k) { return cnt.p + 4 * nleft_lists + k; };
-        int* const coarse_queue = cnt.p + (cnt.n - 6);
-        int* const big_ctl = coarse_queue + 1;   // [0] points too big, [1] and [3] queue heads, [2] and [4] left
+        int* const coarse_queue = cnt.p + (cnt.n - 7);
+        int* const big_ctl = coarse_queue + 1;   // [0] points too big, [1], [3] and [5] queue heads, [2] and [4] left
         int list = 0, deferred = 0;
         GroupArgs A{};
         A.lock = alock.p;
@@ -3329,13 +3331,14 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
             return D3G_OK;
         };
         // What the levels' passes could not do, while the host looks on: points with
-        // undecided tests, with fewer and fewer groups in the way of one another; regions
-        // beyond the widest groups' scratch (and points worn out by conflicts) with one of
-        // kBigCapacity, by 16 groups, then - such regions of one set overlap, and take
-        // longer than a group waits for another - by one alone; the rest by k_insert_full.
+        // undecided tests, with fewer and fewer groups in the way of one another while at
+        // least half of them go in; then these, regions beyond the widest groups' scratch and
+        // points worn out by conflicts with room for kBigCapacity, by 16 groups, and - such
+        // regions of one set overlap, and take longer than a group waits for another - by one
+        // alone; the rest by k_insert_full.
         auto drain = [&]() -> int {
-            int nd = 0, nb[5] = {0, 0, 0, 0, 0};
-            std::vector<int> seen(ndefer_lists + 6);
+            int nd = 0, nb[6] = {0, 0, 0, 0, 0, 0};
+            std::vector<int> seen(ndefer_lists + 7);
             auto look = [&]() -> int {
                 uint32_t hs = 0;
                 D3G_CUDA(cudaGetLastError());
@@ -3344,7 +3347,7 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
                 D3G_CUDA(cudaMemcpyAsync(&hs, status.p, sizeof hs, cudaMemcpyDeviceToHost, s));
                 D3G_CUDA(cudaStreamSynchronize(s));
                 nd = seen[size_t(deferred)];
-                std::copy(seen.end() - 5, seen.end(), nb);
+                std::copy(seen.end() - 6, seen.end(), nb);
                 if (opt.timing) {
                     float am = 0.f;
                     cudaEventElapsedTime(&am, kev[0], kev[1]);
@@ -3357,38 +3360,44 @@ int build_sets_impl(const double* d_xyz, const int64_t* h_off, int nsets, const 
                 return st;
             };
             D3G_TRY(look());
-            for (int k = 0; nd > 0 && k < kExactPasses; ++k) {
+            for (int k = 0; nd > 4 * nb[0] && k < kExactPasses; ++k) {   // (else most regions are large)
+                const int before = nd;
                 D3G_TRY(exact_pass(nd, int64_t(nv) - nd, std::max(kNumSMs * kExactBlocks * (kGroupThreads / 32) >> (3 * k), 16)));
                 D3G_TRY(look());
+                if (2 * nd > before) break;        // (in each other's way, or of large regions)
             }
-            if (nb[0] > 0) {
-                // (the list behind the deferred one is free here)
-                int* const lists[3] = {big.p, defer_of(deferred + 1), big.p};
+            if (nb[0] + nd > 0) {
                 // (the exact stage's stack only where some point has needed it)
-                auto* kernel = deferred > 0 ? k_insert_groups<32, kExact, kBigCapacity, 32>
-                                            : k_insert_groups<32, kNear, kBigCapacity, 32>;
+                auto* kernel = deferred > 0 || nd > 0 ? k_insert_groups<32, kExact, kBigCapacity, 32>
+                                                      : k_insert_groups<32, kNear, kBigCapacity, 32>;
                 D3G_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                               int(sizeof(GroupScratch<32, kBigCapacity>))));
+                int* const rest = defer_of(deferred + 1);      // (free here)
                 GroupArgs B = A;
                 B.cavity = opt.cavity_capacity > 0 ? cav_normal : kBigCapacity;
-                for (int k = 0; k < 2; ++k) {
-                    B.items = lists[k];
-                    B.n_items = big_ctl + 2 * k;
-                    B.most = k == 0 ? INT_MAX : kLonePoints;
-                    B.next = big_ctl + 1 + 2 * k;
-                    B.left = B.big = lists[k + 1];
-                    B.n_left = B.n_big = big_ctl + 2 + 2 * k;
-                    B.ngroups = k == 0 ? std::min(16, std::max(1, nv / kPoolSlots)) : 1;
+                auto pass = [&](int* items, const int* n, int most, int* next, int* out, int* n_out, int ngroups) {
+                    B.items = items;
+                    B.n_items = n;
+                    B.most = most;
+                    B.next = next;
+                    B.left = B.big = B.defer = out;
+                    B.n_left = B.n_big = B.n_defer = n_out;
+                    B.ngroups = std::min(ngroups, std::max(1, nv / kPoolSlots));
                     kernel<<<unsigned(B.ngroups), 32, sizeof(GroupScratch<32, kBigCapacity>), s>>>(T, B, Rd, vx.p);
                     R.stats.launches_async += 1;
+                };
+                if (nb[0] > 0) pass(big.p, big_ctl, INT_MAX, big_ctl + 1, rest, big_ctl + 2, kBigGroups);
+                if (nd > 0) pass(defer_of(deferred), n_defer_of(deferred), INT_MAX, big_ctl + 5, rest, big_ctl + 2, kBigGroups);
+                D3G_TRY(look());
+                const int left_over = nb[2];
+                if (left_over > 0) {
+                    pass(rest, big_ctl + 2, kLonePoints, big_ctl + 3, big.p, big_ctl + 4, 1);
                     D3G_TRY(look());
-                    if (nb[2] == 0) break;
                 }
-                D3G_TRY(finish_points(lists[1] + kLonePoints, nb[2] - kLonePoints));
-                D3G_TRY(finish_points(lists[2], nb[4]));
+                D3G_TRY(finish_points(rest + kLonePoints, left_over - kLonePoints));
+                D3G_TRY(finish_points(big.p, nb[4]));
             }
-            D3G_TRY(finish_points(defer_of(deferred), nd));
-            D3G_CUDA(cudaMemsetAsync(big_ctl, 0, 5 * sizeof(int), s));
+            D3G_CUDA(cudaMemsetAsync(big_ctl, 0, 6 * sizeof(int), s));
             D3G_CUDA(cudaMemsetAsync(n_defer_of(deferred), 0, sizeof(int), s));
             return D3G_OK;
         };
