@@ -388,12 +388,19 @@ int predicates_device(const double* d_pts, int64_t n_pts, const int32_t* d_idx, 
     unsigned long long* qcount = counters.p + 1;
     unsigned long long* wcount = counters.p + 2;
     unsigned long long* ncount = counters.p + 3;   // calls k_near_in_sphere leaves
-    DevBuf<int64_t> queue, rest, wqueue;
+    DevBuf<int64_t> queue, wqueue;
     const int64_t wcap = std::min<int64_t>(nq, kWideQueueCap);
     const int blk = 256;
     const bool queued = kind == D3G_ORIENT3D || kind == D3G_IN_SPHERE || kind == D3G_IN_SPHERE_UNPERTURBED;
     if (queued) {
-        D3G_TRY(queue.alloc(size_t(nq), stream));
+        // in_sphere: two queues in one block, or (without room for the second) every queued
+        // call goes to the exact stage.
+        const int room = kind == D3G_ORIENT3D ? D3G_ERR_OOM : queue.alloc(2 * size_t(nq), stream);
+        if (room == D3G_ERR_OOM) {
+            cudaGetLastError();
+            D3G_TRY(queue.alloc(size_t(nq), stream));
+        } else if (room != D3G_OK) return room;
+        int64_t* const rest = room == D3G_OK ? queue.p + nq : nullptr;
         D3G_TRY(wqueue.alloc(size_t(wcap), stream));
         const unsigned g = grid_for(nq, blk, int64_t(kNumSMs) * 16);
         if (kind == D3G_ORIENT3D) {
@@ -404,15 +411,11 @@ int predicates_device(const double* d_pts, int64_t n_pts, const int32_t* d_idx, 
         } else {
             k_filter_in_sphere<<<g, blk, 0, stream>>>(d_pts, n_pts, d_idx, nq, d_out, queue.p,
                                                       qcount, status);
-            // (without room for a second queue, every queued call goes to the exact stage)
-            const int room = rest.alloc(size_t(nq), stream);
-            if (room == D3G_OK)
+            if (rest)
                 k_near_in_sphere<<<kNumSMs * 8, 128, 0, stream>>>(d_pts, d_idx, d_out, queue.p, qcount,
-                                                                  kind == D3G_IN_SPHERE ? 1 : 0, rest.p, ncount, status);
-            else if (room == D3G_ERR_OOM) cudaGetLastError();
-            else return room;
-            k_exact_in_sphere<<<kNumSMs * 8, 128, 0, stream>>>(d_pts, d_idx, d_out, room == D3G_OK ? rest.p : queue.p,
-                                                               room == D3G_OK ? ncount : qcount,
+                                                                  kind == D3G_IN_SPHERE ? 1 : 0, rest, ncount, status);
+            k_exact_in_sphere<<<kNumSMs * 8, 128, 0, stream>>>(d_pts, d_idx, d_out, rest ? rest : queue.p,
+                                                               rest ? ncount : qcount,
                                                                kind == D3G_IN_SPHERE ? 1 : 0, wqueue.p, wcount,
                                                                wcap, status);
         }
@@ -425,7 +428,6 @@ int predicates_device(const double* d_pts, int64_t n_pts, const int32_t* d_idx, 
     D3G_CUDA(cudaMemcpyAsync(host_counters, counters.p, sizeof host_counters, cudaMemcpyDeviceToHost,
                              stream));
     queue.release();
-    rest.release();
     D3G_CUDA(cudaStreamSynchronize(stream));
     // The wide tier, for the calls queued: kWideSlots at a time, each thread
     // with its own piece of the arena.
