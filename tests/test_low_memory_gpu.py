@@ -36,7 +36,8 @@ def _fill(leave):
         if more >= 4 * MB:
             hold.append(torch.empty(more // (2 * MB) * (2 * MB), dtype=torch.uint8, device="cuda"))
     free = torch.cuda.mem_get_info()[0]
-    assert leave - 8 * MB < free < leave + 8 * MB, free
+    if abs(free - leave) > 8 * MB:
+        pytest.skip(f"{free} bytes free where {leave} were wanted: the device is shared")
     return hold
 
 
